@@ -50,7 +50,7 @@ struct HNode {
     uint64_t lb_off = 64, tab_off = 0, starts_off = 0, g_sizes = 0, g_incl = 0, g_layout = 0, tab_cap = 0;
     uint64_t hist_tiles = 0, split_tiles = 0, gfc_warps = 0;
     // decode scratch layout (relative to scratch)
-    uint64_t dlb_off = 0, dends_off = 0, druns_off = 0, dtiles_off = 0, dsizes_off = 0, dincl_off = 0;
+    uint64_t dlb_off = 0, dpre_off = 0, dends_off = 0, druns_off = 0, dtiles_off = 0, dsizes_off = 0, dincl_off = 0;
     int last_c_level = 0, last_d_level = 0;
     // compress input view: the node reads stream in_sid through vop[] (V_SCALE ops take their
     // constant from scale node vnode[k]); a virtual node's own output is never written, its child
@@ -97,8 +97,12 @@ struct Launch {
 // passes whose tiles chain through a decoupled look-back (claimed in order from a counter)
 bool dyn_pass(int op)
 {
-    return op == B_SPLIT || op == B_RLE_HEADS || op == B_GFC_SCAN || op == B_DELTA_DEC || op == B_RLE_SCAN;
+    return op == B_SPLIT || op == B_RLE_HEADS || op == B_GFC_SCAN || op == B_DELTA_DEC || op == B_RLE_SCAN ||
+           op == B_MERGE_COUNT;
 }
+
+// blocks of the counting pass of a merge over n elements
+uint64_t merge_count_tiles(uint64_t n) { return std::max<uint64_t>(1, cdiv(n, kBCountTile)); }
 
 constexpr uint32_t kMinMaxTileMin = 1024;  // the smallest min/max tile (tiles are reserved for it)
 
@@ -318,9 +322,14 @@ void BatchEngine::plan_passes()
         uint64_t d = 0;
         const uint64_t tiles = std::max<uint64_t>(1, cdiv(n, kBTile));
         switch (nd.enc) {
-        case GTSC_DELTA: case GTSC_PATCH: case GTSC_PATCH_OUTSIDE: case GTSC_DICT: case GTSC_CONST:
+        case GTSC_DELTA:
             nd.dlb_off = nd.c_bytes;
             d = align_up(lookback_bytes(tiles), 256);
+            break;
+        case GTSC_PATCH: case GTSC_PATCH_OUTSIDE: case GTSC_DICT: case GTSC_CONST:
+            nd.dlb_off = nd.c_bytes;
+            nd.dpre_off = nd.dlb_off + align_up(lookback_bytes(merge_count_tiles(n)), 256);
+            d = nd.dpre_off + align_up(8 * cdiv(n, kBMergeUnit) + 16, 256) - nd.c_bytes;
             break;
         case GTSC_RLE:
             nd.dlb_off = nd.c_bytes;
@@ -575,15 +584,15 @@ void BatchEngine::plan_passes()
         case GTSC_DELTA: { BItem it = ditem(B_DELTA_DEC, t2k); it.p[0] = nd.dlb_off; ps.push_back(it); break; }
         case GTSC_SCALE: ps.push_back(ditem(B_SCALE_ADD, t2k)); break;
         case GTSC_PATCH: case GTSC_PATCH_OUTSIDE: case GTSC_DICT: case GTSC_CONST: {
-            BItem it = ditem(B_MERGE, cdiv(t2k, kBMergeSub));
+            BItem it = ditem(B_MERGE, cdiv(n, kBMergeTile));
             it.mode = (int16_t)(nd.enc == GTSC_PATCH || nd.enc == GTSC_PATCH_OUTSIDE ? SPLIT_LOWER : nd.enc == GTSC_DICT ? SPLIT_DICT : SPLIT_NOT_CONST);
             it.p[0] = nd.dlb_off;
-            it.p[1] = t2k;
+            it.p[1] = nd.dpre_off;
             // the stencil counts need only the node's metadata, parsed before the first level: one
             // launch ahead of every level (a merge may itself run at level 0)
             BItem cnt = it;
             cnt.op = B_MERGE_COUNT;
-            cnt.tiles = (uint32_t)t2k;
+            cnt.tiles = (uint32_t)merge_count_tiles(n);
             pass_d.push_back(Pass{-1, B_MERGE_COUNT, id, cnt});
             ps.push_back(it);
             break;
@@ -708,7 +717,8 @@ void BatchEngine::layout(cudaStream_t s)
                     for (int k : live) {
                         const BItem &b = items[L.first + k];
                         if (j < b.tiles) {
-                            item_of.push_back((uint32_t)(b.tile_base + j));
+                            item_of.push_back((uint32_t)k);
+                            item_of.push_back(j);
                             live[w++] = k;
                         }
                     }
@@ -738,8 +748,9 @@ void BatchEngine::layout(cudaStream_t s)
         const uint64_t n = nd.in_cap / nd.es;
         const uint64_t t2k = std::max<uint64_t>(1, cdiv(n, kBTile));
         switch (nd.enc) {
-        case GTSC_DELTA: case GTSC_PATCH: case GTSC_PATCH_OUTSIDE: case GTSC_DICT: case GTSC_CONST: case GTSC_RLE:
-            zr(zero_d, sc + nd.dlb_off, lookback_zero_bytes(t2k));
+        case GTSC_DELTA: case GTSC_RLE: zr(zero_d, sc + nd.dlb_off, lookback_zero_bytes(t2k)); break;
+        case GTSC_PATCH: case GTSC_PATCH_OUTSIDE: case GTSC_DICT: case GTSC_CONST:
+            zr(zero_d, sc + nd.dlb_off, lookback_zero_bytes(merge_count_tiles(n)));
             break;
         case GTSC_GFC:
             if (nd.gfc_warps) zr(zero_d, sc + nd.dlb_off, lookback_zero_bytes(std::max<uint64_t>(1, cdiv(nd.gfc_warps, kBTile))));
@@ -909,11 +920,10 @@ void BatchEngine::plan_persistent(const std::vector<Launch> &launches, const std
         const bool dyn = dyn_pass(L.op);
         const uint32_t per = dyn ? 1u : kPersistChunk;
         for (uint64_t t = 0; t < L.tiles; t += per) {
-            // the unit's first tile: look-back passes in the launch's claim order (item_of after its
-            // tile table), the others in tile order
-            const uint64_t tt = dyn ? item_of[L.map_off + L.tiles + t] : t;
-            const int gi = L.first + (int)item_of[L.map_off + tt];
-            const uint64_t tile = tt - items[gi].tile_base;
+            // the unit's first tile: look-back passes in the launch's claim order (the claim table
+            // behind its tile table), the others in tile order
+            const int gi = L.first + (int)item_of[L.map_off + (dyn ? L.tiles + 2 * t : t)];
+            const uint64_t tile = dyn ? item_of[L.map_off + L.tiles + 2 * t + 1] : t - items[gi].tile_base;
             const uint32_t cnt = (uint32_t)std::min<uint64_t>(per, L.tiles - t);
             if (tile >= (1u << 28)) fail(GTSC_ERR_CAPACITY, "batch: an item has too many tiles for the persistent schedule");
             units.push_back(PUnit{(uint32_t)gi, (uint32_t)tile | (cnt << 28)});

@@ -42,7 +42,7 @@ enum BOp : int {
     B_GFC_SIZES,
     B_GFC_DEC,
     B_VMETA,           // compress: metadata of a node whose output is read through a view
-    B_MERGE_COUNT,     // decode: stencil matches per merge tile and per group of 64 tiles
+    B_MERGE_COUNT,     // decode: stencil matches before every merge unit
     B_NUM_OPS
 };
 
@@ -241,7 +241,9 @@ void launch_batch_stage(int op, const BItem *d_items, const uint32_t *d_item_of,
 // tile sizes (elements) of the batched passes
 constexpr uint32_t kBVPT = 16;         // values per thread of the element-wise and look-back passes
 constexpr uint32_t kBTile = 256 * kBVPT; // elements per tile of those passes (256 threads per block)
-constexpr uint32_t kBMergeSub = 4;      // kBTile tiles per block of the merge pass
+constexpr uint32_t kBMergeUnit = 1024;  // merge: elements of a warp's unit (32 rows of 32)
+constexpr uint32_t kBMergeTile = 8 * kBMergeUnit;    // ... of a block
+constexpr uint32_t kBCountTile = 128 * kBMergeUnit;  // ... of a block of the counting pass
 constexpr uint32_t kBGfcChunks = 8;     // GFC chunks (warps) per tile
 constexpr uint32_t kBHistSmem = 2048;    // shared hash slots of a histogram block (8-byte values)
 constexpr uint32_t kBHistPacked = 4096;  // 8 x this = the bytes of a histogram block's shared table

@@ -11,6 +11,7 @@
 #include "batch_dev.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace gtsc {
 
@@ -208,35 +209,10 @@ __device__ void p_scale_add(const BItem &it, uint32_t tile, StreamDesc *S, uint3
 }
 
 // ------------------------------------------------------------------------------- merge
-// elements [p0, p0 + cnt) of a decode view into shared memory at element slot `at`; unpacked views
-// take plain loads, packed ones the view's bit extraction
-template <int ES>
-__device__ __forceinline__ void stage_view(const DViewCtx &v, uint64_t p0, uint32_t cnt, uint8_t *sm, uint32_t at)
-{
-    if (v.b == 0) {
-        const uint64_t c = v.c0 + v.c1;
-        for (uint32_t i = threadIdx.x; i < cnt; i += kBThreads)
-            st_elem<ES>(sm, at + i, wrap_es(ld_elem<ES>(v.p, p0 + i) + c, ES));  // plain views are aligned
-    } else {
-        for (uint32_t i = threadIdx.x; i < cnt; i += kBThreads) st_elem<ES>(sm, at + i, dview_elem<ES>(v, p0 + i));
-    }
-}
-
-// Merge tiles find their offsets in the match / non-match streams without a look-back chain: a
-// counting pass (B_MERGE_COUNT, any order) stores each tile's number of stencil matches and adds it
-// to its group of kMergeGroup tiles; a merge tile's exclusive prefix is then the sum of the groups
-// before its own plus the tiles before it inside its group.  Scratch at it.p[0]: 16 bytes, the
-// group sums (u64), then the tile counts (u32) -- within the look-back area's 16 + 16 * tiles.
-constexpr uint32_t kMergeGroup = 64;
-
-__device__ __forceinline__ unsigned long long *merge_groups(const BItem &it)
-{
-    return (unsigned long long *)(it.scratch + it.p[0] + 16);  // p[1] = tiles of kBTile elements
-}
-__device__ __forceinline__ uint32_t *merge_counts(const BItem &it)
-{
-    return (uint32_t *)(it.scratch + it.p[0] + 16 + 8ull * ((it.p[1] + kMergeGroup - 1) / kMergeGroup));
-}
+// A merge works in units of kBMergeUnit = 1024 elements, one warp each, and finds a unit's offsets
+// in the match / non-match streams without waiting: a counting pass (B_MERGE_COUNT, look-back over
+// tiles of 128 units, which read only the stencil) writes the matches before every unit.
+// Scratch: the counting pass's look-back at it.p[0], the unit prefixes (u64) at it.p[1].
 
 // the stencil of a merge node and the element count its rest byte gives (0 when malformed)
 template <int ES>
@@ -254,91 +230,191 @@ __device__ __forceinline__ const uint8_t *merge_stencil(const BItem &it, const S
     return stencil;
 }
 
+// stencil bits of elements [32 k, 32 k + 32), zero at and past n; `bits` (any address) holds one bit
+// an element.  Reads only aligned words that hold a bit of an element below n.
+__device__ __forceinline__ uint32_t stencil_word(const uint8_t *bits, uint64_t k, uint64_t n)
+{
+    if (32 * k >= n) return 0u;
+    const uint32_t mis = (uint32_t)((uintptr_t)bits & 3);
+    const uint32_t *w = (const uint32_t *)(bits - mis) + k;
+    const uint32_t lo = ldg(w);
+    const uint32_t hi = mis && 8 * (4 * k + 4 - mis) < n ? ldg(w + 1) : 0u;
+    const uint32_t v = __funnelshift_r(lo, hi, 8 * mis);
+    const uint64_t left = n - 32 * k;
+    return left < 32 ? v & ((1u << left) - 1) : v;
+}
+
 template <int ES>
 __device__ void p_merge_count(const BItem &it, uint32_t tile, StreamDesc *S)
 {
-    __shared__ unsigned long long ws[32];
+    constexpr uint32_t UNITS = kBCountTile / kBMergeUnit, WARPS = kBThreads / 32, R = UNITS / WARPS;
+    constexpr uint32_t PER = UNITS / 32;  // units a lane scans
+    __shared__ __align__(16) uint32_t s_cnt[UNITS];
+    static_assert(kBMergeUnit == 32 * 32 && UNITS % (WARPS * 4) == 0, "a warp row of stencil words is one unit");
     uint64_t n;
-    const uint8_t *stencil = merge_stencil<ES>(it, S[it.in[0]], n);
-    const uint64_t base = (uint64_t)tile * kBTile + (uint64_t)threadIdx.x * kBVPT;
-    uint32_t bits = 0;
+    const uint8_t *bits = merge_stencil<ES>(it, S[it.in[0]], n) + 1;
+    // a tile past the output has no successor waiting on its look-back descriptor
+    if (tile > 0 && (uint64_t)tile * kBCountTile >= n) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t u0 = (uint64_t)tile * UNITS;
+    uint32_t w[R];
 #pragma unroll
-    for (int q = 0; q < (int)kBVPT / 8; q++)
-        if (base + 8 * q < n) bits |= (uint32_t)stencil[1 + base / 8 + q] << (8 * q);
-    const uint32_t valid_mask = base >= n ? 0u : (n - base >= kBVPT ? (1u << kBVPT) - 1 : ((1u << (n - base)) - 1));
-    unsigned long long total;
-    block_exclusive_scan<kBThreads>((unsigned long long)__popc(bits & valid_mask), ws, total);
-    if (threadIdx.x == 0) {
-        merge_counts(it)[tile] = (uint32_t)total;
-        if (total) atomicAdd(merge_groups(it) + tile / kMergeGroup, total);
+    for (int j = 0; j < (int)R; j++) w[j] = stencil_word(bits, 32 * (u0 + j * WARPS + warp) + lane, n);
+#pragma unroll
+    for (int j = 0; j < (int)R; j++) {
+        const uint32_t c = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(w[j]));
+        if (lane == 0) s_cnt[j * WARPS + warp] = c;
     }
-}
-
-// matches before `tile` (its exclusive prefix) from the counting pass; the same in every thread
-__device__ __forceinline__ unsigned long long merge_prefix(const BItem &it, uint32_t tile, unsigned long long *ws)
-{
-    const uint32_t g = tile / kMergeGroup;
-    const unsigned long long *groups = merge_groups(it);
-    const uint32_t *counts = merge_counts(it);
-    unsigned long long part = 0;
-    for (uint32_t k = threadIdx.x; k < g; k += kBThreads) part += groups[k];
-    for (uint32_t k = g * kMergeGroup + threadIdx.x; k < tile; k += kBThreads) part += counts[k];
-    unsigned long long total;
-    block_exclusive_scan<kBThreads>(part, ws, total);
-    return total;
-}
-
-// The counting launch of the merges: one warp per tile (512 stencil bytes, 16 per lane), so no
-// block barrier sits between a tile's loads and its count.
-__global__ void __launch_bounds__(kBThreads)
-k_merge_count(const BItem *items, const uint32_t *item_of, StreamDesc *S, const uint32_t *status, uint32_t total_tiles)
-{
-    if (*(volatile const uint32_t *)(status + 1)) return;
-    const int lane = threadIdx.x & 31;
-    const uint32_t warps = gridDim.x * (kBThreads / 32);
-    for (uint32_t t = blockIdx.x * (kBThreads / 32) + (threadIdx.x >> 5); t < total_tiles; t += warps) {
-        const BItem &it = items[item_of[t]];
-        const uint32_t tile = t - (uint32_t)it.tile_base;
-        uint64_t n;
-        const uint8_t *stencil;
-        switch (it.es) {
-        case 1: stencil = merge_stencil<1>(it, S[it.in[0]], n); break;
-        case 2: stencil = merge_stencil<2>(it, S[it.in[0]], n); break;
-        case 4: stencil = merge_stencil<4>(it, S[it.in[0]], n); break;
-        default: stencil = merge_stencil<8>(it, S[it.in[0]], n); break;
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t mine[PER], c = 0;
+#pragma unroll
+        for (int k = 0; k < (int)PER; k++) c += mine[k] = s_cnt[PER * lane + k];
+        uint32_t x = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
         }
-        const uint64_t e0 = (uint64_t)tile * kBTile + (uint64_t)lane * 128;  // this lane's 128 elements
-        uint32_t c = 0;
-        if (e0 < n) {
-            const uint64_t valid = n - e0 < 128 ? n - e0 : 128;
-            const uint8_t *b = stencil + 1 + e0 / 8;
-            for (uint32_t q = 0; q < (valid + 7) / 8; q++) {
-                uint32_t byte = b[q];
-                const uint64_t left = valid - 8ull * q;
-                if (left < 8) byte &= (1u << left) - 1;
-                c += __popc(byte);
-            }
-        }
-        for (int o = 16; o; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-        if (lane == 0) {
-            merge_counts(it)[tile] = c;
-            if (c) atomicAdd(merge_groups(it) + tile / kMergeGroup, (unsigned long long)c);
+        const uint32_t total = __shfl_sync(0xffffffffu, x, 31);
+        const Lookback lb = lookback_at(it.scratch + it.p[0], it.tiles);
+        unsigned long long e = lookback_exclusive(lb, tile, total) + (x - c);
+        unsigned long long *pre = (unsigned long long *)(it.scratch + it.p[1]);
+#pragma unroll
+        for (int k = 0; k < (int)PER; k++) {
+            const uint64_t u = u0 + PER * lane + k;
+            if (u * kBMergeUnit < n) pre[u] = e;
+            e += mine[k];
         }
     }
 }
 
-// Shared staging of the merge and the RLE expansion, declared once at file scope: a __shared__
-// array inside a function template is one array per instantiation (per element size), which a
-// kernel running every pass kind for every element size could not hold.
-static __shared__ uint32_t s_merge_codes[kBTile / 16 + 2];              // the tile's dictionary code words
-static __shared__ uint16_t s_merge_bits[kBThreads], s_merge_excl[kBThreads];  // stencil bits, matches before
-static __shared__ uint16_t s_rle_end[kBTile + 2];                       // the tile's run ends
-
+// One of a unit's two sources: values of b bits (mask) from bit s of the words at w (a plain stream
+// is one of full-width values), `left` values from there to the stream's end, c added to each.
 template <int ES>
-__device__ void p_merge(const BItem &it, uint32_t stile, StreamDesc *S, uint32_t *status, uint8_t *sm)
+struct MergeSrc {
+    using V = std::conditional_t<ES == 8, uint64_t, uint32_t>;
+    const uint32_t *w = nullptr;
+    uint32_t s = 0, b = 0;
+    V mask = 0, c = 0;
+    uint64_t left = 0;
+    __device__ __forceinline__ void set(const uint8_t *p, uint64_t off_bits, uint32_t width, uint64_t first, uint64_t n,
+                                        uint64_t add)
+    {
+        const uint64_t bit = off_bits + first * width;
+        w = (const uint32_t *)p + (bit >> 5);
+        s = (uint32_t)(bit & 31);
+        b = width;
+        mask = width >= 8 * sizeof(V) ? ~(V)0 : ((V)1 << width) - 1;
+        left = n > first ? n - first : 0;
+        c = (V)add;
+    }
+    __device__ __forceinline__ void set(const DViewCtx &v, uint64_t first)
+    {
+        const uint32_t mis = (uint32_t)((uintptr_t)v.p & 3);
+        if (v.b) set(v.p, v.off_bits, (uint32_t)v.b, first, v.n, v.c0 + v.c1);
+        else set(v.p - mis, 8 * mis, 8 * ES, first, v.n, v.c0 + v.c1);
+    }
+};
+
+// R rows of 32 elements of one unit, from row j0.  In row j lane l's element is a match when bit l of
+// the row's stencil word is set (lane j holds the word); its rank among the unit's matches is the
+// matches before the row (pre, lane j) plus the word's set bits below l.  So each row's two runs are
+// read where they lie, consecutive words by consecutive lanes, and the row is stored as 32
+// consecutive elements.  A lane picks its source before it loads, so both classes take one path; all
+// R rows are loaded before the first is used, as one row at a time waits out a memory latency each.
+// CHECK: a row may pass the unit's end (cnt) or a stream's end; else whole rows whose every value
+// is followed by another whole word of its stream.
+template <int ES, int MODE, bool CHECK, int R>
+__device__ __forceinline__ bool merge_rows(const MergeSrc<ES> &ys, const MergeSrc<ES> &ns, const uint64_t (&top)[4],
+                                           uint32_t word, uint32_t pre, uint32_t j0, uint8_t *dst, uint32_t cnt)
 {
-    // a block merges kBMergeSub consecutive tiles of its item; the setup below is done once for them
-    __shared__ unsigned long long ws[32];
+    using V = typename MergeSrc<ES>::V;
+    constexpr bool ONE = MODE == SPLIT_NOT_CONST;  // only matches are read
+    const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1;
+    uint32_t bit[R], w0[R], w1[R], w2[ES == 8 ? R : 1], yes = 0;
+    bool bad = false;
+#pragma unroll
+    for (int q = 0; q < R; q++) {
+        const uint32_t m = __shfl_sync(0xffffffffu, word, j0 + q);
+        const uint32_t r = __shfl_sync(0xffffffffu, pre, j0 + q) + __popc(m & below), e = 32 * (j0 + q) + lane;
+        const bool y = (m >> lane) & 1u, first = ONE || y;
+        yes |= (uint32_t)y << q;
+        const uint32_t idx = y ? r : e - r, b = first ? ys.b : ns.b;
+        bit[q] = (first ? ys.s : ns.s) + idx * b;
+        const uint32_t *w = (first ? ys.w : ns.w) + (bit[q] >> 5);
+        bool get = !ONE || y;
+        if (CHECK) {
+            get = get && e < cnt;
+            bad |= get && idx >= (first ? ys.left : ns.left);
+            get = get && idx < (first ? ys.left : ns.left);
+        }
+        w0[q] = get ? ldg(w) : 0u;
+        w1[q] = get && (!CHECK || (bit[q] & 31) + b > 32) ? ldg(w + 1) : 0u;
+        if constexpr (ES == 8) w2[q] = get && (bit[q] & 31) + b > 64 ? ldg(w + 2) : 0u;
+    }
+#pragma unroll
+    for (int q = 0; q < R; q++) {
+        const bool y = (yes >> q) & 1u;
+        V v;
+        if constexpr (ES == 8)
+            v = ((uint64_t)__funnelshift_r(w1[q], w2[q], bit[q]) << 32) | __funnelshift_r(w0[q], w1[q], bit[q]);
+        else
+            v = __funnelshift_r(w0[q], w1[q], bit[q]);
+        if (MODE == SPLIT_DICT) {
+            // a match's 2-bit code
+            const V lo = (uint32_t)v & 1u ? (V)top[1] : (V)top[0], hi = (uint32_t)v & 1u ? (V)top[3] : (V)top[2];
+            const V t = (uint32_t)v & 2u ? hi : lo, x = (v & ns.mask) + ns.c;
+            v = y ? t : x;
+        } else if (ONE) {
+            const V x = (v & ys.mask) + ys.c;
+            v = y ? x : (V)top[0];
+        } else {
+            v = (v & (y ? ys.mask : ns.mask)) + (y ? ys.c : ns.c);
+        }
+        const uint32_t e = 32 * (j0 + q) + lane;
+        if (!CHECK || e < cnt) st_elem<ES>(dst, e, v);
+    }
+    return bad;
+}
+
+template <int ES, int MODE>
+__device__ __forceinline__ bool merge_unit(const MergeSrc<ES> &ys, const MergeSrc<ES> &ns, const uint64_t (&top)[4],
+                                           uint32_t word, uint8_t *dst, uint32_t cnt)
+{
+    constexpr int R = ES == 8 ? 4 : 8;
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t pre = (uint32_t)__popc(word);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, pre, o);
+        if (lane >= o) pre += y;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, pre, 31);
+    pre -= (uint32_t)__popc(word);
+    // 64 more values (at least 64 bits) past the unit's in each stream that it reads
+    const uint32_t rest = MODE == SPLIT_NOT_CONST ? 0 : kBMergeUnit - total;
+    bool bad = false;
+    if (cnt == kBMergeUnit && (total == 0 || ys.left >= total + 64) && (rest == 0 || ns.left >= rest + 64)) {
+#pragma unroll 1
+        for (uint32_t j = 0; j < kBMergeUnit / 32; j += R)
+            merge_rows<ES, MODE, false, R>(ys, ns, top, word, pre, j, dst, cnt);
+    } else {
+#pragma unroll 1
+        for (uint32_t j = 0; 32 * j < cnt; j += R)
+            bad |= merge_rows<ES, MODE, true, R>(ys, ns, top, word, pre, j, dst, cnt);
+    }
+    return bad;
+}
+
+// Decode of patch / dict / const (n stencil bits and C value bytes read, n * s written), bound by
+// memory latency: a warp holds one unit, no shared memory and no barrier, 8 rows of loads in flight
+// (4 of 8-byte values).  Before, a block staged both runs in shared memory behind two block scans a
+// 4096-value tile.  2^26 int32: Zipf(1.1) dictionary 0.401 -> 0.152 ms, patch 0.395 -> 0.154 ms (3.5
+// TB/s); with one row in flight 0.26 and 0.23 ms.
+template <int ES>
+__device__ void p_merge(const BItem &it, uint32_t tile, StreamDesc *S, uint32_t *status)
+{
     const int mode = it.mode;
     const StreamDesc meta = S[it.in[0]];
     // dictionary: in1 is the packed code stream (read plainly); otherwise both inputs may be views
@@ -348,8 +424,9 @@ __device__ void p_merge(const BItem &it, uint32_t stile, StreamDesc *S, uint32_t
     if (mode != SPLIT_DICT) v1 = dview_ctx<ES>(it, S, 1, ok1);
     if (mode != SPLIT_NOT_CONST) v2 = dview_ctx<ES>(it, S, 2, ok2);
     StreamDesc &out = S[it.out[0]];
+    const bool first = tile == 0 && threadIdx.x == 0;
     if (!ok1 || !ok2) {
-        if (stile == 0 && threadIdx.x == 0) set_status(status, GTSC_ERR_FORMAT);
+        if (first) set_status(status, GTSC_ERR_FORMAT);
         return;
     }
     const uint64_t len1 = mode == SPLIT_DICT ? in1.len : v1.n * ES, len2 = v2.n * ES;
@@ -360,120 +437,63 @@ __device__ void p_merge(const BItem &it, uint32_t stile, StreamDesc *S, uint32_t
     uint64_t n = 0;
     if (!empty) {
         if (sbytes < 1) {
-            if (stile == 0 && threadIdx.x == 0) set_status(status, GTSC_ERR_FORMAT);
+            if (first) set_status(status, GTSC_ERR_FORMAT);
             return;
         }
         const int rest = (int8_t)stencil[0];
         int64_t nn = (int64_t)(sbytes - 1) * 8;
         if (rest) nn -= 8 - rest;
         if (nn < 0 || rest < 0 || rest > 7) {
-            if (stile == 0 && threadIdx.x == 0) set_status(status, GTSC_ERR_FORMAT);
+            if (first) set_status(status, GTSC_ERR_FORMAT);
             return;
         }
         n = (uint64_t)nn;
     }
     if (n * ES > out.cap) {
-        if (stile == 0 && threadIdx.x == 0) set_status(status, GTSC_ERR_CAPACITY);
+        if (first) set_status(status, GTSC_ERR_CAPACITY);
         return;
     }
-    if (stile == 0 && threadIdx.x == 0) out.len = n * ES;
-    // dictionary stream: 16-byte header, 4 values, codes
-    uint64_t top[4] = {0, 0, 0, 0}, yes_cap = 0, no_cap = v2.n;
-    const uint8_t *codes = nullptr;
+    if (first) out.len = n * ES;
+    const uint64_t u = (uint64_t)tile * (kBMergeTile / kBMergeUnit) + (threadIdx.x >> 5);  // this warp's unit
+    const uint64_t e0 = u * kBMergeUnit;
+    if (e0 >= n) return;
+    const uint64_t yes0 = ((const unsigned long long *)(it.scratch + it.p[1]))[u], no0 = e0 - yes0;
+    const uint32_t word = stencil_word(stencil + 1, 32 * u + (threadIdx.x & 31), n);
+    const uint32_t cnt = (uint32_t)(n - e0 < kBMergeUnit ? n - e0 : kBMergeUnit);
+    uint8_t *dst = out.ptr + e0 * ES;
+    uint64_t top[4] = {0, 0, 0, 0};
+    MergeSrc<ES> ys, ns;
+    bool bad;
     if (mode == SPLIT_DICT) {
+        // dictionary stream: 16-byte header, 4 values, codes (2 bits a match)
         if (in1.len >= 16 + 4ull * ES) {
             const uint64_t m = ld_unaligned<8>(in1.ptr + 8);
             for (int k = 0; k < 4; k++) top[k] = ld_unaligned<ES>(in1.ptr + 16 + k * ES);
-            codes = in1.ptr + 16 + 4 * ES;
-            yes_cap = (in1.len - 16 - 4ull * ES) / 4 * 16;
-            if (m < yes_cap) yes_cap = m;
+            const uint8_t *codes = in1.ptr + 16 + 4 * ES;
+            const uint64_t held = (in1.len - 16 - 4ull * ES) / 4 * 16;
+            const uint32_t mis = (uint32_t)((uintptr_t)codes & 3);
+            ys.set(codes - mis, 8 * mis, 2, yes0, m < held ? m : held, 0);
         }
+        ns.set(v2, no0);
+        bad = merge_unit<ES, SPLIT_DICT>(ys, ns, top, word, dst, cnt);
     } else if (mode == SPLIT_NOT_CONST) {
         if (meta.len >= (uint64_t)ES) top[0] = ld_unaligned<ES>(meta.ptr);
-        yes_cap = v1.n;
+        ys.set(v1, yes0);
+        bad = merge_unit<ES, SPLIT_NOT_CONST>(ys, ns, top, word, dst, cnt);
     } else {
-        yes_cap = v1.n;
+        ys.set(v1, yes0);
+        ns.set(v2, no0);
+        bad = merge_unit<ES, SPLIT_LOWER>(ys, ns, top, word, dst, cnt);
     }
-    bool bad = false;
-    for (uint32_t sub = 0; sub < kBMergeSub; sub++) {
-    const uint32_t tile = stile * kBMergeSub + sub;
-    if ((uint64_t)tile * kBTile >= n) break;  // past the output
-    const uint64_t base = (uint64_t)tile * kBTile + (uint64_t)threadIdx.x * kBVPT;
-    const uint32_t valid_mask = base >= n ? 0u : (n - base >= kBVPT ? (1u << kBVPT) - 1 : ((1u << (n - base)) - 1));
-    uint32_t bits = 0;
-#pragma unroll
-    for (int q = 0; q < (int)kBVPT / 8; q++)
-        if (base + 8 * q < n) bits |= (uint32_t)stencil[1 + base / 8 + q] << (8 * q);
-    bits &= valid_mask;
-    unsigned long long total;
-    const unsigned long long excl = block_exclusive_scan<kBThreads>((unsigned long long)__popc(bits), ws, total);
-    const unsigned long long prefix = merge_prefix(it, tile, ws);
-    // the tile's runs of both streams are staged in shared memory with coalesced loads (matches
-    // first, then the rest), then every thread assembles its values from there
-    const uint64_t tile_base = (uint64_t)tile * kBTile;
-    const uint64_t tile_n = tile_base < n ? (n - tile_base < kBTile ? n - tile_base : kBTile) : 0;
-    const uint64_t ny = total, nn = tile_n - ny;
-    const uint64_t yes0 = prefix, no0 = tile_base - (tile_base < n ? yes0 : 0);
-    // dictionary: the code words of the tile's matches, staged once (coalesced, whole words)
-    uint32_t *s_codes = s_merge_codes;
-    const uint64_t w0 = yes0 >> 4;
-    if (mode == SPLIT_DICT && ny) {
-        const uint64_t nw = ((yes0 + ny + 15) >> 4) - w0;
-        const uint64_t avail = in1.len >= 16 + 4ull * ES ? (in1.len - 16 - 4ull * ES) / 4 : 0;
-        const bool al = ((uintptr_t)codes & 3) == 0;
-        for (uint64_t k = threadIdx.x; k < nw; k += kBThreads) {
-            const uint64_t w = w0 + k;
-            s_codes[k] = w >= avail ? 0u : al ? ldg((const uint32_t *)codes + w) : (uint32_t)ld_unaligned<4>(codes + 4 * w);
-        }
-    }
-    // in-tile counts fit 32 bits; a stream position past the stream's end is corrupt input
-    const uint32_t ny32 = (uint32_t)ny, nn32 = (uint32_t)nn;
-    if (mode != SPLIT_DICT) {
-        const uint32_t ok = yes_cap > yes0 ? (uint32_t)(yes_cap - yes0 < ny ? yes_cap - yes0 : ny) : 0u;
-        bad |= ok < ny32;
-        stage_view<ES>(v1, yes0, ok, sm, 0);
-    }
-    if (mode != SPLIT_NOT_CONST) {
-        const uint32_t ok = no_cap > no0 ? (uint32_t)(no_cap - no0 < nn ? no_cap - no0 : nn) : 0u;
-        bad |= ok < nn32;
-        stage_view<ES>(v2, no0, ok, sm, ny32);
-    }
-    // every thread's 16 stencil bits and the matches before them, for the striped assembly below
-    uint16_t *s_bits = s_merge_bits, *s_excl = s_merge_excl;
-    s_bits[threadIdx.x] = (uint16_t)bits;
-    s_excl[threadIdx.x] = (uint16_t)excl;
-    __syncthreads();
-    // step j writes elements j * 256 + t: consecutive threads read consecutive staged values (no
-    // bank conflicts) and store consecutive outputs (coalesced)
-    const uint32_t y0 = (uint32_t)(yes0 & 15);
-    const uint32_t lim = yes_cap > yes0 ? (uint32_t)(yes_cap - yes0 < kBTile ? yes_cap - yes0 : kBTile) : 0u;
-    uint8_t *dst = out.ptr + tile_base * ES;
-#pragma unroll 4
-    for (uint32_t e = threadIdx.x; e < (uint32_t)tile_n; e += kBThreads) {
-        const uint32_t o = e >> 4, q = e & 15;
-        const uint32_t bb = s_bits[o];
-        const uint32_t r = s_excl[o] + __popc(bb & ((1u << q) - 1));  // matches before e in the tile
-        uint64_t val;
-        if ((bb >> q) & 1u) {
-            if (mode == SPLIT_DICT) {
-                bad |= r >= lim;
-                const uint32_t y = y0 + r;
-                const uint32_t c = (s_codes[y >> 4] >> (2 * (y & 15))) & 3u;  // select, not an indexed array
-                val = c == 0 ? top[0] : c == 1 ? top[1] : c == 2 ? top[2] : top[3];
-            } else {
-                val = ld_elem_sm<ES>(sm, r);
-            }
-        } else {
-            val = mode == SPLIT_NOT_CONST ? top[0] : ld_elem_sm<ES>(sm, ny32 + (e - r));
-        }
-        st_elem<ES>(dst, e, val);
-    }
-    __syncthreads();  // the next tile restages the shared buffers
-    }
-    if (bad) set_status(status, GTSC_ERR_FORMAT);
+    if (bad) set_status(status, GTSC_ERR_FORMAT);  // a position past a stream's end: corrupt input
 }
 
 // ------------------------------------------------------------------------------- RLE decode
+// Shared staging of the RLE expansion, declared once at file scope: a __shared__ array inside a
+// function template is one array per instantiation (per element size), which a kernel running every
+// pass kind for every element size could not hold.
+static __shared__ uint16_t s_rle_end[kBTile + 2];  // the tile's run ends
+
 // node scratch: p[0] look-back, p[1] run ends (u64)
 __device__ void p_rle_scan(const BItem &it, uint32_t tile, StreamDesc *S, uint32_t *status)
 {
@@ -859,15 +879,6 @@ __device__ __forceinline__ uint32_t dec_extent(const BItem &it, const StreamDesc
         const uint64_t runs = *(const unsigned long long *)(it.scratch + it.p[2]);
         const uint64_t n = runs ? ((const unsigned long long *)(it.scratch + it.p[1]))[runs - 1] : 0;
         e = cdiv(n, kBTile);
-    } else if constexpr (OP == B_MERGE_COUNT) {
-        uint64_t n;
-        switch (it.es) {
-        case 1: merge_stencil<1>(it, S[it.in[0]], n); break;
-        case 2: merge_stencil<2>(it, S[it.in[0]], n); break;
-        case 4: merge_stencil<4>(it, S[it.in[0]], n); break;
-        default: merge_stencil<8>(it, S[it.in[0]], n); break;
-        }
-        e = cdiv(n, kBTile);
     } else if constexpr (OP == B_F2I_DEC) {
         const StreamDesc meta = S[it.in[0]];
         const int p = meta.len >= 4 ? (int32_t)ld_unaligned<4>(meta.ptr) : 0;
@@ -884,19 +895,21 @@ __device__ __forceinline__ void run_dec(const BItem &it, uint32_t tile, StreamDe
 
 constexpr bool dec_persistent(int op)
 {
-    return op == B_AFL_UNPACK || op == B_SCALE_ADD || op == B_F2I_DEC || op == B_RLE_EXPAND || op == B_MERGE_COUNT;
+    return op == B_AFL_UNPACK || op == B_SCALE_ADD || op == B_F2I_DEC || op == B_RLE_EXPAND;
 }
+
+// resident blocks per SM the compiler keeps registers for: the merge's rows need 64 registers
+constexpr int dec_min_blocks(int op) { return op == B_MERGE ? 4 : 5; }
 
 // One launch of a decode pass over every item: look-back passes one tile per block in claim order,
 // the others persistent over the tiles (see k_bstage).
 template <int OP>
-__global__ void __launch_bounds__(kBThreads, 5)
+__global__ void __launch_bounds__(kBThreads, dec_min_blocks(OP))
 k_bdec(const BItem *items, const uint32_t *item_of, StreamDesc *S, uint32_t *counter, uint32_t *status,
        uint32_t total_tiles)
 {
-    constexpr bool DYN = OP == B_DELTA_DEC || OP == B_RLE_SCAN;
-    constexpr int kSmem = OP == B_MERGE                             ? 8 * kBTile
-                          : OP == B_GFC_DEC                         ? kGfcRing * (kBThreads / 32)
+    constexpr bool DYN = OP == B_DELTA_DEC || OP == B_RLE_SCAN || OP == B_MERGE_COUNT;
+    constexpr int kSmem = OP == B_GFC_DEC                           ? kGfcRing * (kBThreads / 32)
                           : OP == B_RLE_EXPAND                      ? kXchgBlockBytes  // warp exchange
                                                                     : 16;
     __shared__ __align__(16) unsigned char smem[kSmem];
@@ -946,7 +959,7 @@ __device__ __forceinline__ void run_dec(const BItem &it, uint32_t tile, StreamDe
     else if constexpr (OP == B_AFL_UNPACK) { GTSC_ES_SWITCH(p_afl_unpack<E>(it, tile, S, status)) }
     else if constexpr (OP == B_DELTA_DEC) { GTSC_ES_SWITCH(p_delta_dec<E>(it, tile, S, status)) }
     else if constexpr (OP == B_SCALE_ADD) { GTSC_ES_SWITCH(p_scale_add<E>(it, tile, S, status)) }
-    else if constexpr (OP == B_MERGE) { GTSC_ES_SWITCH(p_merge<E>(it, tile, S, status, smem)) }
+    else if constexpr (OP == B_MERGE) { GTSC_ES_SWITCH(p_merge<E>(it, tile, S, status)) }
     else if constexpr (OP == B_MERGE_COUNT) { GTSC_ES_SWITCH(p_merge_count<E>(it, tile, S)) }
     else if constexpr (OP == B_RLE_SCAN) p_rle_scan(it, tile, S, status);
     else if constexpr (OP == B_RLE_EXPAND) { GTSC_ES_SWITCH(p_rle_expand<E>(it, tile, S, status, smem)) }
@@ -961,7 +974,7 @@ __device__ __forceinline__ void run_dec(const BItem &it, uint32_t tile, StreamDe
 
 #ifdef GTSC_PERSISTENT_TU
 // ------------------------------------------------------------------------------- persistent step
-constexpr size_t kPersistSmemD = std::max<size_t>({8 * kBTile, kGfcRing * (kBThreads / 32), kXchgBlockBytes});
+constexpr size_t kPersistSmemD = std::max<size_t>({kGfcRing * (kBThreads / 32), kXchgBlockBytes});
 
 __device__ __forceinline__ uint32_t persist_extent_d(int op, const BItem &it, const StreamDesc *S)
 {
@@ -970,7 +983,6 @@ __device__ __forceinline__ uint32_t persist_extent_d(int op, const BItem &it, co
     case B_SCALE_ADD: return dec_extent<B_SCALE_ADD>(it, S);
     case B_F2I_DEC: return dec_extent<B_F2I_DEC>(it, S);
     case B_RLE_EXPAND: return dec_extent<B_RLE_EXPAND>(it, S);
-    case B_MERGE_COUNT: return dec_extent<B_MERGE_COUNT>(it, S);
     default: return it.tiles;
     }
 }
@@ -1204,15 +1216,7 @@ void launch_batch_decode_stage(int op, const BItem *d_items, const uint32_t *d_i
         GTSC_STAGE(B_DELTA_DEC)
         GTSC_STAGE(B_SCALE_ADD)
         GTSC_STAGE(B_MERGE)
-    case B_MERGE_COUNT: {
-        int per_sm = 0;
-        GTSC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_merge_count, kBThreads, 0));
-        const uint64_t warps = (total_tiles + kBThreads / 32 - 1) / (kBThreads / 32);
-        const uint64_t resident = (uint64_t)std::max(per_sm, 1) * (uint64_t)sm_count();
-        const unsigned g = (unsigned)std::min<uint64_t>(warps, resident);
-        k_merge_count<<<g, kBThreads, 0, s>>>(d_items, d_item_of, d_streams, d_status, (uint32_t)total_tiles);
-        break;
-    }
+        GTSC_STAGE(B_MERGE_COUNT)
         GTSC_STAGE(B_RLE_SCAN)
         GTSC_STAGE(B_RLE_EXPAND)
         GTSC_STAGE(B_F2I_DEC)

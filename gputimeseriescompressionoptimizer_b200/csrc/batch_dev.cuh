@@ -740,6 +740,9 @@ __device__ __forceinline__ void persist_loop(const PersistArgs &a, Extent extent
     if (threadIdx.x == 0) persist_flush(a, cur, pend);
 }
 
+// DYN launches: after the launch's tile -> item table (gridDim.x entries) comes its claim table, the
+// (item, tile) of every claim (items interleaved round-robin, each item's tiles in order): one load
+// behind the claim's atomic, as every dependent access before a tile's data delays its look-back chain.
 template <bool DYN>
 __device__ __forceinline__ const BItem &locate(const BItem *items, const uint32_t *item_of, uint32_t *counter,
                                                uint32_t &tile)
@@ -747,12 +750,15 @@ __device__ __forceinline__ const BItem &locate(const BItem *items, const uint32_
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_idx;
     if (threadIdx.x == 0) {
-        // DYN launches: the claim order (items interleaved round-robin, each item's tiles in order)
-        // follows the launch's tile -> item table
-        const uint32_t t = DYN ? item_of[gridDim.x + atomicAdd(counter, 1u)] : blockIdx.x;
-        const uint32_t idx = item_of[t];
-        s_idx = idx;
-        s_tile = (uint32_t)(t - items[idx].tile_base);
+        if constexpr (DYN) {
+            const uint32_t *claim = item_of + gridDim.x + 2ull * atomicAdd(counter, 1u);
+            s_idx = ldg(claim);
+            s_tile = ldg(claim + 1);
+        } else {
+            const uint32_t idx = item_of[blockIdx.x];
+            s_idx = idx;
+            s_tile = (uint32_t)(blockIdx.x - items[idx].tile_base);
+        }
     }
     __syncthreads();
     tile = s_tile;

@@ -1,0 +1,56 @@
+"""The batched passes at the edges of their units and tiles: every column's blob equals the oracle's
+byte for byte and decodes bit for bit (both batch schedules, run_batch).  Sizes lie around the 32-value
+rows, the 1024-value warp units, the 8192- and 4096-value tiles and the 131072-value counting tiles."""
+import numpy as np
+import pytest
+
+import oracle as OR
+from test_batch_gpu import run_batch
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [1, 31, 32, 33, 1023, 1024, 1025, 4095, 4097, 8191, 8192, 8193, 16400, 32769, 131071, 131073, 262177]
+IDS = {OR.CHAR: "char", OR.SHORT: "short", OR.INT: "int", OR.TIME: "time", OR.FLOAT: "float", OR.DOUBLE: "double"}
+
+
+def values(rng, kind, n, npt):
+    """ties: four values and a rest; spread: few repeats; edge: one class only until the last values"""
+    if kind == "ties":
+        x = rng.choice([3, 5, 7, 11, 0, 100, 101], n, p=[.3, .25, .2, .1, .05, .05, .05])
+    elif kind == "spread":
+        x = rng.integers(0, 120 if np.dtype(npt).itemsize == 1 else 30000, n)
+    else:
+        x = np.full(n, 42)
+        x[-max(n // 50, 1):] = rng.integers(0, 100, max(n // 50, 1))
+    return x.astype(npt)
+
+
+@pytest.mark.parametrize("dt", list(IDS), ids=list(IDS.values()))
+@pytest.mark.parametrize("path", [[OR.DICT, OR.NONE, OR.NONE], [OR.CONST, OR.NONE], [OR.PATCH, OR.NONE, OR.NONE]],
+                         ids=["dict", "const", "patch"])
+def test_split_and_merge_edges(G, O, rng, dt, path):
+    cols, dts, trees = [], [], []
+    for n in SIZES:
+        for kind in ["ties", "spread", "edge"]:
+            cols.append(values(rng, kind, n, OR.NP_TYPES[dt]))
+            dts.append(dt)
+            trees.append(G.tree_from_path(path, dt))
+    run_batch(G, O, cols, dts, trees)
+
+
+@pytest.mark.parametrize("dt", [OR.SHORT, OR.INT, OR.TIME], ids=["short", "int", "time"])
+@pytest.mark.parametrize("path", [[OR.DICT, OR.NONE, OR.AFL, OR.NONE], [OR.CONST, OR.AFL, OR.NONE],
+                                  [OR.PATCH, OR.AFL, OR.NONE, OR.AFL, OR.NONE],
+                                  [OR.PATCH, OR.SCALE, OR.AFL, OR.NONE, OR.SCALE, OR.AFL, OR.NONE],
+                                  [OR.DELTA, OR.CONST, OR.AFL, OR.NONE],
+                                  [OR.DELTA, OR.SCALE, OR.PATCH, OR.AFL, OR.NONE, OR.AFL, OR.NONE]],
+                         ids=["dict", "const", "patch", "patch-scale", "delta-const", "delta-scale-patch"])
+def test_split_and_merge_through_views(G, O, rng, dt, path):
+    """sources read through delta / scale views, decoded values unpacked from AFL streams in place"""
+    cols, dts, trees = [], [], []
+    for n in SIZES[1:]:
+        for kind in ["ties", "spread", "edge"]:
+            cols.append(values(rng, kind, n, OR.NP_TYPES[dt]))
+            dts.append(dt)
+            trees.append(G.tree_from_path(path, dt))
+    run_batch(G, O, cols, dts, trees)
