@@ -97,7 +97,7 @@ struct Launch {
 // passes whose tiles chain through a decoupled look-back (claimed in order from a counter)
 bool dyn_pass(int op)
 {
-    return op == B_SPLIT || op == B_RLE_HEADS || op == B_GFC_SCAN || op == B_DELTA_DEC || op == B_RLE_SCAN ||
+    return op == B_RLE_HEADS || op == B_GFC_SCAN || op == B_DELTA_DEC || op == B_RLE_SCAN ||
            op == B_MERGE_COUNT;
 }
 
@@ -285,16 +285,16 @@ void BatchEngine::plan_passes()
         uint64_t c = 64;
         switch (nd.enc) {
         case GTSC_PATCH: case GTSC_PATCH_OUTSIDE:
-            nd.split_tiles = std::max<uint64_t>(1, cdiv(n, kBTile));
-            c = 64 + align_up(lookback_bytes(nd.split_tiles), 256);
+            nd.split_tiles = std::max<uint64_t>(1, cdiv(n, kBSplitTile));
+            c = 64 + align_up(bsplit_bytes(nd.split_tiles), 256);
             break;
         case GTSC_DICT: case GTSC_CONST: {
-            nd.split_tiles = std::max<uint64_t>(1, cdiv(n, kBTile));
+            nd.split_tiles = std::max<uint64_t>(1, cdiv(n, kBSplitTile));
             nd.hist_tiles = std::max<uint64_t>(1, cdiv(n, tune.hist_tile));
             uint64_t cap = 1024;
             while (cap < 2 * n + 64) cap <<= 1;
             nd.tab_cap = cap;
-            nd.tab_off = 64 + align_up(lookback_bytes(nd.split_tiles), 256);
+            nd.tab_off = 64 + align_up(bsplit_bytes(nd.split_tiles), 256);
             c = nd.tab_off + align_up(bhist_bytes(cap, nd.hist_tiles), 256);
             break;
         }
@@ -387,13 +387,17 @@ void BatchEngine::plan_passes()
         auto add = [&](BItem it) { ps.push_back(it); };
         const int nops = view_ops(nd.vop);
         const bool scale_view = nops > 0 && nd.vop[nops - 1] == V_SCALE;
-        // split items: p[2] / p[3] = 1 + the node whose min/max the matches / the rest feed (0 =
-        // none); layout() turns them into that node's scratch address
-        auto set_folds = [&](BItem &sp) {
+        // a split's two passes; of the counting one p[2] / p[3] = 1 + the node whose min/max the matches /
+        // the rest feed (0 = none); layout() turns them into that node's scratch address
+        auto add_split = [&](const BItem &sp) {
+            BItem cnt = sp;
+            cnt.op = B_SPLIT_COUNT;
             for (int kid : nd.kids) {
                 const int slot = folded_minmax(kid);
-                if (slot) sp.p[1 + slot] = (uint64_t)kid + 1;
+                if (slot) cnt.p[1 + slot] = (uint64_t)kid + 1;
             }
+            add(cnt);
+            add(sp);
         };
         if (nd.virt) {
             // delta: metadata only, the child can start at once; scale: min/max, then metadata
@@ -434,8 +438,7 @@ void BatchEngine::plan_passes()
             sp.mode = SPLIT_LOWER;
             sp.p[0] = 64;
             sp.p[1] = nd.enc == GTSC_PATCH_OUTSIDE;  // the outside variant's stencil
-            set_folds(sp);
-            add(sp);
+            add_split(sp);
             break;
         }
         case GTSC_DICT: case GTSC_CONST: {
@@ -456,8 +459,7 @@ void BatchEngine::plan_passes()
             sp.order = (int16_t)native_order(nd.dt);
             sp.mode = (int16_t)(nd.enc == GTSC_DICT ? SPLIT_DICT : SPLIT_NOT_CONST);
             sp.p[0] = 64;
-            set_folds(sp);
-            add(sp);
+            add_split(sp);
             break;
         }
         case GTSC_RLE: {
@@ -668,6 +670,13 @@ void BatchEngine::layout(cudaStream_t s)
     d_framed = A + framed_off;
     for (size_t i = 0; i < streams.size(); i++)
         if (sid_off[i] != UINT64_MAX) streams[i].ptr = A + sid_off[i];
+    // a split's metadata starts where its stencil (after the value, if any, and the rest byte) lies on
+    // a 4-byte boundary, so that the split stores whole stencil words (the slack behind every stream
+    // holds the shift)
+    for (auto &nd : nodes) {
+        const bool split = nd.enc == GTSC_PATCH || nd.enc == GTSC_PATCH_OUTSIDE || nd.enc == GTSC_DICT || nd.enc == GTSC_CONST;
+        if (split) streams[nd.out_sid[0]].ptr += (4 - (nd.enc == GTSC_CONST ? nd.es + 1 : 1) % 4) % 4;
+    }
     for (size_t c = 0; c < col_root.size(); c++) {
         streams[col_in_sid[c]].len = col_bytes[c];
         streams[col_out_sid[c]].cap = col_bytes[c];
@@ -690,10 +699,10 @@ void BatchEngine::layout(cudaStream_t s)
             while (j < ps.size() && ps[j].level == ps[i].level && ps[j].op == ps[i].op) {
                 BItem it = ps[j].item;
                 it.scratch = A + nodes[ps[j].node].scratch;
-                if (ps[j].op == B_SPLIT)  // the children whose min / max the split accumulates
+                if (ps[j].op == B_SPLIT_COUNT)  // the children whose min / max the split accumulates
                     for (int q = 2; q < 4; q++)
                         it.p[q] = it.p[q] ? (uint64_t)(uintptr_t)(A + nodes[it.p[q] - 1].scratch) : 0;
-                if (ps[j].op < B_NONE_COPY || ps[j].op == B_VMETA)  // compress passes: the view's scale nodes
+                if (ps[j].op < B_NONE_COPY || ps[j].op == B_VMETA || ps[j].op == B_SPLIT_COUNT)  // compress: the view's scale nodes
                     for (int v = 0; v < kMaxViewOps; v++) {
                         const int sn = nodes[ps[j].node].vnode[v];
                         it.vscr[v] = sn >= 0 ? A + nodes[sn].scratch : nullptr;
@@ -743,7 +752,8 @@ void BatchEngine::layout(cudaStream_t s)
         uint8_t *sc = A + nd.scratch;
         zr(zero_c, sc, 64);
         if (nd.enc == GTSC_FLOAT_TO_INT) zr(zero_c, sc + 64, 64);
-        if (nd.split_tiles) zr(zero_c, sc + 64, lookback_zero_bytes(nd.split_tiles));
+        if (nd.split_tiles)  // RLE: the look-back; splits: the groups' matches
+            zr(zero_c, sc + 64, nd.enc == GTSC_RLE ? lookback_zero_bytes(nd.split_tiles) : bsplit_group_bytes(nd.split_tiles));
         if (nd.gfc_warps) zr(zero_c, sc + 64, lookback_zero_bytes(std::max<uint64_t>(1, cdiv(nd.gfc_warps, kBTile))));
         const uint64_t n = nd.in_cap / nd.es;
         const uint64_t t2k = std::max<uint64_t>(1, cdiv(n, kBTile));
@@ -1166,6 +1176,7 @@ static uint64_t item_bytes(const BItem &it, const std::vector<StreamDesc> &S)
     case B_MINMAX: case B_HIST: case B_F2I_STATS: return in;
     case B_TOPK: case B_F2I_RAW: case B_GFC_SCAN: return 0;
     case B_DELTA_ENC: case B_SCALE_SUB: case B_AFL_PACK: case B_F2I_ENC: return in + L(it.out[0]) + L(it.out[1]);
+    case B_SPLIT_COUNT: return in + L(it.out[0]);
     case B_SPLIT: return in + L(it.out[0]) + L(it.out[1]) + L(it.out[2]);
     case B_RLE_HEADS: return in + L(it.out[0]) + L(it.out[2]) + L(it.out[1]);  // values, run starts
     case B_RLE_LENGTHS: return 2 * L(it.out[1]);

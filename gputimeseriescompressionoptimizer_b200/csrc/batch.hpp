@@ -21,7 +21,7 @@ enum BOp : int {
     B_AFL_PACK,
     B_HIST,            // dict / const histogram
     B_TOPK,            // one block per item
-    B_SPLIT,           // patch / const / dict split (mode in item.mode)
+    B_SPLIT,           // patch / const / dict: the values to their two streams (mode in item.mode)
     B_RLE_HEADS,
     B_RLE_LENGTHS,
     B_F2I_STATS,
@@ -43,6 +43,7 @@ enum BOp : int {
     B_GFC_DEC,
     B_VMETA,           // compress: metadata of a node whose output is read through a view
     B_MERGE_COUNT,     // decode: stencil matches before every merge unit
+    B_SPLIT_COUNT,     // compress: stencil and matches of every split unit
     B_NUM_OPS
 };
 
@@ -244,6 +245,16 @@ constexpr uint32_t kBTile = 256 * kBVPT; // elements per tile of those passes (2
 constexpr uint32_t kBMergeUnit = 1024;  // merge: elements of a warp's unit (32 rows of 32)
 constexpr uint32_t kBMergeTile = 8 * kBMergeUnit;    // ... of a block
 constexpr uint32_t kBCountTile = 128 * kBMergeUnit;  // ... of a block of the counting pass
+constexpr uint32_t kBSplitUnit = 1024;  // split: values of a warp's unit (32 rows of 32)
+constexpr uint32_t kBSplitTile = 8 * kBSplitUnit;    // ... of a block
+constexpr uint32_t kBSplitGroup = 64;                // tiles whose matches are summed together
+
+// scratch of a split: the groups' matches (u64), then per tile its 8 units' matches (u16 each)
+__host__ __device__ inline uint64_t bsplit_group_bytes(uint64_t tiles)
+{
+    return (8 * ((tiles + kBSplitGroup - 1) / kBSplitGroup) + 15) / 16 * 16;
+}
+inline uint64_t bsplit_bytes(uint64_t tiles) { return bsplit_group_bytes(tiles) + 16 * tiles; }
 constexpr uint32_t kBGfcChunks = 8;     // GFC chunks (warps) per tile
 constexpr uint32_t kBHistSmem = 2048;    // shared hash slots of a histogram block (8-byte values)
 constexpr uint32_t kBHistPacked = 4096;  // 8 x this = the bytes of a histogram block's shared table

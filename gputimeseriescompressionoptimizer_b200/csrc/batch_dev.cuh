@@ -6,6 +6,8 @@
 #include "scan.cuh"
 #include "vec.cuh"
 
+#include <type_traits>
+
 namespace gtsc {
 
 constexpr int kBThreads = 256;
@@ -320,6 +322,7 @@ __device__ __forceinline__ uint64_t d_gfc_start(const DGfc &g, int64_t w) { retu
 // view's length, computed once per block.
 struct ViewCtx {
     uint64_t c[kMaxViewOps];
+    uint64_t cc;     // the ops as one: y[i] = (the nd-th difference of x at i) - cc, wrapping
     uint64_t n;      // view elements
     uint64_t n_src;  // source elements
     int nd;          // delta ops (source elements read past the view's end)
@@ -333,18 +336,66 @@ __device__ __forceinline__ ViewCtx view_ctx(const BItem &it, const StreamDesc &s
     v.n_src = src.len / ES;
     v.nd = 0;
     v.plain = it.vop[0] == V_NONE;
+    v.cc = 0;
 #pragma unroll
     for (int k = 0; k < kMaxViewOps; k++) {
         v.c[k] = 0;
-        if (it.vop[k] == V_DELTA) ++v.nd;
+        if (it.vop[k] == V_DELTA) {
+            ++v.nd;
+            v.cc = 0;  // a constant taken from every element drops out of their differences
+        }
         else if (it.vop[k] == V_SCALE) {
             uint64_t mnb = 0, mxb = 0;
             acc_minmax((const MinMaxAcc *)it.vscr[k], ES, ORD_INT, mnb, mxb);
             v.c[k] = scale_min(mnb, mxb, ES);
+            v.cc += v.c[k];
         }
     }
     v.n = v.n_src > (uint64_t)v.nd ? v.n_src - v.nd : 0;
     return v;
+}
+
+template <int ES>
+using elem_t = std::conditional_t<
+    ES == 8, uint64_t, std::conditional_t<ES == 4, uint32_t, std::conditional_t<ES == 2, uint16_t, uint8_t>>>;
+// the type a value is computed in
+template <int ES>
+using word_t = std::conditional_t<ES == 8, uint64_t, uint32_t>;
+
+// R rows of 32 view elements from base, one element of each row a lane (row j: base + 32 j + lane);
+// FULL: all of them exist; else zeros at and past element `cnt` of the rows.  All loads are issued
+// before any is used.
+template <int ES, int R, bool FULL>
+__device__ __forceinline__ void load_rows(const ViewCtx &vc, const uint8_t *src, uint64_t base, uint32_t cnt,
+                                          word_t<ES> (&v)[R])
+{
+    const uint32_t lane = threadIdx.x & 31;
+    const elem_t<ES> *p = (const elem_t<ES> *)src + base + lane;
+    const int left = (int)cnt - (int)lane;  // row j has an element for this lane when 32 j < left
+#pragma unroll
+    for (int j = 0; j < R; j++) v[j] = FULL || 32 * j < left ? ldg(p + 32 * j) : (word_t<ES>)0;
+    if (vc.plain) return;
+    // the nd-th difference as a sum of nd + 1 elements (the view's element i exists, so x[i + nd] does)
+    using W = word_t<ES>;
+    const int nd = vc.nd;
+    const W k0 = nd & 1 ? (W)-1 : (W)1, k1 = nd == 1 ? (W)1 : nd == 2 ? (W)-2 : (W)3, k2 = nd == 2 ? (W)1 : (W)-3;
+    const W cc = (W)vc.cc;
+#pragma unroll
+    for (int j = 0; j < R; j++) v[j] = k0 * v[j] - cc;
+    if (nd >= 1) {
+#pragma unroll
+        for (int j = 0; j < R; j++)
+            if (FULL || 32 * j < left) v[j] += k1 * (W)ldg(p + 32 * j + 1);
+    }
+    if (nd >= 2) {
+#pragma unroll
+        for (int j = 0; j < R; j++)
+            if (FULL || 32 * j < left) v[j] += k2 * (W)ldg(p + 32 * j + 2) + (nd == 3 ? (W)ldg(p + 32 * j + 3) : (W)0);
+    }
+    if (ES < 4) {
+#pragma unroll
+        for (int j = 0; j < R; j++) v[j] = (elem_t<ES>)v[j];
+    }
 }
 
 // view elements [base, base + VPT) (garbage at and past the view's end)

@@ -2,7 +2,7 @@
 //
 // Each pass is one templated stage kernel launched with one block per (item, tile); the block finds
 // its item by binary search over the items' first tiles.  Passes that rank elements across tiles
-// (split, RLE heads, GFC offsets) claim tiles from a counter and chain them with the decoupled
+// (RLE heads, GFC offsets) claim tiles from a counter and chain them with the decoupled
 // look-back of scan.cuh, per item.  Every pass reads its input length from the stream table and
 // writes its outputs' lengths there; tile 0 (or the tile that ends the input) writes metadata.
 // Byte layouts are the per-encoding ones of encodings.cu (and of the reference).
@@ -738,7 +738,8 @@ __device__ void p_topk(const BItem &it, uint32_t tile, StreamDesc *S, unsigned c
     if (threadIdx.x == 0) {
         const int k = it.mode;  // 1: const -> meta[0..es), 4: dict -> out1[16 ..)
         uint8_t *dst = k == 1 ? S[it.out[0]].ptr : S[it.out[1]].ptr + 16;
-        for (int j = 0; j < k; j++) st_elem<ES>(dst, j, sc[j].count ? sc[j].bits : 0ull);
+        for (int j = 0; j < k * ES; j++)  // bytes: a const node's metadata may start anywhere
+            dst[j] = (uint8_t)((sc[j / ES].count ? sc[j / ES].bits : 0ull) >> (8 * (j % ES)));
         t.hdr->used = 0;
         t.hdr->special = 0;
         t.hdr->overflow = 0;
@@ -747,191 +748,368 @@ __device__ void p_topk(const BItem &it, uint32_t tile, StreamDesc *S, unsigned c
 }
 
 // ------------------------------------------------------------------------------- split
-__device__ __forceinline__ uint32_t spad(uint32_t x) { return x + (x >> 4); }
+// the outside variant of patch, beside SplitMode
+constexpr int kSplitOutside = 100;
+// code bytes of a warp in a dictionary's split: a unit's, from any place in a code word
+constexpr uint32_t kSplitCodes = kBSplitUnit + 16;
+
+// calls f with an element size as a constant (an integral_constant)
+template <class F>
+__device__ __forceinline__ void with_size(int es, F f)
+{
+    switch (es) {
+    case 1: f(std::integral_constant<int, 1>()); break;
+    case 2: f(std::integral_constant<int, 2>()); break;
+    case 4: f(std::integral_constant<int, 4>()); break;
+    default: f(std::integral_constant<int, 8>()); break;
+    }
+}
+
+// a split's element as a signed value, for the min / max of its classes
+template <int ES>
+using sword_t = std::conditional_t<ES == 8, int64_t, int32_t>;
 
 template <int ES>
-__device__ void p_split(const BItem &it, uint32_t tile, StreamDesc *S, uint32_t *status, unsigned char *sm)
+__device__ __forceinline__ void warp_min_max(sword_t<ES> &mn, sword_t<ES> &mx)
 {
-    __shared__ unsigned long long ws[32];
-    __shared__ unsigned long long s_prefix;
-    const int mode = it.mode;
+    if constexpr (ES == 8) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const int64_t a = __shfl_xor_sync(0xffffffffu, mn, o), b = __shfl_xor_sync(0xffffffffu, mx, o);
+            mn = a < mn ? a : mn;
+            mx = b > mx ? b : mx;
+        }
+    } else {
+        mn = __reduce_min_sync(0xffffffffu, mn);
+        mx = __reduce_max_sync(0xffffffffu, mx);
+    }
+}
+
+// a < b in the element's own arithmetic (lt_native), in registers of its width
+template <int ES, bool FP>
+__device__ __forceinline__ bool lt_word(word_t<ES> a, word_t<ES> b)
+{
+    if constexpr (FP && ES == 8) return __longlong_as_double((long long)a) < __longlong_as_double((long long)b);
+    else if constexpr (FP) return __uint_as_float(a) < __uint_as_float(b);
+    else return (std::make_signed_t<elem_t<ES>>)a < (std::make_signed_t<elem_t<ES>>)b;
+}
+
+// 16 bytes holding one 2-bit code each (or anything, where no code is) -> a code word (byte k's low
+// bits at 2 k)
+__device__ __forceinline__ uint32_t pack_codes(const uint4 &q)
+{
+    // the product's top byte gathers the four codes of a word: no two of its terms share a bit
+    auto four = [](uint32_t w) { return ((w & 0x03030303u) * 0x01041040u) >> 24; };
+    return four(q.x) | four(q.y) << 8 | four(q.z) << 16 | four(q.w) << 24;
+}
+
+// What a split compares its values with.
+template <int ES>
+struct SplitArgs {
+    word_t<ES> match[4];  // const / dict: the values looked for; a NaN never matches: another one in its place
+    bool all_nan;         // none is left
+    word_t<ES> thr, low;  // patch: the threshold (outside: the high bound) and the low bound
+};
+
+// the classes of R rows: x is a match
+template <int ES, int MODE, bool FP>
+__device__ __forceinline__ bool split_yes(word_t<ES> x, const SplitArgs<ES> &a)
+{
+    if constexpr (MODE == SPLIT_NOT_CONST) return x != a.match[0] || a.all_nan;
+    else if constexpr (MODE == SPLIT_DICT)
+        return (x == a.match[0] || x == a.match[1] || x == a.match[2] || x == a.match[3]) && !a.all_nan;
+    else if constexpr (MODE == kSplitOutside)  // OutsideOperator (stencil_operators.hpp:14-25)
+        return !(lt_word<ES, FP>(a.thr, x) || lt_word<ES, FP>(x, a.low));
+    else return lt_word<ES, FP>(x, a.thr);
+}
+
+// R rows of a unit: their ballots go to lane j (row j) of `mine`; FOLD: the signed min / max of the
+// matches and of the rest go to mm
+template <int ES, int MODE, bool FP, bool FOLD, bool FULL, int R>
+__device__ __forceinline__ void split_ballots(const ViewCtx &vc, const uint8_t *src, uint64_t base, uint32_t cnt,
+                                              uint32_t j0, const SplitArgs<ES> &a, uint32_t &mine, sword_t<ES> (&mm)[4])
+{
+    using SV = sword_t<ES>;
+    constexpr SV LO = ES == 8 ? (SV)INT64_MIN : (SV)INT32_MIN, HI = ~LO;
+    const uint32_t lane = threadIdx.x & 31;
+    const int left = (int)cnt - (int)lane;
+    word_t<ES> v[R];
+    load_rows<ES, R, FULL>(vc, src, base, cnt, v);
+#pragma unroll
+    for (int j = 0; j < R; j++) {
+        const bool in = FULL || 32 * j < left, y = in && split_yes<ES, MODE, FP>(v[j], a);
+        const uint32_t b = __ballot_sync(0xffffffffu, y);
+        mine = lane == j0 + j ? b : mine;
+        if (FOLD) {
+            const SV x = (SV)(std::make_signed_t<elem_t<ES>>)v[j];
+            const bool no = in && !y;
+            mm[0] = min(mm[0], y ? x : HI);
+            mm[1] = max(mm[1], y ? x : LO);
+            mm[2] = min(mm[2], no ? x : HI);
+            mm[3] = max(mm[3], no ? x : LO);
+        }
+    }
+}
+
+// A split takes two passes over its input: this one finds the classes (n * s read, n / 8 written) and
+// the other moves the values, so that no block ever waits for another's count.  One warp a unit of
+// 1024 values, in rows of 32: a row's ballot is its stencil word.  Also the min / max of the classes
+// that an AFL child packs (integer order, as its own min/max pass would compute it).
+template <int ES, int MODE, bool FP>
+__device__ __forceinline__ void split_count(const BItem &it, uint32_t tile, StreamDesc *S)
+{
+    using V = word_t<ES>;
+    using SV = sword_t<ES>;
+    constexpr int R = 8;
+    constexpr bool CONST = MODE == SPLIT_NOT_CONST, DICT = MODE == SPLIT_DICT;
+    constexpr uint32_t WARPS = kBThreads / 32;
     const StreamDesc in = S[it.in[0]];
     const ViewCtx vc = view_ctx<ES>(it, in);
     const uint64_t n = vc.n;
     const Order o = (Order)it.order;
-    Lookback lb = lookback_at(it.scratch + it.p[0], it.tiles);
-    // stencil location and the values matched against
     uint8_t *meta = S[it.out[0]].ptr;
-    uint8_t *stencil = mode == SPLIT_NOT_CONST ? meta + ES + 1 : meta + 1;
-    uint64_t top[4] = {0, 0, 0, 0}, thr = 0, lo = 0;
-    const bool outside = mode == SPLIT_LOWER && it.p[1] != 0;
-    if (mode == SPLIT_LOWER) {
-        uint64_t mnb = 0, mxb = 0;
-        if (!acc_minmax((const MinMaxAcc *)it.scratch, ES, o, mnb, mxb) && n) mnb = mxb = view_elem<ES>(it, vc, in.ptr, 0);
-        if (outside) d_outside_patch_bounds(mnb, mxb, it.dt, ES, lo, thr);  // thr: the high bound
-        else thr = d_patch_threshold(mnb, mxb, it.dt, ES);
-    } else if (mode == SPLIT_NOT_CONST) {
-        top[0] = ld_elem<ES>(meta, 0);
-    } else {
-        const uint8_t *tp = S[it.out[1]].ptr + 16;
-        for (int k = 0; k < 4; k++) top[k] = ld_unaligned<ES>(tp + k * ES);
-    }
     if (tile == 0 && threadIdx.x == 0) {
-        (mode == SPLIT_NOT_CONST ? meta[ES] : meta[0]) = (uint8_t)(n % 8);
+        meta[CONST ? ES : 0] = (uint8_t)(n % 8);
         if (n == 0) {
             S[it.out[0]].len = 0;
             S[it.out[1]].len = 0;
-            if (mode != SPLIT_NOT_CONST) S[it.out[2]].len = 0;
+            if (!CONST) S[it.out[2]].len = 0;
         }
     }
-    // a tile past the input has no successor waiting on its look-back descriptor (every later
-    // tile is past the input too), so it leaves at once; grids are sized for the worst case
-    if (tile > 0 && (uint64_t)tile * kBTile >= n) return;
-    const uint64_t base = (uint64_t)tile * kBTile + (uint64_t)threadIdx.x * kBVPT;
-    uint64_t v[kBVPT];
-    load_view_x<ES, kBVPT>(it, vc, in.ptr, base, v, sm);  // sm is free until the staging below
-    uint32_t bits = 0, codes = 0;
-    if (mode == SPLIT_LOWER && outside) {
-        // OutsideOperator (stencil_operators.hpp:14-25): false when x > high or x < low
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t w0 = (uint64_t)tile * kBSplitTile + warp * kBSplitUnit;  // the warp's first value
+    const uint32_t cnt = w0 >= n ? 0u : (uint32_t)(n - w0 < kBSplitUnit ? n - w0 : kBSplitUnit);
+    SplitArgs<ES> a{};
+    if constexpr (CONST || DICT) {
+        const uint8_t *tp = CONST ? meta : S[it.out[1]].ptr + 16;
+        V good = 0;
+        a.all_nan = true;
 #pragma unroll
-        for (int j = 0; j < (int)kBVPT; j++)
-            bits |= (uint32_t)!(lt_native(thr, v[j], ES, o) || lt_native(v[j], lo, ES, o)) << j;
-    } else if (mode == SPLIT_LOWER) {
+        for (int k = CONST ? 0 : 3; k >= 0; k--) {
+            const V x = CONST ? (V)ld_unaligned<ES>(tp) : (V)ld_elem<ES>(tp, k);
+            a.match[k] = x;
+            if (!is_nan_bits(x, o)) {
+                good = x;
+                a.all_nan = false;
+            }
+        }
 #pragma unroll
-        for (int j = 0; j < (int)kBVPT; j++) bits |= (uint32_t)lt_native(v[j], thr, ES, o) << j;
+        for (int k = CONST ? 0 : 3; k >= 0; k--)
+            if (is_nan_bits(a.match[k], o)) a.match[k] = good;
     } else {
-        // equal bits and not NaN (bsame): NaN-ness once per value, not once per candidate
-        const bool fp = o != ORD_INT;
-#pragma unroll
-        for (int j = 0; j < (int)kBVPT; j++) {
-            const bool nan = fp && is_nan_bits(v[j], o);
-            if (mode == SPLIT_NOT_CONST) {
-                bits |= (uint32_t)(nan || v[j] != top[0]) << j;
-            } else {
-                const uint32_t e0 = v[j] == top[0], e1 = v[j] == top[1], e2 = v[j] == top[2], e3 = v[j] == top[3];
-                bits |= (uint32_t)(!nan && (e0 | e1 | e2 | e3)) << j;
-                codes |= (nan ? 0u : (e1 | (e2 << 1) | (e3 * 3u))) << (2 * j);
-            }
+        uint64_t mnb = 0, mxb = 0, thr, low = 0;
+        if (!acc_minmax((const MinMaxAcc *)it.scratch, ES, o, mnb, mxb) && n) mnb = mxb = view_elem<ES>(it, vc, in.ptr, 0);
+        if (MODE == kSplitOutside) d_outside_patch_bounds(mnb, mxb, it.dt, ES, low, thr);  // thr: the high bound
+        else thr = d_patch_threshold(mnb, mxb, it.dt, ES);
+        a.thr = (V)thr;
+        a.low = (V)low;
+    }
+    const bool fold_y = it.p[2] != 0, fold_n = it.p[3] != 0;
+    constexpr SV LO = ES == 8 ? (SV)INT64_MIN : (SV)INT32_MIN, HI = ~LO;
+    SV mm[4] = {HI, LO, HI, LO};
+    uint32_t mine = 0;
+    if (fold_y || fold_n) {
+#pragma unroll 1
+        for (uint32_t j = 0; 32 * j < cnt; j += R) {
+            if (32 * (j + R) <= cnt) split_ballots<ES, MODE, FP, true, true, R>(vc, in.ptr, w0 + 32 * j, 32 * R, j, a, mine, mm);
+            else split_ballots<ES, MODE, FP, true, false, R>(vc, in.ptr, w0 + 32 * j, cnt - 32 * j, j, a, mine, mm);
+        }
+    } else {
+#pragma unroll 1
+        for (uint32_t j = 0; 32 * j < cnt; j += R) {
+            if (32 * (j + R) <= cnt) split_ballots<ES, MODE, FP, false, true, R>(vc, in.ptr, w0 + 32 * j, 32 * R, j, a, mine, mm);
+            else split_ballots<ES, MODE, FP, false, false, R>(vc, in.ptr, w0 + 32 * j, cnt - 32 * j, j, a, mine, mm);
         }
     }
-    if (base < n) {
-        const uint64_t valid = n - base;
-        if (valid < kBVPT) {  // Stencil::pack's index clamp: the last element fills the last byte
-            const uint32_t last = (bits >> (valid - 1)) & 1u;
-            for (int j = (int)valid; j < (int)kBVPT; j++) bits = (bits & ~(1u << j)) | (last << j);
-        }
-#pragma unroll
-        for (int q = 0; q < (int)kBVPT / 8; q++)
-            if (base + 8 * q < n) stencil[base / 8 + q] = (uint8_t)(bits >> (8 * q));
+    const uint32_t total = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(mine));
+    if (32 * lane < cnt) {
+        uint32_t word = mine;
+        const uint32_t left = cnt - 32 * lane;  // Stencil::pack's index clamp: the last element fills the last byte
+        if (left < 32 && ((word >> (left - 1)) & 1u)) word |= ~0u << left;
+        ((uint32_t *)(meta + (CONST ? ES + 1 : 1)))[w0 / 32 + lane] = word;  // 4-byte aligned (layout)
     }
-    const uint32_t valid_mask = base >= n ? 0u : (n - base >= kBVPT ? (1u << kBVPT) - 1 : ((1u << (n - base)) - 1));
-    const uint32_t yes_bits = bits & valid_mask;
-    if (it.p[2] | it.p[3]) {
-        // min / max of the matches and of the rest, for the AFL children that read them (integer
-        // order, as their own min/max pass would compute it); only the classes with such a child
-        const bool fold_y = it.p[2] != 0, fold_n = it.p[3] != 0;
-        uint64_t ymin = ~0ull, ymax = 0, nmin = ~0ull, nmax = 0;
-#pragma unroll
-        for (int j = 0; j < (int)kBVPT; j++) {
-            const uint64_t k = order_key(v[j], ES, ORD_INT);
-            const bool in = (valid_mask >> j) & 1u, y = (yes_bits >> j) & 1u;
-            if (fold_y && in && y) { ymin = k < ymin ? k : ymin; ymax = k > ymax ? k : ymax; }
-            if (fold_n && in && !y) { nmin = k < nmin ? k : nmin; nmax = k > nmax ? k : nmax; }
+    __shared__ uint32_t s_tot[WARPS];
+    __shared__ unsigned long long s_fold[WARPS][4];
+    if (lane == 0) s_tot[warp] = total;
+    if (fold_y || fold_n) {
+        warp_min_max<ES>(mm[0], mm[1]);
+        warp_min_max<ES>(mm[2], mm[3]);
+        if (lane == 0) {  // as the accumulators hold them; 0 = nothing seen
+            const uint64_t sign = 1ull << 63;
+            const bool ys = fold_y && total, ns = fold_n && cnt > total;
+            s_fold[warp][0] = ys ? ~((uint64_t)(int64_t)mm[0] ^ sign) : 0ull;
+            s_fold[warp][1] = ys ? (uint64_t)(int64_t)mm[1] ^ sign : 0ull;
+            s_fold[warp][2] = ns ? ~((uint64_t)(int64_t)mm[2] ^ sign) : 0ull;
+            s_fold[warp][3] = ns ? (uint64_t)(int64_t)mm[3] ^ sign : 0ull;
         }
-        block_minmax(ymin, ymax);
-        block_minmax(nmin, nmax);
-        if (threadIdx.x == 0) {
-            MinMaxAcc *ay = (MinMaxAcc *)it.p[2], *an = (MinMaxAcc *)it.p[3];
-            if (ay && ymin != ~0ull) atomicMax(&ay->nkmin, (unsigned long long)~ymin);
-            if (ay && ymax != 0) atomicMax(&ay->kmax, (unsigned long long)ymax);
-            if (an && nmin != ~0ull) atomicMax(&an->nkmin, (unsigned long long)~nmin);
-            if (an && nmax != 0) atomicMax(&an->kmax, (unsigned long long)nmax);
-        }
-    }
-    unsigned long long total;
-    const unsigned long long excl = block_exclusive_scan<kBThreads>((unsigned long long)__popc(yes_bits), ws, total);
-    if (threadIdx.x < 32) {
-        const unsigned long long e = lookback_exclusive(lb, tile, total);
-        if (threadIdx.x == 0) s_prefix = e;
     }
     __syncthreads();
-    // the tile's values go to shared memory in output order (matches first, then the rest), then
-    // the block writes both runs with coalesced stores
-    const uint64_t tile_base = (uint64_t)tile * kBTile;
-    const uint64_t tile_n = tile_base < n ? (n - tile_base < kBTile ? n - tile_base : kBTile) : 0;
-    const uint64_t ny = total, nn = tile_n - ny;
-    const uint64_t yes0 = s_prefix, no0 = tile_base - (tile_base < n ? yes0 : 0);
-    // staged at spad(position): one spare slot per 16, so the runs of consecutive threads (16 apart
-    // when most values match) fall into different banks.  Only the runs that are written are
-    // staged: a dictionary writes codes for its matches, a const node only its mismatches.
-    uint32_t ly = (uint32_t)excl, ln = threadIdx.x * kBVPT - (uint32_t)excl;
-    const uint32_t ny32 = (uint32_t)ny;
-    const bool stage_y = mode != SPLIT_DICT, stage_n = mode != SPLIT_NOT_CONST;
-#pragma unroll
-    for (int j = 0; j < (int)kBVPT; j++) {
-        if (!((valid_mask >> j) & 1u)) break;
-        if ((yes_bits >> j) & 1u) {
-            if (stage_y) st_elem<ES>(sm, spad(ly), v[j]);
-            ++ly;
+    if (warp == 0) {
+        static_assert(WARPS == 8, "a tile's unit counts are 8 halfwords");
+        const uint32_t c = lane < WARPS ? s_tot[lane] : 0u;
+        unsigned long long *groups = (unsigned long long *)(it.scratch + it.p[0]);
+        uint16_t *counts = (uint16_t *)((uint8_t *)groups + bsplit_group_bytes(it.tiles));
+        if (lane < WARPS) counts[(uint64_t)tile * WARPS + lane] = (uint16_t)c;
+        const uint32_t sum = __reduce_add_sync(0xffffffffu, c);
+        if (lane == 0 && sum) atomicAdd(groups + tile / kBSplitGroup, (unsigned long long)sum);
+    } else if (warp == 1 && lane < 4 && (lane < 2 ? fold_y : fold_n)) {
+        unsigned long long x = 0;
+        for (int w = 0; w < (int)WARPS; w++) x = s_fold[w][lane] > x ? s_fold[w][lane] : x;
+        MinMaxAcc *acc = (MinMaxAcc *)it.p[lane < 2 ? 2 : 3];
+        unsigned long long *dst = lane & 1 ? &acc->kmax : &acc->nkmin;
+        if (x > *(volatile unsigned long long *)dst) atomicMax(dst, x);  // most tiles do not move it
+    }
+}
+
+__device__ __forceinline__ void p_split_count(const BItem &it, uint32_t tile, StreamDesc *S)
+{
+    with_size(it.es, [&](auto es) {
+        constexpr int E = decltype(es)::value;
+        if (it.mode == SPLIT_DICT) split_count<E, SPLIT_DICT, false>(it, tile, S);
+        else if (it.mode == SPLIT_NOT_CONST) split_count<E, SPLIT_NOT_CONST, false>(it, tile, S);
+        else if (E >= 4 && it.order != ORD_INT) {
+            if (it.p[1]) split_count<E, kSplitOutside, (E >= 4)>(it, tile, S);
+            else split_count<E, SPLIT_LOWER, (E >= 4)>(it, tile, S);
         } else {
-            if (stage_n) st_elem<ES>(sm, spad(ny32 + ln), v[j]);
-            ++ln;
+            if (it.p[1]) split_count<E, kSplitOutside, false>(it, tile, S);
+            else split_count<E, SPLIT_LOWER, false>(it, tile, S);
         }
-    }
-    if (mode == SPLIT_DICT) {
-        // 2-bit codes of this thread's matches: at most two code words; a word wholly inside the
-        // thread's range is stored, a shared one is merged with atomicOr (the words start zeroed)
-        uint32_t *words = (uint32_t *)(S[it.out[1]].ptr + 16 + 4 * ES);
-        const uint64_t y0 = yes0 + excl, y1 = y0 + __popc(yes_bits);
-        uint32_t acc0 = 0u, acc1 = 0u;  // the first and the second code word of the range
-        uint32_t r = (uint32_t)(y0 & 15);  // position inside the first word (at most 15 + 16 < 32)
+    });
+}
+
+// R rows of a unit to their runs: yes / no point at the unit's first match / other value (no: at this
+// lane's), code at its first code byte
+template <int ES, int MODE, bool FULL, int R>
+__device__ __forceinline__ void split_rows(const ViewCtx &vc, const uint8_t *src, uint64_t base, uint32_t cnt, uint32_t j0,
+                                           uint32_t word, uint32_t pre, const word_t<ES> (&top)[4], elem_t<ES> *yes,
+                                           elem_t<ES> *no, unsigned char *code)
+{
+    const uint32_t lane = threadIdx.x & 31, bit = 1u << lane;
+    const int left = (int)cnt - (int)lane;
+    word_t<ES> v[R];
+    load_rows<ES, R, FULL>(vc, src, base, cnt, v);
 #pragma unroll
-        for (int j = 0; j < (int)kBVPT; j++)
-            if ((yes_bits >> j) & 1u) {
-                const uint32_t bits2 = ((codes >> (2 * j)) & 3u) << (2 * (r & 15));
-                if (r < 16) acc0 |= bits2;
-                else acc1 |= bits2;
-                ++r;
+    for (int j = 0; j < R; j++) {
+        const uint32_t m = __shfl_sync(0xffffffffu, word, j0 + j);
+        const uint32_t r = __shfl_sync(0xffffffffu, pre, j0 + j) + __popc(m & (bit - 1));
+        if (m & bit) {
+            if constexpr (MODE == SPLIT_DICT) {
+                const uint32_t e1 = v[j] == top[1], e2 = v[j] == top[2], e3 = v[j] == top[3];
+                code[r] = (uint8_t)(e1 | (e2 << 1) | (e3 * 3u));
+            } else {
+                yes[r] = (elem_t<ES>)v[j];
             }
-        if (y1 > y0) {
-            for (uint64_t w = y0 >> 4; w <= (y1 - 1) >> 4; w++) {
-                const uint32_t a = w == (y0 >> 4) ? acc0 : acc1;
-                if (16 * w >= y0 && 16 * w + 16 <= y1) words[w] = a;
-                else if (a) atomicOr(words + w, a);
-            }
+        } else if (MODE != SPLIT_NOT_CONST && (FULL || 32 * j < left)) {
+            no[32 * (int)(j0 + j) - (int)r] = (elem_t<ES>)v[j];
         }
     }
-    __syncthreads();
-    if (mode != SPLIT_DICT) {
-        uint8_t *yes = S[it.out[1]].ptr + yes0 * ES;
-        for (uint32_t i = threadIdx.x; i < ny32; i += kBThreads) st_elem<ES>(yes, i, ld_elem_sm<ES>(sm, spad(i)));
+}
+
+// The second pass: every unit's values to the match and the other stream (n * s read again -- from L2
+// for all but the largest columns -- and written).  The matches before a unit are the sums of the groups
+// before its tile's, of the tiles before it in the group and of the units before it in the tile; a
+// value's rank in its unit comes from the stencil words.  Rows are stored straight to the two runs;
+// only a dictionary's 2-bit codes pass through shared memory, to be packed 16 a word.
+// 2^26 int32, both passes: patch 0.430 -> 0.206 ms, Zipf(1.1) dictionary 0.506 -> 0.247 ms.  One pass with
+// the rows held in registers behind a look-back took 0.26 and 0.29 ms (its warps wait at the barrier of
+// the look-back); the same with two tiles in flight a block 0.27 and 0.33 ms (too few warps).
+template <int ES, int MODE>
+__device__ __forceinline__ void split_move(const BItem &it, uint32_t tile, StreamDesc *S, unsigned char *sm)
+{
+    using V = word_t<ES>;
+    constexpr int R = 8;
+    constexpr bool CONST = MODE == SPLIT_NOT_CONST, DICT = MODE == SPLIT_DICT;
+    const StreamDesc in = S[it.in[0]];
+    const ViewCtx vc = view_ctx<ES>(it, in);
+    const uint64_t n = vc.n;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t w0 = (uint64_t)tile * kBSplitTile + warp * kBSplitUnit;  // the warp's first value
+    if (w0 >= n) return;
+    const uint32_t cnt = (uint32_t)(n - w0 < kBSplitUnit ? n - w0 : kBSplitUnit);
+    const uint8_t *meta = S[it.out[0]].ptr;
+    uint32_t word = 32 * lane < cnt ? ldg((const uint32_t *)(meta + (CONST ? ES + 1 : 1)) + w0 / 32 + lane) : 0u;
+    if (cnt < 32 * lane + 32 && cnt > 32 * lane) word &= (1u << (cnt - 32 * lane)) - 1;
+    // the matches before the unit
+    const unsigned long long *groups = (const unsigned long long *)(it.scratch + it.p[0]);
+    const uint4 *counts = (const uint4 *)((const uint8_t *)groups + bsplit_group_bytes(it.tiles));
+    unsigned long long part = 0;
+    const uint32_t g = tile / kBSplitGroup;
+    for (uint32_t k = lane; k < g; k += 32) part += ldg(groups + k);
+    auto halves = [](uint32_t w) { return (w & 0xffffu) + (w >> 16); };
+    for (uint32_t k = g * kBSplitGroup + lane; k < tile; k += 32) {
+        const uint4 q = ldg(counts + k);
+        part += halves(q.x) + halves(q.y) + halves(q.z) + halves(q.w);
     }
-    if (mode != SPLIT_NOT_CONST) {
-        uint8_t *no = S[it.out[2]].ptr + no0 * ES;
-        const uint32_t nn32 = (uint32_t)nn;
-        for (uint32_t i = threadIdx.x; i < nn32; i += kBThreads)
-            st_elem<ES>(no, i, ld_elem_sm<ES>(sm, spad(ny32 + i)));
+    if (lane < warp) part += ldg((const uint16_t *)(counts + tile) + lane);
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(0xffffffffu, part, d);
+    const uint64_t yes0 = part, no0 = w0 - yes0;
+    uint32_t pre = __popc(word);
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, pre, d);
+        if (lane >= d) pre += y;
     }
-    const uint64_t yes_pos = yes0 + ny;
-    if (base < n && base + kBVPT >= n) {  // the thread holding the last element: lengths and headers
-        const uint64_t m = yes_pos;  // this is the last tile: its matches end the match stream
-        if (mode == SPLIT_LOWER) {
-            S[it.out[0]].len = 1 + (n + 7) / 8;
-            S[it.out[1]].len = m * ES;
-            S[it.out[2]].len = (n - m) * ES;
-        } else if (mode == SPLIT_NOT_CONST) {
+    const uint32_t total = __shfl_sync(0xffffffffu, pre, 31);
+    pre -= __popc(word);
+    V top[4] = {0, 0, 0, 0};
+    if constexpr (DICT)
+        for (int k = 1; k < 4; k++) top[k] = (V)ld_elem<ES>(S[it.out[1]].ptr + 16, k);
+    elem_t<ES> *yes = DICT ? nullptr : (elem_t<ES> *)S[it.out[1]].ptr + yes0;
+    elem_t<ES> *no = CONST ? nullptr : (elem_t<ES> *)S[it.out[2]].ptr + no0 + lane;
+    unsigned char *codes = sm + warp * kSplitCodes;
+    const uint32_t c0 = (uint32_t)(yes0 & 15);  // the unit's first code inside its code word
+#pragma unroll 1
+    for (uint32_t j = 0; 32 * j < cnt; j += R) {
+        // a const node moves its mismatches only: rows without one are not read again
+        if (CONST && !__any_sync(0xffffffffu, lane >= j && lane < j + R && word)) continue;
+        if (32 * (j + R) <= cnt) split_rows<ES, MODE, true, R>(vc, in.ptr, w0 + 32 * j, 32 * R, j, word, pre, top, yes, no, codes + c0);
+        else split_rows<ES, MODE, false, R>(vc, in.ptr, w0 + 32 * j, cnt - 32 * j, j, word, pre, top, yes, no, codes + c0);
+    }
+    if constexpr (DICT) {
+        // the unit's codes, 16 a word; the first and the last word may be shared with the neighbour
+        // units and are or-ed in (the words start zeroed)
+        __syncwarp();
+        uint32_t *words = (uint32_t *)(S[it.out[1]].ptr + 16 + 4 * ES) + (yes0 >> 4);
+        const uint32_t end = total ? c0 + total : 0;
+        for (uint32_t k = lane; 16 * k < end; k += 32) {
+            uint32_t x = pack_codes(((const uint4 *)codes)[k]);
+            const uint32_t lo = 16 * k < c0 ? c0 - 16 * k : 0, hi = end - 16 * k < 16 ? end - 16 * k : 16;
+            if (lo == 0 && hi == 16) {
+                words[k] = x;
+            } else {  // bytes outside [lo, hi) are of an earlier unit
+                x &= (hi == 16 ? ~0u : (1u << (2 * hi)) - 1) & (~0u << (2 * lo));
+                if (x) atomicOr(words + k, x);
+            }
+        }
+        __syncwarp();  // the next tile's codes
+    }
+    if (lane == 0 && w0 + kBSplitUnit >= n) {  // the unit of the last value: lengths and headers
+        const uint64_t m = yes0 + total;
+        if constexpr (CONST) {
             S[it.out[0]].len = ES + 1 + (n + 7) / 8;
             S[it.out[1]].len = m * ES;
-        } else {
+        } else if constexpr (DICT) {
             uint64_t *sz = (uint64_t *)S[it.out[1]].ptr;
             sz[0] = 4;
             sz[1] = m;
             S[it.out[0]].len = 1 + (n + 7) / 8;
             S[it.out[1]].len = m ? 16 + 4 * ES + 4 * ((m + 15) / 16) : 0;
             S[it.out[2]].len = (n - m) * ES;
+        } else {
+            S[it.out[0]].len = 1 + (n + 7) / 8;
+            S[it.out[1]].len = m * ES;
+            S[it.out[2]].len = (n - m) * ES;
         }
     }
-    (void)status;
+}
+
+template <int ES>
+__device__ __forceinline__ void p_split(const BItem &it, uint32_t tile, StreamDesc *S, unsigned char *sm)
+{
+    if (it.mode == SPLIT_DICT) split_move<ES, SPLIT_DICT>(it, tile, S, sm);
+    else if (it.mode == SPLIT_NOT_CONST) split_move<ES, SPLIT_NOT_CONST>(it, tile, S, sm);
+    else split_move<ES, SPLIT_LOWER>(it, tile, S, sm);
 }
 
 // ------------------------------------------------------------------------------- RLE
@@ -1408,12 +1586,11 @@ constexpr size_t stage_smem(int op)
     return op == B_AFL_PACK ? 8 * (kBTile + kBTile / 16 + 8)
          : op == B_HIST     ? 8 * kBHistPacked + 8 * 4 * (kBThreads / 32)
          : op == B_TOPK     ? sizeof(Cand) * kBThreads * 4
-         : op == B_SPLIT    ? 8 * (kBTile + kBTile / 16)  // >= kXchgBlockBytes (its loads)
+         : op == B_SPLIT    ? kSplitCodes * (kBThreads / 32)  // a dictionary's codes, a byte each
          : op == B_RLE_HEADS ? kXchgBlockBytes
          : op == B_GFC_COMPRESS ? kGfcStage * (kBThreads / 32)
                             : 16;
 }
-static_assert(stage_smem(B_SPLIT) >= kXchgBlockBytes, "the split loads through the warp exchange");
 
 // Tiles of an item that do work in a pass (the grid is sized for worst-case capacities; the real
 // stream lengths are only known on the device).  Tile 0 of a pass that writes metadata always
@@ -1437,6 +1614,9 @@ __device__ __forceinline__ uint32_t stage_extent(const BItem &it, const StreamDe
     } else if constexpr (OP == B_SCALE_SUB || OP == B_AFL_PACK || OP == B_F2I_ENC || OP == B_F2I_RAW) {
         e = cdiv(view_n(), kBTile);
         if (e == 0) e = 1;
+    } else if constexpr (OP == B_SPLIT_COUNT || OP == B_SPLIT) {
+        e = cdiv(view_n(), kBSplitTile);
+        if (e == 0) e = 1;
     } else if constexpr (OP == B_F2I_STATS) e = cdiv(view_n(), kBTile);
     else if constexpr (OP == B_RLE_LENGTHS) e = cdiv(S[it.out[1]].len / 4, kBTile);
     else if constexpr (OP == B_GFC_COMPRESS || OP == B_GFC_COMPACT) {
@@ -1455,7 +1635,7 @@ __device__ __forceinline__ void run_stage(const BItem &it, uint32_t tile, Stream
 constexpr bool stage_persistent(int op)
 {
     return op == B_MINMAX || op == B_DELTA_ENC || op == B_SCALE_SUB || op == B_AFL_PACK || op == B_F2I_STATS ||
-           op == B_F2I_ENC || op == B_F2I_RAW || op == B_RLE_LENGTHS;
+           op == B_F2I_ENC || op == B_F2I_RAW || op == B_RLE_LENGTHS || op == B_SPLIT_COUNT || op == B_SPLIT;
 }
 
 // One launch of a pass over every item.  Look-back passes take one tile per block in claim order;
@@ -1465,7 +1645,7 @@ constexpr bool stage_persistent(int op)
 constexpr int stage_min_blocks(int op)
 {
     // the histogram at 4 (64 registers, no spills) measured 6 % faster than at 5 (48 registers, spilling)
-    return op == B_SPLIT || op == B_GFC_COMPRESS || op == B_TOPK || op == B_HIST ? 4 : 5;
+    return op == B_GFC_COMPRESS || op == B_TOPK || op == B_HIST ? 4 : 5;
 }
 
 template <int OP>
@@ -1473,7 +1653,7 @@ __global__ void __launch_bounds__(kBThreads, stage_min_blocks(OP))
 k_bstage(const BItem *items, const uint32_t *item_of, StreamDesc *S, uint32_t *counter, uint32_t *status,
          uint32_t total_tiles)
 {
-    constexpr bool DYN = OP == B_SPLIT || OP == B_RLE_HEADS || OP == B_GFC_SCAN;
+    constexpr bool DYN = OP == B_RLE_HEADS || OP == B_GFC_SCAN;
     __shared__ __align__(16) unsigned char smem[stage_smem(OP)];
     if constexpr (!stage_persistent(OP)) {
         uint32_t tile;
@@ -1523,7 +1703,8 @@ __device__ __forceinline__ void run_stage(const BItem &it, uint32_t tile, Stream
     else if constexpr (OP == B_HIST) { GTSC_ES_SWITCH(p_hist<E>(it, tile, S, status, smem)) }
     else if constexpr (OP == B_TOPK) { GTSC_ES_SWITCH(p_topk<E>(it, tile, S, smem)) }
     else if constexpr (OP == B_VMETA) { GTSC_ES_SWITCH(p_vmeta<E>(it, S)) }
-    else if constexpr (OP == B_SPLIT) { GTSC_ES_SWITCH(p_split<E>(it, tile, S, status, smem)) }
+    else if constexpr (OP == B_SPLIT_COUNT) { p_split_count(it, tile, S); }
+    else if constexpr (OP == B_SPLIT) { GTSC_ES_SWITCH(p_split<E>(it, tile, S, smem)) }
     else if constexpr (OP == B_RLE_HEADS) { GTSC_ES_SWITCH(p_rle_heads<E>(it, tile, S, smem)) }
     else if constexpr (OP == B_RLE_LENGTHS) { p_rle_lengths(it, tile, S); }
     else if constexpr (OP == B_F2I_STATS) { GTSC_ES_SWITCH(p_f2i_stats<E>(it, tile, S)) }
@@ -1563,6 +1744,8 @@ __device__ __forceinline__ uint32_t persist_extent_c(int op, const BItem &it, co
     case B_F2I_ENC: return stage_extent<B_F2I_ENC>(it, S);
     case B_F2I_RAW: return stage_extent<B_F2I_RAW>(it, S);
     case B_RLE_LENGTHS: return stage_extent<B_RLE_LENGTHS>(it, S);
+    case B_SPLIT_COUNT: return stage_extent<B_SPLIT_COUNT>(it, S);
+    case B_SPLIT: return stage_extent<B_SPLIT>(it, S);
     default: return it.tiles;
     }
 }
@@ -1583,6 +1766,7 @@ __global__ void __launch_bounds__(kBThreads, 4) k_bpersist_c(PersistArgs a)
             GTSC_RUN(B_AFL_PACK)
             GTSC_RUN(B_HIST)
             GTSC_RUN(B_TOPK)
+            GTSC_RUN(B_SPLIT_COUNT)
             GTSC_RUN(B_SPLIT)
             GTSC_RUN(B_RLE_HEADS)
             GTSC_RUN(B_RLE_LENGTHS)
@@ -1652,6 +1836,7 @@ void launch_batch_stage(int op, const BItem *d_items, const uint32_t *d_item_of,
         GTSC_STAGE(B_AFL_PACK)
         GTSC_STAGE(B_HIST)
         GTSC_STAGE(B_TOPK)
+        GTSC_STAGE(B_SPLIT_COUNT)
         GTSC_STAGE(B_SPLIT)
         GTSC_STAGE(B_RLE_HEADS)
         GTSC_STAGE(B_RLE_LENGTHS)
