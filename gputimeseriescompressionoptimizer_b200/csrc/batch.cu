@@ -92,6 +92,8 @@ struct Launch {
     uint64_t tiles;
     uint64_t map_off;  // this launch's tile -> item table in the item_of array
     int level;
+    std::vector<int> after;  // the launches of this one's columns at each column's level before
+    bool last = true;        // no launch comes after it
 };
 
 // passes whose tiles chain through a decoupled look-back (claimed in order from a counter)
@@ -179,6 +181,9 @@ public:
                          const std::vector<int> &item_col, std::vector<PUnit> &units, std::vector<PItem> &pi,
                          uint32_t &total);
     PersistArgs persist_args(bool compress) const;
+    void plan_order(std::vector<Launch> &launches, const std::vector<int> &item_col) const;
+    void record_launches(const std::vector<Launch> &launches, const BItem *d_items, int counter, cudaStream_t s,
+                         const std::function<void(int)> &mark);
 };
 
 // ---------------------------------------------------------------------------------- compile
@@ -695,7 +700,7 @@ void BatchEngine::layout(cudaStream_t s)
         });
         for (size_t i = 0; i < ps.size();) {
             size_t j = i;
-            Launch L{ps[i].op, (int)items.size(), 0, 0, 0, ps[i].level};
+            Launch L{ps[i].op, (int)items.size(), 0, 0, 0, ps[i].level, {}, true};
             while (j < ps.size() && ps[j].level == ps[i].level && ps[j].op == ps[i].op) {
                 BItem it = ps[j].item;
                 it.scratch = A + nodes[ps[j].node].scratch;
@@ -740,6 +745,8 @@ void BatchEngine::layout(cudaStream_t s)
     };
     build(pass_c, items_c, launch_c, item_col_c);
     build(pass_d, items_d, launch_d, item_col_d);
+    plan_order(launch_c, item_col_c);
+    plan_order(launch_d, item_col_d);
     plan_persistent(launch_c, items_c, item_col_c, punit_c, pitem_c, q_total_c);
     plan_persistent(launch_d, items_d, item_col_d, punit_d, pitem_d, q_total_d);
 
@@ -904,6 +911,81 @@ void BatchEngine::layout(cudaStream_t s)
     GTSC_CUDA(cudaStreamSynchronize(s));
 }
 
+// What each launch of a phase waits for: a pass depends only on passes of its own column at lower
+// levels, so a launch follows the launches that hold its columns' passes at the level each column had
+// before.  The others of its level, and launches of columns that it does not hold, run beside it.
+void BatchEngine::plan_order(std::vector<Launch> &launches, const std::vector<int> &item_col) const
+{
+    struct Seen {
+        int level = INT32_MIN;
+        std::vector<int> now, before;  // the column's launches at its level, and at the level before
+    };
+    std::vector<Seen> seen(col_root.size());
+    for (int i = 0; i < (int)launches.size(); i++) {
+        Launch &L = launches[i];
+        for (int k = L.first; k < L.first + L.count; k++) {
+            Seen &c = seen[item_col[k]];
+            if (c.level != L.level) {  // launches are sorted by level
+                c.before.swap(c.now);
+                c.now.clear();
+                c.level = L.level;
+            }
+            if (c.now.empty() || c.now.back() != i) {
+                c.now.push_back(i);
+                L.after.insert(L.after.end(), c.before.begin(), c.before.end());
+            }
+        }
+        std::sort(L.after.begin(), L.after.end());
+        L.after.erase(std::unique(L.after.begin(), L.after.end()), L.after.end());
+        for (int a : L.after) launches[a].last = false;
+    }
+}
+
+// The launches of a phase.  While the stream is being captured, each becomes a graph node behind the
+// nodes it waits for (plan_order) instead of behind the launch before it: a table's short launches --
+// most of a step's time when its columns are short -- and the ends of its long ones overlap.  64
+// columns of 4 Ki to 64 Ki values, compress + decompress: 1465 -> 708 us; 256 columns up to 16 Mi values,
+// compress: 7070 -> 5710 us.
+void BatchEngine::record_launches(const std::vector<Launch> &launches, const BItem *d_items, int counter,
+                                  cudaStream_t s, const std::function<void(int)> &mark)
+{
+    cudaStreamCaptureStatus cap;
+    unsigned long long id;
+    cudaGraph_t graph;
+    const cudaGraphNode_t *deps;
+    size_t n_deps;
+    GTSC_CUDA(cudaStreamGetCaptureInfo(s, &cap, &id, &graph, &deps, &n_deps));
+    const bool capturing = cap == cudaStreamCaptureStatusActive;
+    std::vector<cudaGraphNode_t> start, wait;
+    std::vector<std::vector<cudaGraphNode_t>> node(launches.size());
+    if (capturing) start.assign(deps, deps + n_deps);
+    auto set_deps = [&]() {
+        GTSC_CUDA(cudaStreamUpdateCaptureDependencies(s, wait.data(), wait.size(), cudaStreamSetCaptureDependencies));
+    };
+    for (size_t i = 0; i < launches.size(); i++) {
+        const Launch &L = launches[i];
+        if (capturing) {
+            wait.clear();
+            for (int a : L.after) wait.insert(wait.end(), node[a].begin(), node[a].end());
+            if (wait.empty()) wait = start;
+            set_deps();
+        }
+        launch_batch_stage(L.op, d_items + L.first, d_item_of + L.map_off, L.count, L.tiles, d_streams,
+                           d_counters + counter++, d_status, s);
+        if (capturing) {
+            GTSC_CUDA(cudaStreamGetCaptureInfo(s, &cap, &id, &graph, &deps, &n_deps));
+            node[i].assign(deps, deps + n_deps);
+        }
+        mark(L.op);
+    }
+    if (capturing && !launches.empty()) {  // what follows the phase waits for every launch
+        wait.clear();
+        for (size_t i = 0; i < launches.size(); i++)
+            if (launches[i].last) wait.insert(wait.end(), node[i].begin(), node[i].end());
+        set_deps();
+    }
+}
+
 // The persistent schedule of one phase (batch.hpp, PUnit): the level launches end to end as one
 // queue of units, and per item its column and the number of that column's tiles in earlier levels.
 void BatchEngine::plan_persistent(const std::vector<Launch> &launches, const std::vector<BItem> &items,
@@ -974,12 +1056,7 @@ void BatchEngine::record_compress(cudaStream_t s, const std::function<void(int)>
         launch_batch_persistent_c(persist_args(true), s);
         mark(M_PERSIST);
     } else {
-        int ctr = 0;
-        for (auto &L : launch_c) {
-            launch_batch_stage(L.op, d_items_c + L.first, d_item_of + L.map_off, L.count, L.tiles, d_streams,
-                               d_counters + ctr++, d_status, s);
-            mark(L.op);
-        }
+        record_launches(launch_c, d_items_c, 0, s, mark);
     }
     launch_frame_sizes(d_cols, nc, d_nodes_c, d_streams, d_col_off, d_total, d_framed, s);
     mark(M_FRAME_SIZES);
@@ -1006,12 +1083,7 @@ void BatchEngine::record_decompress(cudaStream_t s, const std::function<void(int
         mark(M_PERSIST);
         return;
     }
-    int ctr = (int)launch_c.size();
-    for (auto &L : launch_d) {
-        launch_batch_stage(L.op, d_items_d + L.first, d_item_of + L.map_off, L.count, L.tiles, d_streams,
-                           d_counters + ctr++, d_status, s);
-        mark(L.op);
-    }
+    record_launches(launch_d, d_items_d, (int)launch_c.size(), s, mark);
 }
 
 void BatchEngine::capture(cudaStream_t s)
