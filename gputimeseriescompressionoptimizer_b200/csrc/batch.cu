@@ -47,7 +47,7 @@ struct HNode {
     uint64_t scratch = 0;             // offset in the arena
     uint64_t c_bytes = 0, d_bytes = 0;
     // compress scratch layout
-    uint64_t lb_off = 64, tab_off = 0, starts_off = 0, g_sizes = 0, g_incl = 0, g_layout = 0, tab_cap = 0;
+    uint64_t lb_off = 64, cand_off = 0, tab_off = 0, starts_off = 0, g_sizes = 0, g_incl = 0, g_layout = 0, tab_cap = 0;
     uint64_t hist_tiles = 0, split_tiles = 0, gfc_warps = 0;
     // decode scratch layout (relative to scratch)
     uint64_t dlb_off = 0, dpre_off = 0, dends_off = 0, druns_off = 0, dtiles_off = 0, dsizes_off = 0, dincl_off = 0;
@@ -139,6 +139,7 @@ public:
     uint32_t *d_done_c = nullptr, *d_done_d = nullptr, *d_ext_c = nullptr, *d_ext_d = nullptr;
     uint32_t *d_queue = nullptr;  // [0] compress claim counter, [1] decode claim counter
     BatchTuning tune;             // launch parameters (schedule, tile sizes)
+    uint32_t hist_tile = 0;       // the histogram tile in use
     std::vector<BatchColumn> src_cols;  // the columns (current inputs) and trees, for re-tuning
     std::vector<Tree> src_trees;
     std::vector<uint32_t> item_of;           // tile -> item tables of every launch, back to back
@@ -284,6 +285,14 @@ int BatchEngine::folded_minmax(int id) const
 
 void BatchEngine::plan_passes()
 {
+    // The histogram tile: what leaves a few tiles for each of four resident blocks per SM, between
+    // kBHistTileMin (a smaller tile spends its time on its 5120 counters) and the tuned tile.  64 columns
+    // of 4 Ki to 64 Ki values: 32K tiles leave all but a few SMs idle (a launch takes 0.2 ms, 15 us at 4K).
+    uint64_t hist_values = 0;
+    for (auto &nd : nodes)
+        if (nd.enc == GTSC_DICT || nd.enc == GTSC_CONST) hist_values += nd.in_cap / nd.es;
+    const uint64_t share = align_up(cdiv(hist_values, 24 * (uint64_t)sm_count()), 1024);
+    hist_tile = (uint32_t)std::min<uint64_t>(tune.hist_tile, std::max<uint64_t>(share, kBHistTileMin));
     // scratch sizes
     for (auto &nd : nodes) {
         const uint64_t n = nd.in_cap / nd.es;
@@ -295,11 +304,12 @@ void BatchEngine::plan_passes()
             break;
         case GTSC_DICT: case GTSC_CONST: {
             nd.split_tiles = std::max<uint64_t>(1, cdiv(n, kBSplitTile));
-            nd.hist_tiles = std::max<uint64_t>(1, cdiv(n, tune.hist_tile));
+            nd.hist_tiles = std::max<uint64_t>(1, cdiv(n, hist_tile));
             uint64_t cap = 1024;
             while (cap < 2 * n + 64) cap <<= 1;
             nd.tab_cap = cap;
-            nd.tab_off = 64 + align_up(bsplit_bytes(nd.split_tiles), 256);
+            nd.cand_off = 64 + align_up(bsplit_bytes(nd.split_tiles), 256);
+            nd.tab_off = nd.cand_off + align_up(kBCandBytes, 256);
             c = nd.tab_off + align_up(bhist_bytes(cap, nd.hist_tiles), 256);
             break;
         }
@@ -454,12 +464,19 @@ void BatchEngine::plan_passes()
             h.p[0] = nd.tab_cap;
             h.p[1] = nd.hist_tiles;
             h.p[2] = nd.tab_off;
-            h.p[3] = tune.hist_tile;
-            add(h);
-            BItem tk = h;
-            tk.op = B_TOPK;
-            tk.tiles = (uint32_t)nd.hist_tiles;  // one block per histogram tile
-            add(tk);
+            h.p[3] = hist_tile;
+            h.cand = nd.cand_off;
+            auto pass = [&](int op, uint64_t tiles) {
+                BItem x = h;
+                x.op = (int16_t)op;
+                x.tiles = (uint32_t)tiles;
+                add(x);
+            };
+            pass(B_HIST_SAMPLE, 1);
+            pass(B_HIST, nd.hist_tiles);
+            pass(B_TOPK, 1);
+            pass(B_HIST_FULL, nd.hist_tiles);
+            pass(B_TOPK_FULL, nd.hist_tiles);
             BItem sp = base_item(nd, B_SPLIT, nd.split_tiles);
             sp.order = (int16_t)native_order(nd.dt);
             sp.mode = (int16_t)(nd.enc == GTSC_DICT ? SPLIT_DICT : SPLIT_NOT_CONST);
@@ -707,7 +724,7 @@ void BatchEngine::layout(cudaStream_t s)
                 if (ps[j].op == B_SPLIT_COUNT)  // the children whose min / max the split accumulates
                     for (int q = 2; q < 4; q++)
                         it.p[q] = it.p[q] ? (uint64_t)(uintptr_t)(A + nodes[it.p[q] - 1].scratch) : 0;
-                if (ps[j].op < B_NONE_COPY || ps[j].op == B_VMETA || ps[j].op == B_SPLIT_COUNT)  // compress: the view's scale nodes
+                if (ps[j].op < B_NONE_COPY || ps[j].op == B_VMETA || ps[j].op >= B_SPLIT_COUNT)  // compress: the view's scale nodes
                     for (int v = 0; v < kMaxViewOps; v++) {
                         const int sn = nodes[ps[j].node].vnode[v];
                         it.vscr[v] = sn >= 0 ? A + nodes[sn].scratch : nullptr;
@@ -761,6 +778,7 @@ void BatchEngine::layout(cudaStream_t s)
         if (nd.enc == GTSC_FLOAT_TO_INT) zr(zero_c, sc + 64, 64);
         if (nd.split_tiles)  // RLE: the look-back; splits: the groups' matches
             zr(zero_c, sc + 64, nd.enc == GTSC_RLE ? lookback_zero_bytes(nd.split_tiles) : bsplit_group_bytes(nd.split_tiles));
+        if (nd.cand_off) zr(zero_c, sc + nd.cand_off, kBCandZero);
         if (nd.gfc_warps) zr(zero_c, sc + 64, lookback_zero_bytes(std::max<uint64_t>(1, cdiv(nd.gfc_warps, kBTile))));
         const uint64_t n = nd.in_cap / nd.es;
         const uint64_t t2k = std::max<uint64_t>(1, cdiv(n, kBTile));
@@ -1246,7 +1264,7 @@ static uint64_t item_bytes(const BItem &it, const std::vector<StreamDesc> &S)
     const uint64_t in = L(it.in[0]);
     switch (it.op) {
     case B_MINMAX: case B_HIST: case B_F2I_STATS: return in;
-    case B_TOPK: case B_F2I_RAW: case B_GFC_SCAN: return 0;
+    case B_TOPK: case B_HIST_SAMPLE: case B_HIST_FULL: case B_TOPK_FULL: case B_F2I_RAW: case B_GFC_SCAN: return 0;
     case B_DELTA_ENC: case B_SCALE_SUB: case B_AFL_PACK: case B_F2I_ENC: return in + L(it.out[0]) + L(it.out[1]);
     case B_SPLIT_COUNT: return in + L(it.out[0]);
     case B_SPLIT: return in + L(it.out[0]) + L(it.out[1]) + L(it.out[2]);
@@ -1443,7 +1461,7 @@ BatchEngine *batch_autotune(BatchEngine *e, cudaStream_t s, TuneReport *report)
     const bool has_hist = std::any_of(e->items_c.begin(), e->items_c.end(), [](const BItem &it) { return it.op == B_HIST; });
     if (has_hist) {
         e->tune.persistent_c = false;
-        float best_h = time_passes(e, {B_HIST, B_TOPK}, s, 3);
+        float best_h = time_passes(e, {B_HIST, B_TOPK, B_HIST_FULL, B_TOPK_FULL}, s, 3);
         e->tune.persistent_c = keep_c;
         for (uint32_t tile : {8192u, 16384u, 32768u}) {
             if (tile == best.hist_tile) continue;
@@ -1454,7 +1472,7 @@ BatchEngine *batch_autotune(BatchEngine *e, cudaStream_t s, TuneReport *report)
             float t = 1e30f;
             try {
                 batch_compress(x, s);
-                t = time_passes(x, {B_HIST, B_TOPK}, s, 3);
+                t = time_passes(x, {B_HIST, B_TOPK, B_HIST_FULL, B_TOPK_FULL}, s, 3);
             } catch (...) {
                 batch_destroy(x);
                 throw;

@@ -19,8 +19,8 @@ enum BOp : int {
     B_DELTA_ENC,
     B_SCALE_SUB,
     B_AFL_PACK,
-    B_HIST,            // dict / const histogram
-    B_TOPK,            // one block per item
+    B_HIST,            // dict / const: exact counts of the candidates, bounds of the other values
+    B_TOPK,            // the most frequent values, where the bounds prove them
     B_SPLIT,           // patch / const / dict: the values to their two streams (mode in item.mode)
     B_RLE_HEADS,
     B_RLE_LENGTHS,
@@ -44,6 +44,9 @@ enum BOp : int {
     B_VMETA,           // compress: metadata of a node whose output is read through a view
     B_MERGE_COUNT,     // decode: stencil matches before every merge unit
     B_SPLIT_COUNT,     // compress: stencil and matches of every split unit
+    B_HIST_SAMPLE,     // compress: dict / const: the candidates, from a sample
+    B_HIST_FULL,       // compress: dict / const: the full histogram, where the bounds prove nothing
+    B_TOPK_FULL,       // compress: its most frequent values
     B_NUM_OPS
 };
 
@@ -85,6 +88,7 @@ struct BItem {
     int32_t out[3];              // output stream ids (compress: meta, out1, out2; decode: out[0])
     uint8_t *scratch;            // the node's scratch: accumulators, look-back state, tables
     uint64_t p[4];               // pass parameters (scratch offsets, capacities)
+    uint64_t cand;              // dict / const histogram passes: the candidates' offset in the scratch
     int8_t vop[kMaxViewOps];     // the input view: ops applied to in[0] (compress passes)
     int8_t vflags;               // bit 0: AFL width from the view's last scale (no own min/max pass)
     uint8_t *vscr[kMaxViewOps];  // V_SCALE: that scale node's scratch (its MinMaxAcc)
@@ -127,7 +131,7 @@ class BatchEngine;
 struct BatchTuning {
     uint32_t minmax_tile = 8192;   // min/max pass: a multiple of 256 x minmax_vpt, 1K .. 16K
     uint32_t minmax_vpt = 16;      // min/max pass: consecutive values a thread loads per round (1 .. 16)
-    uint32_t hist_tile = 32768;    // histogram pass (dict / const), 8K .. 32K
+    uint32_t hist_tile = 32768;    // histogram pass (dict / const), 8K .. 32K: the largest tile
     bool persistent_c = false;     // compress step: one persistent launch instead of the levels
     bool persistent_d = false;     // decompress step: the same
 };
@@ -256,10 +260,19 @@ __host__ __device__ inline uint64_t bsplit_group_bytes(uint64_t tiles)
 }
 inline uint64_t bsplit_bytes(uint64_t tiles) { return bsplit_group_bytes(tiles) + 16 * tiles; }
 constexpr uint32_t kBGfcChunks = 8;     // GFC chunks (warps) per tile
-constexpr uint32_t kBHistSmem = 2048;    // shared hash slots of a histogram block (8-byte values)
-constexpr uint32_t kBHistPacked = 4096;  // 8 x this = the bytes of a histogram block's shared table
-constexpr uint32_t kBHistSlots16 = 5456; // its slots for values of up to 4 bytes (16-bit counts)
-constexpr uint32_t kBHistTileMax = 32768; // largest histogram tile (a 16-bit count holds its values)
+constexpr uint32_t kBHistTileMax = 32768;   // largest histogram tile
+constexpr uint32_t kBHistTileMin = 4096;    // the smallest that the batch chooses by itself
+constexpr uint32_t kBHistThreads = 512;     // threads of a histogram block of the stage launch
+constexpr uint32_t kBHistBytes = 96 << 10;  // its shared table: two blocks an SM
+constexpr uint32_t kBHistBytesPersist = 32 << 10;  // ... of the persistent kernel
+
+// The candidates of a dict / const node: a table of 512 buckets of two keys, their exact counts, and
+// counts of all other values by 4096 hash buckets.
+constexpr uint32_t kBCandSlots = 1024, kBCandCoarse = 4096;
+// scratch: flag (1 = nothing proven), the smallest NaNs, counts, coarse counts (zeroed each step), then
+// the keys
+constexpr uint64_t kBCandZero = 48 + 4 * (kBCandSlots + kBCandCoarse);
+constexpr uint64_t kBCandBytes = kBCandZero + 8 * kBCandSlots;
 
 // scratch layout of a histogram item
 struct BHistHdr {

@@ -398,6 +398,47 @@ __device__ __forceinline__ void load_rows(const ViewCtx &vc, const uint8_t *src,
     }
 }
 
+// 16 bytes' worth of consecutive view elements from base (a multiple of them), zeros past the view's
+// end: one vector load where the source holds all of them, 16-byte aligned
+template <int ES>
+__device__ __forceinline__ void load_vec(const ViewCtx &vc, const uint8_t *src, uint64_t base, word_t<ES> (&v)[16 / ES])
+{
+    using W = word_t<ES>;
+    constexpr int N = 16 / ES;
+    const elem_t<ES> *p = (const elem_t<ES> *)src + base;
+    W x[N + kMaxViewOps];
+    const bool whole = base + N <= vc.n;  // then the source has them too
+    if (whole && ((uintptr_t)src & 15) == 0) {
+        const uint4 q = ld_chunk((const uint8_t *)p);
+#pragma unroll
+        for (int j = 0; j < N; j++) x[j] = (W)chunk_elem<ES>(q, j);
+        if (vc.plain) {
+#pragma unroll
+            for (int j = 0; j < N; j++) v[j] = x[j];
+            return;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < N; j++) x[j] = base + j < vc.n_src ? (W)ldg(p + j) : (W)0;
+    }
+    if (!vc.plain) {
+        const int nd = vc.nd;
+        const W k0 = nd & 1 ? (W)-1 : (W)1, k1 = nd == 1 ? (W)1 : nd == 2 ? (W)-2 : (W)3, k2 = nd == 2 ? (W)1 : (W)-3;
+        const W cc = (W)vc.cc;
+#pragma unroll
+        for (int j = 0; j < kMaxViewOps; j++) x[N + j] = j < nd && base + N + j < vc.n_src ? (W)ldg(p + N + j) : (W)0;
+#pragma unroll
+        for (int j = 0; j < N; j++) {  // as load_rows
+            W y = k0 * x[j] - cc;
+            if (nd >= 1) y += k1 * x[j + 1];
+            if (nd >= 2) y += k2 * x[j + 2] + (nd == 3 ? x[j + 3] : (W)0);
+            x[j] = (elem_t<ES>)y;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < N; j++) v[j] = whole || base + j < vc.n ? x[j] : (W)0;
+}
+
 // view elements [base, base + VPT) (garbage at and past the view's end)
 template <int ES, int VPT>
 __device__ __forceinline__ void load_view(const BItem &it, const ViewCtx &vc, const uint8_t *src, uint64_t base,

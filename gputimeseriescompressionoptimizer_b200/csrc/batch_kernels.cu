@@ -388,7 +388,12 @@ __device__ void g_insert(const HTab &t, unsigned long long key, unsigned int c, 
     for (uint64_t probe = 0; probe < t.cap && probe < 8192; probe++) {
         const unsigned long long prev = atomicCAS(t.keys + h, EMPTY, key);
         if (prev == EMPTY) {
-            const unsigned int u = atomicAdd(&t.hdr->used, 1u);
+            // the lanes that took a slot together reserve their places in the list with one addition
+            const unsigned took = __activemask(), lane = threadIdx.x & 31;
+            const int leader = __ffs(took) - 1;
+            unsigned int u = 0;
+            if ((int)lane == leader) u = atomicAdd(&t.hdr->used, (unsigned)__popc(took));
+            u = __shfl_sync(took, u, leader) + __popc(took & ((1u << lane) - 1));
             t.used[u] = (unsigned int)h;
             atomicAdd(t.counts + h, c);
             return;
@@ -429,323 +434,830 @@ __device__ __forceinline__ void g_insert_many(const HTab &t, const unsigned long
     }
 }
 
-template <int ES>
-__device__ void p_hist(const BItem &it, uint32_t tile, StreamDesc *S, uint32_t *status, unsigned char *smem)
+// The shared table of a histogram block: buckets of two (key, count) slots.  Values of up to 4 bytes
+// have 32-bit keys (8 bytes a slot), 8-byte values 64-bit ones (12).  An empty slot holds a mark, any
+// value that does not hash to its bucket, so that a lookup needs no test for empty slots: MARK, and
+// MARK2 in MARK's own bucket.  The two marks themselves are never put in the table.  Behind it lie
+// the warps' queues of values to insert.
+constexpr uint32_t kHistQueue = 64;  // values of a warp's queue
+
+// Accesses of the tables by shared-memory address: through generic pointers each addition was compiled
+// with a test of the address space around it (full histogram of 2^26 Zipf ids 0.309 -> 0.287 ms).
+__device__ __forceinline__ void sm_add(uint32_t a, uint32_t c) { asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(a), "r"(c) : "memory"); }
+__device__ __forceinline__ void sm_pair(uint32_t a, uint32_t &x, uint32_t &y)
 {
-    constexpr unsigned long long EMPTY = ~0ull;
-    unsigned long long *skeys = (unsigned long long *)smem;
-    unsigned int *scounts = (unsigned int *)(smem + 8 * kBHistSmem);
-    unsigned long long(*snan)[4] = (unsigned long long(*)[4])(smem + 8 * kBHistPacked);
-    const StreamDesc in = S[it.in[0]];
-    const ViewCtx vc = view_ctx<ES>(it, in);
-    const uint64_t n = vc.n;
-    const uint64_t HT = it.p[3];  // the tuned histogram tile
-    const uint64_t t0 = (uint64_t)tile * HT;
-    const HTab t = htab(it);
-    const Order o = (Order)it.order;
-    if (it.mode == 4 && t0 < n) {
-        // dict: clear this tile's share of the 2-bit code words (out1 after its 16 + 4*es header)
-        uint32_t *words = (uint32_t *)(S[it.out[1]].ptr + 16 + 4 * ES);
-        const uint64_t e_end = n < t0 + HT ? n : t0 + HT;
-        for (uint64_t w = t0 / 16 + threadIdx.x; w < (e_end + 15) / 16; w += kBThreads) words[w] = 0u;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(x), "=r"(y) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void sm_pair(uint32_t a, uint64_t &x, uint64_t &y)
+{
+    asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(a) : "memory");
+}
+__device__ __forceinline__ uint32_t sm_cas(uint32_t a, uint32_t old, uint32_t v)
+{
+    asm volatile("atom.shared.cas.b32 %0, [%1], %2, %3;" : "=r"(v) : "r"(a), "r"(old), "r"(v) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint64_t sm_cas(uint32_t a, uint64_t old, uint64_t v)
+{
+    asm volatile("atom.shared.cas.b64 %0, [%1], %2, %3;" : "=l"(v) : "r"(a), "l"(old), "l"(v) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sm_put(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ void sm_put(uint32_t a, uint64_t v) { asm volatile("st.shared.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory"); }
+__device__ __forceinline__ void sm_get(uint32_t a, uint32_t &v) { asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory"); }
+__device__ __forceinline__ void sm_get(uint32_t a, uint64_t &v) { asm volatile("ld.shared.u64 %0, [%1];" : "=l"(v) : "r"(a) : "memory"); }
+
+template <int ES>
+struct HistTable {
+    using K = word_t<ES>;
+    static constexpr K MARK = (K)0x8f1b5c37a4d96e21ull, MARK2 = (K)0xe3779a4d51c2b867ull;
+    static constexpr uint32_t KB = sizeof(K);
+    uint32_t keys, counts, queue;  // shared-memory addresses; the queue of this warp
+    uint32_t buckets;
+    __device__ __forceinline__ HistTable(const unsigned char *smem, uint32_t bytes)
+    {
+        const uint32_t table = bytes - (blockDim.x / 32) * kHistQueue * 8;
+        buckets = table / (2 * (KB + 4)) & ~1u;  // whole 16-byte pieces of either array
+        keys = (uint32_t)__cvta_generic_to_shared(smem);
+        counts = keys + 2 * buckets * KB;
+        queue = keys + table + (threadIdx.x / 32) * kHistQueue * 8;
     }
-    unsigned long long nan_min[4] = {EMPTY, EMPTY, EMPTY, EMPTY};
-    if (ES <= 4 && t0 < n) {
-        // values of up to 4 bytes: 32-bit keys and 16-bit counts (a tile holds at most
-        // kBHistTileMax = 32768 values, so a count never wraps), two counts a word, as many slots as
-        // the block's shared buffer holds (5456: a 32K tile of Zipf ids, 3,500-4,000 distinct
-        // values, leaves the table under 3/4 full, so few inserts run out of probes).  A value
-        // already in the table costs a plain key read and one 32-bit atomicAdd.  0xffffffff marks an
-        // empty slot, so that value itself is counted apart.  Each thread reads 16 consecutive bytes
-        // a round (one vector load), two rounds in flight before either is inserted; slots are
-        // chosen by a multiplicative hash scaled to the table.
-        constexpr uint32_t SL = kBHistSlots16;
-        static_assert(6 * SL <= 8 * kBHistPacked, "the table fits the shared buffer");
-        static_assert(kBHistTileMax <= 65535, "a 16-bit count holds a tile's values");
-        uint32_t *k32 = (uint32_t *)smem;
-        uint32_t *c16w = k32 + SL;
-        __shared__ uint32_t s_ones;
-        for (int i = threadIdx.x; i < (int)SL; i += kBThreads) k32[i] = 0xffffffffu;
-        for (int i = threadIdx.x; i < (int)SL / 2; i += kBThreads) c16w[i] = 0u;
-        if (threadIdx.x == 0) s_ones = 0;
-        __syncthreads();
-        const uint64_t end = n < t0 + HT ? n : t0 + HT;
-        constexpr int VPT = 16 / ES;
-        constexpr uint64_t R = (uint64_t)kBThreads * VPT;  // values of one round of the block
-        // a thread counts a run of equal values in registers and inserts the run once when the
-        // value changes (a constant or run-heavy column then costs a compare per value)
-        uint32_t run_key = 0, run_cnt = 0;
-        auto add = [&](uint32_t kk, uint32_t c) {
-            uint32_t h = (uint32_t)(((uint64_t)(kk * 0x9E3779B1u) * SL) >> 32);
-            for (int p = 0; p < 8; p++) {
-                uint32_t cur = ((volatile uint32_t *)k32)[h];
-                if (cur == 0xffffffffu) cur = atomicCAS(&k32[h], 0xffffffffu, kk);
-                if (cur == 0xffffffffu || cur == kk) {
-                    atomicAdd(&c16w[h >> 1], c << (16 * (h & 1)));
+    __device__ __forceinline__ uint32_t bucket(K v) const
+    {
+        uint32_t m = (uint32_t)v;
+        if (ES == 8) m ^= (uint32_t)((uint64_t)v >> 32);
+        return __umulhi(m * 0x9E3779B1u, buckets);  // multiplicative hash scaled to the buckets
+    }
+    __device__ __forceinline__ K mark(uint32_t b) const { return b == bucket(MARK) ? MARK2 : MARK; }
+    // v's count if its bucket holds it, else 0
+    __device__ __forceinline__ uint32_t find(K v) const
+    {
+        const uint32_t b = bucket(v);
+        K k0, k1;
+        sm_pair(keys + 2 * KB * b, k0, k1);
+        const uint32_t c = counts + 8 * b;
+        return k0 == v ? c : k1 == v ? c + 4 : 0u;
+    }
+};
+
+struct HistShared {
+    unsigned long long nan[4];  // the smallest NaN sort keys so far
+    uint32_t used;              // slots taken
+};
+static __shared__ HistShared s_hist;
+
+// c occurrences of a value that its bucket does not hold yet.  A full table takes no more keys: what
+// its bucket does not hold goes to the node's global table.
+template <int ES>
+__device__ __noinline__ void hist_insert(unsigned char *smem, uint32_t bytes, const BItem &it, word_t<ES> v, uint32_t c,
+                                         uint32_t *status)
+{
+    using T = HistTable<ES>;
+    const T h(smem, bytes);
+    if (v != T::MARK && v != T::MARK2) {
+        uint32_t b = h.bucket(v);
+        const int probes = *(volatile uint32_t *)&s_hist.used < h.buckets + h.buckets / 2 ? 4 : 1;
+        for (int p = 0; p < probes; p++) {
+            const typename T::K mark = h.mark(b);
+            typename T::K k[2];
+            sm_pair(h.keys + 2 * T::KB * b, k[0], k[1]);
+#pragma unroll
+            for (int w = 0; w < 2; w++) {
+                if (k[w] == mark) {
+                    k[w] = sm_cas(h.keys + T::KB * (2 * b + w), mark, v);
+                    if (k[w] == mark) {
+                        atomicAdd(&s_hist.used, 1u);
+                        k[w] = v;
+                    }
+                }
+                if (k[w] == v) {
+                    sm_add(h.counts + 4 * (2 * b + w), c);
                     return;
                 }
-                h = h + 1 == SL ? 0 : h + 1;
             }
-            g_insert(t, (unsigned long long)kk, c, status);
-        };
-        auto insert = [&](uint32_t kk, bool valid) {
-            if (!valid) return;
-            if (run_cnt && kk == run_key) {  // run_key is never a NaN or 0xffffffff
-                ++run_cnt;
-                return;
-            }
-            if (ES == 4 && is_nan_bits(kk, o)) {
-                unsigned long long k = order_key(kk, ES, o);
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (k < nan_min[j]) { const unsigned long long x = nan_min[j]; nan_min[j] = k; k = x; }
-                return;
-            }
-            if (kk == 0xffffffffu) {
-                atomicAdd(&s_ones, 1u);
-                return;
-            }
-            if (run_cnt) add(run_key, run_cnt);
-            run_key = kk;
-            run_cnt = 1;
-        };
-        const uint32_t lane = threadIdx.x & 31u;
-        const uint64_t wfirst = t0 + (uint64_t)(threadIdx.x - lane) * VPT;
-        for (uint64_t w0 = wfirst; w0 < end; w0 += 2 * R) {
-            const uint64_t b0 = w0 + (uint64_t)lane * VPT, b1 = b0 + R;
-            uint32_t u[2][VPT];
-            {
-                uint64_t v[VPT];
-                if (b0 < end) load_view_any<ES, VPT>(it, vc, in.ptr, b0, v);
-#pragma unroll
-                for (int j = 0; j < VPT; j++) u[0][j] = (uint32_t)v[j];
-                if (b1 < end) load_view_any<ES, VPT>(it, vc, in.ptr, b1, v);
-#pragma unroll
-                for (int j = 0; j < VPT; j++) u[1][j] = (uint32_t)v[j];
-            }
-#pragma unroll
-            for (int r = 0; r < 2; r++) {
-                const uint64_t base = r ? b1 : b0;
-                const uint32_t cnt = base >= end ? 0u : end - base < (uint64_t)VPT ? (uint32_t)(end - base) : VPT;
-#pragma unroll
-                for (int j = 0; j < VPT; j++) insert(u[r][j], (uint32_t)j < cnt);
-            }
-        }
-        if (run_cnt) add(run_key, run_cnt);
-        __syncthreads();
-        for (int i0 = threadIdx.x; i0 < (int)SL; i0 += 4 * kBThreads) {
-            unsigned long long k[4];
-            uint32_t c[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int i = i0 + j * kBThreads;
-                const uint32_t kk = i < (int)SL ? k32[i] : 0xffffffffu;
-                k[j] = kk;
-                c[j] = kk != 0xffffffffu ? (c16w[i >> 1] >> (16 * (i & 1))) & 0xffffu : 0u;
-            }
-            g_insert_many<4>(t, k, c, status);
-        }
-        if (threadIdx.x == 0 && s_ones) g_insert(t, 0xffffffffull, s_ones, status);
-    } else if (t0 < n) {
-        // 8-byte values: 64-bit keys, two values a round (one 16-byte load), two rounds in flight
-        for (int i = threadIdx.x; i < (int)kBHistSmem; i += kBThreads) {
-            skeys[i] = EMPTY;
-            scounts[i] = 0;
-        }
-        __syncthreads();
-        const uint64_t end = n < t0 + HT ? n : t0 + HT;
-        constexpr int VPT = 2;
-        constexpr uint64_t R = (uint64_t)kBThreads * VPT;
-        constexpr uint32_t HSH = 32 - 11;  // log2(kBHistSmem) = 11
-        static_assert(kBHistSmem == 2048, "the slot hash takes the top 11 bits");
-        const uint32_t lane = threadIdx.x & 31u;
-        unsigned long long run_key = 0;
-        uint32_t run_cnt = 0;
-        auto add = [&](unsigned long long key, uint32_t c) {
-            if (key != EMPTY) {
-                uint32_t h = ((uint32_t)(key ^ (key >> 32)) * 0x9E3779B1u) >> HSH;
-                for (int p = 0; p < 8; p++) {
-                    unsigned long long cur = ((volatile unsigned long long *)skeys)[h];
-                    if (cur == EMPTY) cur = atomicCAS(&skeys[h], EMPTY, key);
-                    if (cur == EMPTY || cur == key) {
-                        atomicAdd(&scounts[h], c);
-                        return;
-                    }
-                    h = (h + 1) & (kBHistSmem - 1);
-                }
-            }
-            g_insert(t, key, c, status);
-        };
-        auto insert = [&](unsigned long long key, bool valid) {
-            if (!valid) return;
-            if (run_cnt && key == run_key) {  // run_key is never a NaN
-                ++run_cnt;
-                return;
-            }
-            if (is_nan_bits(key, o)) {
-                unsigned long long k = order_key(key, ES, o);
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (k < nan_min[j]) { const unsigned long long x = nan_min[j]; nan_min[j] = k; k = x; }
-                return;
-            }
-            if (run_cnt) add(run_key, run_cnt);
-            run_key = key;
-            run_cnt = 1;
-        };
-        const uint64_t wfirst = t0 + (uint64_t)(threadIdx.x - lane) * VPT;
-        for (uint64_t w0 = wfirst; w0 < end; w0 += 2 * R) {
-            const uint64_t b0 = w0 + (uint64_t)lane * VPT, b1 = b0 + R;
-            uint64_t u[2][VPT];
-            if (b0 < end) load_view_any<ES, VPT>(it, vc, in.ptr, b0, u[0]);
-            if (b1 < end) load_view_any<ES, VPT>(it, vc, in.ptr, b1, u[1]);
-#pragma unroll
-            for (int r = 0; r < 2; r++) {
-                const uint64_t base = r ? b1 : b0;
-                const uint32_t cnt = base >= end ? 0u : end - base < (uint64_t)VPT ? (uint32_t)(end - base) : VPT;
-#pragma unroll
-                for (int j = 0; j < VPT; j++) insert(u[r][j], (uint32_t)j < cnt);
-            }
-        }
-        if (run_cnt) add(run_key, run_cnt);
-        __syncthreads();
-        for (int i0 = threadIdx.x; i0 < (int)kBHistSmem; i0 += 4 * kBThreads) {
-            unsigned long long k[4];
-            uint32_t c[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int i = i0 + j * kBThreads;
-                k[j] = i < (int)kBHistSmem ? skeys[i] : EMPTY;
-                c[j] = k[j] != EMPTY ? scounts[i] : 0u;
-            }
-            g_insert_many<4>(t, k, c, status);
+            b = b + 1 == h.buckets ? 0 : b + 1;
         }
     }
-    // this tile's 4 smallest NaN sort keys
-    for (int off = 16; off > 0; off >>= 1) {
-        unsigned long long other[4], merged[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) other[j] = __shfl_xor_sync(0xffffffffu, nan_min[j], off);
-        int a = 0, b2 = 0;
-#pragma unroll
-        for (int j = 0; j < 4; j++) merged[j] = (nan_min[a] <= other[b2]) ? nan_min[a++] : other[b2++];
-#pragma unroll
-        for (int j = 0; j < 4; j++) nan_min[j] = merged[j];
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0)
-        for (int j = 0; j < 4; j++) snan[warp][j] = nan_min[j];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long best[4] = {EMPTY, EMPTY, EMPTY, EMPTY};
-        for (int w = 0; w < kBThreads / 32; w++)
-            for (int j = 0; j < 4; j++) {
-                unsigned long long k = snan[w][j];
-                for (int q = 0; q < 4; q++)
-                    if (k < best[q]) { const unsigned long long x = best[q]; best[q] = k; k = x; }
-            }
-        for (int j = 0; j < 4; j++) t.nan[4 * tile + j] = best[j];
+    g_insert(htab(it), (unsigned long long)v, c, status);
+}
+
+// keeps the four smallest NaN sort keys: what a slot gives up moves on to the next
+__device__ __noinline__ void hist_nan(unsigned long long k)
+{
+    if (k >= *(volatile unsigned long long *)&s_hist.nan[3]) return;
+    for (int j = 0; j < 4; j++) {
+        const unsigned long long old = atomicMin(&s_hist.nan[j], k);
+        k = old > k ? old : k;
     }
 }
 
+// an empty table (all threads; barriers on both sides are the caller's)
+template <int ES>
+__device__ __forceinline__ void hist_clear(unsigned char *smem, uint32_t bytes)
+{
+    using T = HistTable<ES>;
+    const T h(smem, bytes);
+    constexpr uint32_t PER = 16 / T::KB;  // keys of a 16-byte piece
+    const uint32_t special = h.bucket(T::MARK), keys = 2 * h.buckets / PER, all = keys + 2 * h.buckets / 4;
+    uint4 *q = (uint4 *)smem;
+    constexpr uint64_t M = ES == 8 ? (uint64_t)T::MARK : (uint64_t)T::MARK << 32 | (uint64_t)T::MARK;
+    for (uint32_t i = threadIdx.x; i < all; i += blockDim.x)
+        q[i] = i < keys ? make_uint4((uint32_t)M, (uint32_t)(M >> 32), (uint32_t)M, (uint32_t)(M >> 32)) : make_uint4(0, 0, 0, 0);
+    // MARK's own bucket: by the thread that cleared it
+    if (threadIdx.x == special * 2 / PER % blockDim.x) {
+        sm_put(h.keys + 2 * T::KB * special, T::MARK2);
+        sm_put(h.keys + 2 * T::KB * special + T::KB, T::MARK2);
+    }
+    if (threadIdx.x < 4) s_hist.nan[threadIdx.x] = ~0ull;
+    if (threadIdx.x == 4) s_hist.used = 0;
+}
+
+// the table's counts to the node's global table, the NaN keys to `tile`'s list
+template <int ES>
+__device__ __forceinline__ void hist_flush(unsigned char *smem, uint32_t bytes, const BItem &it, uint32_t tile,
+                                           uint32_t *status)
+{
+    using T = HistTable<ES>;
+    const T h(smem, bytes);
+    const HTab t = htab(it);
+    const uint32_t slots = 2 * h.buckets;
+    for (uint32_t i0 = threadIdx.x; i0 < slots; i0 += 4 * blockDim.x) {
+        unsigned long long k[4];
+        uint32_t c[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const uint32_t i = i0 + j * blockDim.x;
+            typename T::K x = 0;
+            c[j] = 0;  // as an empty slot's
+            if (i < slots) {
+                sm_get(h.keys + T::KB * i, x);
+                sm_get(h.counts + 4 * i, c[j]);
+            }
+            k[j] = x;
+        }
+        g_insert_many<4>(t, k, c, status);
+    }
+    if (threadIdx.x < 4) t.nan[4ull * tile + threadIdx.x] = s_hist.nan[threadIdx.x];
+}
+
+// Counts the values of a tile in the block's table.  Issue-bound before (86 warp instructions per 32
+// values: one value at a time, each a probe loop in which the warp waits for its slowest lane); now a
+// thread takes 16 bytes of values a round, two rounds in flight, looks all of them up at once (one shared
+// load a value gives its bucket's two keys) and adds to the counts of those found.  The others go to
+// the warp's queue and are inserted 32 at a time, so that a row with one new value does not run the
+// insert for one lane.  A thread whose values are all equal adds them at once, a warp of one value
+// adds once.
+template <int ES>
+__device__ __forceinline__ void hist_tile(unsigned char *smem, uint32_t bytes, const BItem &it, uint32_t tile,
+                                          StreamDesc *S, uint32_t *status)
+{
+    using T = HistTable<ES>;
+    using K = typename T::K;
+    constexpr int N = 16 / ES;
+    const T h(smem, bytes);
+    const StreamDesc in = S[it.in[0]];
+    const ViewCtx vc = view_ctx<ES>(it, in);
+    const uint64_t n = vc.n, HT = it.p[3], t0 = (uint64_t)tile * HT;
+    const Order o = (Order)it.order;
+    if (t0 >= n) return;
+    const uint64_t end = n < t0 + HT ? n : t0 + HT;
+    auto insert = [&](K v, uint32_t c) {
+        if (is_nan_bits(v, o)) for (uint32_t q = 0; q < c && q < 4; q++) hist_nan(order_key(v, ES, o));
+        else hist_insert<ES>(smem, bytes, it, v, c, status);
+    };
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t step = (uint64_t)blockDim.x * N;
+    uint32_t queued = 0;  // values in the warp's queue (fewer than 32 between rows)
+    for (uint64_t w0 = t0 + (uint64_t)(threadIdx.x - lane) * N; w0 < end; w0 += 2 * step) {
+        K u[2][N];
+        const uint64_t b0 = w0 + lane * N, b1 = b0 + step;
+        if (b0 < end) load_vec<ES>(vc, in.ptr, b0, u[0]);
+        if (b1 < end) load_vec<ES>(vc, in.ptr, b1, u[1]);
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const uint64_t base = r ? b1 : b0;
+            const int cnt = base >= end ? 0 : end - base < (uint64_t)N ? (int)(end - base) : N;  // this lane's values
+            K(&v)[N] = u[r];
+            bool same = cnt == N;
+#pragma unroll
+            for (int q = 1; q < N; q++) same = same && v[q] == v[0];
+            if (__all_sync(0xffffffffu, same)) {
+                int one;
+                __match_all_sync(0xffffffffu, v[0], &one);
+                if (!one) {
+                    const uint32_t c = h.find(v[0]);
+                    if (c) sm_add(c, N);
+                    else insert(v[0], N);
+                } else if (lane == 0) {
+                    insert(v[0], 32 * N);
+                }
+                __syncwarp();
+                continue;
+            }
+            uint32_t count[N];
+#pragma unroll
+            for (int q = 0; q < N; q++) count[q] = h.find(v[q]);
+#pragma unroll
+            for (int q = 0; q < N; q++) {
+                const bool new_one = q < cnt && !count[q];
+                if (q < cnt && count[q]) sm_add(count[q], 1u);
+                const uint32_t m = __ballot_sync(0xffffffffu, new_one);
+                if (m) {
+                    if (new_one) sm_put(h.queue + T::KB * (queued + __popc(m & ((1u << lane) - 1))), v[q]);
+                    queued += __popc(m);
+                    __syncwarp();
+                    if (queued >= 32) {
+                        K x, rest;
+                        sm_get(h.queue + T::KB * lane, x);
+                        sm_get(h.queue + T::KB * (32 + lane), rest);
+                        insert(x, 1u);
+                        __syncwarp();
+                        queued -= 32;
+                        if (lane < queued) sm_put(h.queue + T::KB * lane, rest);
+                        __syncwarp();
+                    }
+                }
+            }
+        }
+    }
+    if (lane < queued) {
+        K x;
+        sm_get(h.queue + T::KB * lane, x);
+        insert(x, 1u);
+    }
+    __syncwarp();
+}
+
+// one tile on its own (the persistent schedule)
+template <int ES>
+__device__ __forceinline__ void p_hist(const BItem &it, uint32_t tile, StreamDesc *S, uint32_t *status, unsigned char *smem)
+{
+    hist_clear<ES>(smem, kBHistBytesPersist);
+    __syncthreads();
+    hist_tile<ES>(smem, kBHistBytesPersist, it, tile, S, status);
+    __syncthreads();
+    hist_flush<ES>(smem, kBHistBytesPersist, it, tile, status);
+}
+
+// elements of a compress pass's view
+__device__ __forceinline__ uint64_t view_len(const BItem &it, const StreamDesc *S)
+{
+    int nd = 0;
+    for (int k = 0; k < kMaxViewOps; k++) nd += it.vop[k] == V_DELTA;
+    const uint64_t n_src = S[it.in[0]].len / it.es;
+    return n_src > (uint64_t)nd ? n_src - nd : 0;
+}
+
+// The k most frequent values of an item.  A candidate is a count and a sort key (unique among the
+// table's values, so the bits follow from it); more occurrences first, then the smaller key.
 struct Cand {
-    unsigned long long key, bits;
-    unsigned int count;
+    unsigned long long key;
+    uint32_t count;  // 0 = none
 };
 __device__ __forceinline__ bool cbetter(const Cand &a, const Cand &b)
 {
     return a.count > b.count || (a.count == b.count && a.count != 0 && a.key < b.key);
 }
-__device__ __forceinline__ void cpush(Cand *l, const Cand &c)
+__device__ __forceinline__ void cpush(Cand (&l)[4], Cand c)
 {
-    if (!cbetter(c, l[3])) return;
-    l[3] = c;
 #pragma unroll
-    for (int i = 3; i > 0; i--)
-        if (cbetter(l[i], l[i - 1])) { const Cand x = l[i]; l[i] = l[i - 1]; l[i - 1] = x; }
+    for (int i = 0; i < 4; i++) {
+        const bool up = cbetter(c, l[i]);
+        const Cand x = l[i];
+        l[i] = up ? c : x;
+        c = up ? x : c;
+    }
 }
-
-// The k most frequent values of an item, then the table is cleared for the next step.  The item's
-// blocks (one per histogram tile) each take a slice of the used-slot list (and of the NaN lists),
-// reduce it to a top-4, clear their slots and write the top-4 to the partial list; the last block
-// to finish (threadfence + counter) merges the partials, writes the result and resets the header.
-__device__ __forceinline__ void topk_block_reduce(Cand *l, Cand *sc)
+// the four best of a warp's lists: candidate j in every lane's r[j]
+__device__ __forceinline__ void warp_top4(Cand (&l)[4], Cand (&r)[4])
 {
-    for (int j = 0; j < 4; j++) sc[threadIdx.x * 4 + j] = l[j];
-    __syncthreads();
-    for (int width = kBThreads / 2; width > 0; width >>= 1) {
-        if ((int)threadIdx.x < width) {
-            Cand mine[4] = {sc[threadIdx.x * 4], sc[threadIdx.x * 4 + 1], sc[threadIdx.x * 4 + 2], sc[threadIdx.x * 4 + 3]};
-            for (int j = 0; j < 4; j++) cpush(mine, sc[(threadIdx.x + width) * 4 + j]);
-            for (int j = 0; j < 4; j++) sc[threadIdx.x * 4 + j] = mine[j];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const uint32_t best = __reduce_max_sync(0xffffffffu, l[0].count);
+        bool in = l[0].count == best && best;
+        const uint32_t hi = __reduce_min_sync(0xffffffffu, in ? (uint32_t)(l[0].key >> 32) : ~0u);
+        in = in && (uint32_t)(l[0].key >> 32) == hi;
+        const uint32_t lo = __reduce_min_sync(0xffffffffu, in ? (uint32_t)l[0].key : ~0u);
+        in = in && (uint32_t)l[0].key == lo;
+        r[j] = Cand{(unsigned long long)hi << 32 | lo, best};
+        // equal candidates (NaNs) are taken one at a time
+        const unsigned who = __ballot_sync(0xffffffffu, in);
+        if (in && (threadIdx.x & 31) == (uint32_t)__ffs(who) - 1) {
+            l[0] = l[1];
+            l[1] = l[2];
+            l[2] = l[3];
+            l[3] = Cand{0, 0};
         }
-        __syncthreads();
+    }
+}
+// ... of a block's lists, in the first warp's lanes
+__device__ __forceinline__ void block_top4(Cand (&l)[4], Cand (&r)[4])
+{
+    __shared__ Cand s_c[kBThreads / 32 * 4];
+    warp_top4(l, r);
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        if (lane == (uint32_t)j) s_c[4 * warp + j] = r[j];
+    __syncthreads();
+    if (warp == 0) {
+        static_assert(kBThreads / 32 * 4 == 32, "one candidate a lane");
+        Cand m[4] = {s_c[lane], {0, 0}, {0, 0}, {0, 0}};
+        warp_top4(m, r);
     }
 }
 
+// The item's blocks that have work -- one per 2048 table slots taken and NaN keys listed -- each take a
+// slice of the used-slot list (and of the NaN lists), reduce it to a top-4, clear their slots for the
+// next step and write the top-4 to the partial list; the last one to finish (threadfence + counter)
+// merges the partials, writes the result and resets the header.
 template <int ES>
-__device__ void p_topk(const BItem &it, uint32_t tile, StreamDesc *S, unsigned char *smem)
+__device__ __forceinline__ void put_top(const BItem &it, StreamDesc *S, const Cand (&r)[4]);
+
+// block `tile` of `blocks`
+template <int ES>
+__device__ __forceinline__ void topk_blocks(const BItem &it, uint32_t tile, uint32_t blocks, StreamDesc *S)
 {
     constexpr unsigned long long EMPTY = ~0ull;
     __shared__ bool s_last;
-    Cand *sc = (Cand *)smem;
     const HTab t = htab(it);
     const Order o = (Order)it.order;
-    const uint32_t T = it.tiles;
-    const unsigned int used = t.hdr->used;
-    const uint64_t slice = (used + T - 1) / T;
+    const uint64_t used = *(volatile unsigned int *)&t.hdr->used, n = view_len(it, S), nan_n = 4 * ((n + it.p[3] - 1) / it.p[3]);
+    const uint64_t want = (used + nan_n + 2047) / 2048;
+    if (blocks > it.tiles) blocks = it.tiles;  // the partial list holds one entry a histogram tile
+    const uint32_t T = want > blocks ? blocks : want ? (uint32_t)want : 1u;
+    if (tile >= T) return;
+    const uint64_t slice = (used + T - 1) / T, nslice = (nan_n + T - 1) / T;
     const uint64_t lo = (uint64_t)tile * slice, hi = lo + slice < used ? lo + slice : used;
-    const uint64_t nan_n = 4 * it.p[1], nslice = (nan_n + T - 1) / T;
     const uint64_t nlo = (uint64_t)tile * nslice, nhi = nlo + nslice < nan_n ? nlo + nslice : nan_n;
-    Cand l[4];
-    for (int j = 0; j < 4; j++) l[j] = Cand{EMPTY, 0, 0};
-    for (uint64_t i = lo + threadIdx.x; i < hi; i += kBThreads) {
-        const unsigned int h = t.used[i];
-        const unsigned long long k = t.keys[h];
-        cpush(l, Cand{order_key(k, ES, o), k, t.counts[h]});
+    Cand l[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}}, r[4];
+    for (uint64_t i = lo + threadIdx.x; i < hi; i += 4 * kBThreads) {
+        unsigned int h[4], c[4];
+        unsigned long long k[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) h[q] = i + q * kBThreads < hi ? t.used[i + q * kBThreads] : 0u;
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (i + q * kBThreads < hi) {
+                k[q] = t.keys[h[q]];
+                c[q] = t.counts[h[q]];
+                t.keys[h[q]] = EMPTY;
+                t.counts[h[q]] = 0;
+            }
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (i + q * kBThreads < hi) cpush(l, Cand{order_key(k[q], ES, o), c[q]});
     }
-    if (tile == 0 && threadIdx.x == 0 && t.hdr->special) cpush(l, Cand{order_key(EMPTY, ES, o), EMPTY, t.hdr->special});
+    if (tile == 0 && threadIdx.x == 0 && t.hdr->special) cpush(l, Cand{order_key(EMPTY, ES, o), t.hdr->special});
     for (uint64_t i = nlo + threadIdx.x; i < nhi; i += kBThreads) {
         const unsigned long long k = t.nan[i];
-        if (k != EMPTY) cpush(l, Cand{k, order_unkey(k, ES, o), 1u});
+        if (k != EMPTY) cpush(l, Cand{k, 1u});
     }
-    topk_block_reduce(l, sc);
-    // clear this slice of the table for the next step
-    for (uint64_t i = lo + threadIdx.x; i < hi; i += kBThreads) {
-        const unsigned int h = t.used[i];
-        t.keys[h] = EMPTY;
-        t.counts[h] = 0;
+    block_top4(l, r);
+    if (T > 1) {
+        unsigned long long *part = t.part + (uint64_t)tile * 12;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (threadIdx.x == (uint32_t)j) {
+                part[3 * j] = r[j].key;
+                part[3 * j + 1] = r[j].count;
+            }
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) s_last = atomicAdd(&t.hdr->pad, 1u) == T - 1;
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+        Cand m[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
+        for (uint64_t i = threadIdx.x; i < 4ull * T; i += kBThreads) {
+            const volatile unsigned long long *q = t.part + 3 * i;
+            cpush(m, Cand{q[0], (uint32_t)q[1]});
+        }
+        block_top4(m, r);
     }
-    unsigned long long *part = t.part + (uint64_t)tile * 12;
-    if (threadIdx.x < 4) {
-        part[3 * threadIdx.x] = sc[threadIdx.x].key;
-        part[3 * threadIdx.x + 1] = sc[threadIdx.x].bits;
-        part[3 * threadIdx.x + 2] = sc[threadIdx.x].count;
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(&t.hdr->pad, 1u) == T - 1;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    for (int j = 0; j < 4; j++) l[j] = Cand{EMPTY, 0, 0};
-    for (uint64_t i = threadIdx.x; i < 4ull * T; i += kBThreads) {
-        const volatile unsigned long long *q = t.part + 3 * i;
-        cpush(l, Cand{q[0], q[1], (unsigned int)q[2]});
-    }
-    __syncthreads();
-    topk_block_reduce(l, sc);
     if (threadIdx.x == 0) {
-        const int k = it.mode;  // 1: const -> meta[0..es), 4: dict -> out1[16 ..)
-        uint8_t *dst = k == 1 ? S[it.out[0]].ptr : S[it.out[1]].ptr + 16;
-        for (int j = 0; j < k * ES; j++)  // bytes: a const node's metadata may start anywhere
-            dst[j] = (uint8_t)((sc[j / ES].count ? sc[j / ES].bits : 0ull) >> (8 * (j % ES)));
+        put_top<ES>(it, S, r);
         t.hdr->used = 0;
         t.hdr->special = 0;
         t.hdr->overflow = 0;
         t.hdr->pad = 0;
     }
 }
+
+// ------------------------------------------------------------------------------- candidates
+constexpr uint32_t kSampleSmem = 3072 * 12 + 4 * 512 + 4 * 64 + 16;
+// The most frequent values of a node, in most columns without a full histogram: a sample names up to
+// 128 candidates; one pass counts each candidate exactly and every other value in one of 4096 hash
+// buckets; a bucket's count bounds the count of each value in it, so when the least of the k best
+// candidates occurs more often than the largest bucket, those k are the most frequent ones, ties
+// included.  (A NaN never equals another: each occurs once, and the four smallest are candidates too.)
+// Where that proves nothing (values of nearly equal frequency), the item is flagged and the full
+// histogram below runs.  The counting pass has no inserts: one lookup and one addition a value.  It is
+// bound by issue and by the additions of equal values to one counter (14 % of the ids are one value).
+// 2^26 Zipf(1.1) ids: histogram and top-k 0.550 -> 0.165 ms, of which the counting pass 0.125 (2.1 TB/s;
+// 0.154 without the next rounds' loads in flight); the full histogram alone 0.287.  A tick table of 24
+// such columns of 2^20 values: 0.41 -> 0.29 ms.
+constexpr uint32_t kCandBuckets = kBCandSlots / 2;
+struct CandArea {
+    uint32_t *flag, *counts, *coarse;
+    unsigned long long *nan;  // the complements of the four smallest NaN sort keys, 0 = none
+    uint8_t *keys;
+    __device__ __forceinline__ CandArea(const BItem &it)
+    {
+        uint8_t *b = it.scratch + it.cand;
+        flag = (uint32_t *)b;
+        nan = (unsigned long long *)(b + 16);
+        counts = (uint32_t *)(b + 48);
+        coarse = counts + kBCandSlots;
+        keys = b + kBCandZero;
+    }
+};
+// the hash of a value: its top 9 bits are its candidate bucket, its top 12 its coarse bucket
+template <int ES>
+__device__ __forceinline__ uint32_t cand_hash(word_t<ES> v)
+{
+    uint32_t m = (uint32_t)v;
+    if (ES == 8) m = (m ^ (uint32_t)((uint64_t)v >> 32)) + (uint32_t)((uint64_t)v >> 45);
+    return m * 0x9E3779B1u;
+}
+static_assert(kCandBuckets == 1u << 9 && kBCandCoarse == 1u << 12, "cand_hash's bits");
+
+// One block an item: 2048 values spread over the column into a table in shared memory, the most
+// frequent of them (at least twice, unless all distinct ones fit) into the candidate table, the most
+// frequent first, as a bucket holds two.
+template <int ES>
+__device__ __forceinline__ void p_hist_sample(const BItem &it, StreamDesc *S, unsigned char *smem)
+{
+    using K = word_t<ES>;
+    using T = HistTable<ES>;
+    constexpr uint32_t SAMPLE = 2048, SLOTS = 3072, MOST = 128, HEAVY = 8;
+    static_assert(SAMPLE == 1u << 11 && SLOTS * 12 + 4 * kCandBuckets + 4 * 64 + 16 <= kSampleSmem, "the sample's shared memory");
+    K *keys = (K *)smem;
+    uint32_t *counts = (uint32_t *)(smem + SLOTS * 8), *fill = counts + SLOTS, *of_count = fill + kCandBuckets,
+             *least = of_count + 64;
+    const StreamDesc in = S[it.in[0]];
+    const ViewCtx vc = view_ctx<ES>(it, in);
+    const uint64_t n = vc.n;
+    const Order o = (Order)it.order;
+    for (uint32_t i = threadIdx.x; i < SLOTS; i += kBThreads) {
+        keys[i] = T::MARK;
+        counts[i] = 0;
+    }
+    for (uint32_t i = threadIdx.x; i < kCandBuckets + 64; i += kBThreads) fill[i] = 0;  // and of_count
+    __syncthreads();
+    constexpr int PER = SAMPLE / kBThreads;
+    K v[PER];
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const uint64_t i = threadIdx.x + j * kBThreads;
+        const uint64_t pos = n <= SAMPLE ? i : i * n >> 11;
+        v[j] = pos < n ? (K)view_elem<ES>(it, vc, in.ptr, pos) : T::MARK;
+    }
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const K x = v[j];
+        if (x == T::MARK || x == T::MARK2 || is_nan_bits(x, o)) continue;
+        uint32_t s = __umulhi(cand_hash<ES>(x), SLOTS);
+        for (;;) {  // more slots than values: ends
+            K cur = ((volatile K *)keys)[s];
+            if (cur == T::MARK) {
+                if constexpr (ES == 8) cur = atomicCAS((unsigned long long *)keys + s, (unsigned long long)T::MARK, (unsigned long long)x);
+                else cur = atomicCAS(keys + s, T::MARK, x);
+                if (cur == T::MARK) cur = x;
+            }
+            if (cur == x) {
+                atomicAdd(counts + s, 1u);
+                break;
+            }
+            s = s + 1 == SLOTS ? 0 : s + 1;
+        }
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < SLOTS; i += kBThreads)
+        if (counts[i]) atomicAdd(of_count + (counts[i] < 63 ? counts[i] : 63), 1u);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t sum = 0, c = 64;
+        while (c > 1 && sum + of_count[c - 1] <= MOST) sum += of_count[--c];
+        *least = c;  // the smallest count taken
+    }
+    __syncthreads();
+    const uint32_t t = *least;
+    const CandArea area(it);
+    K *image = (K *)area.keys;
+#pragma unroll 1
+    for (int pass = 0; pass < 2; pass++) {
+        for (uint32_t i = threadIdx.x; i < SLOTS; i += kBThreads) {
+            const uint32_t c = counts[i];
+            if (c < t || c == 0 || (c >= HEAVY) != (pass == 0)) continue;
+            const uint32_t b = cand_hash<ES>(keys[i]) >> 23, w = atomicAdd(fill + b, 1u);
+            if (w < 2) image[2 * b + w] = keys[i];
+        }
+        __syncthreads();
+    }
+    const uint32_t special = cand_hash<ES>(T::MARK) >> 23;
+    for (uint32_t b = threadIdx.x; b < kCandBuckets; b += kBThreads)
+        for (uint32_t w = fill[b]; w < 2; w++) image[2 * b + w] = b == special ? T::MARK2 : T::MARK;
+}
+
+// shared memory of the counting pass: keys, counts, coarse counts, a word a lane for the additions of
+// NaNs (unused), the smallest NaNs
+constexpr uint32_t kCandNan = 8 * kBCandSlots + 4 * (kBCandSlots + kBCandCoarse) + 4 * 32, kCandSmem = kCandNan + 32;
+
+// keeps the four largest of the nk given to it: what a place gives up moves on to the next
+__device__ __noinline__ void cand_nan(unsigned long long *nan, unsigned long long nk)
+{
+    if (nk <= *(volatile unsigned long long *)(nan + 3)) return;
+    for (int j = 0; j < 4; j++) {
+        const unsigned long long old = atomicMax(nan + j, nk);
+        nk = old < nk ? old : nk;
+    }
+}
+
+template <int ES>
+__device__ __forceinline__ void cand_load(const BItem &it, unsigned char *smem)
+{
+    const CandArea area(it);
+    constexpr uint32_t KW = kBCandSlots * sizeof(word_t<ES>) / 16, CW = (kCandSmem - 8 * kBCandSlots) / 16;
+    for (uint32_t i = threadIdx.x; i < KW; i += blockDim.x) ((uint4 *)smem)[i] = ldg((const uint4 *)area.keys + i);
+    for (uint32_t i = threadIdx.x; i < CW; i += blockDim.x) ((uint4 *)(smem + 8 * kBCandSlots))[i] = make_uint4(0, 0, 0, 0);
+}
+__device__ __forceinline__ void cand_flush(const BItem &it, const unsigned char *smem)
+{
+    const CandArea area(it);
+    const uint32_t *c = (const uint32_t *)(smem + 8 * kBCandSlots);
+    for (uint32_t i = threadIdx.x; i < kBCandSlots + kBCandCoarse; i += blockDim.x)
+        if (c[i]) atomicAdd(area.counts + i, c[i]);  // coarse follows counts
+    const unsigned long long *nan = (const unsigned long long *)(smem + kCandNan);
+    if (threadIdx.x < 4 && nan[threadIdx.x]) cand_nan(area.nan, nan[threadIdx.x]);
+}
+
+// A tile of the counting pass (n * s read).
+template <int ES, bool FP>
+__device__ __forceinline__ void cand_tile_of(const BItem &it, uint32_t tile, StreamDesc *S, unsigned char *smem)
+{
+    using K = word_t<ES>;
+    constexpr int N = 16 / ES;
+    const StreamDesc in = S[it.in[0]];
+    const ViewCtx vc = view_ctx<ES>(it, in);
+    const uint64_t n = vc.n, HT = it.p[3], t0 = (uint64_t)tile * HT;
+    if (t0 >= n) return;
+    const uint64_t end = n < t0 + HT ? n : t0 + HT;
+    if (it.mode == 4) {
+        // dict: clear this tile's share of the 2-bit code words (out1 after its 16 + 4*es header)
+        uint32_t *words = (uint32_t *)(S[it.out[1]].ptr + 16 + 4 * ES);
+        for (uint64_t w = t0 / 16 + threadIdx.x; w < (end + 15) / 16; w += blockDim.x) words[w] = 0u;
+    }
+    const uint32_t keys = (uint32_t)__cvta_generic_to_shared(smem), counts = keys + 8 * kBCandSlots;
+    const uint32_t lane = threadIdx.x & 31;
+    constexpr Order FO = ES == 8 ? ORD_F64 : ORD_F32;
+    auto place = [&](K v) -> uint32_t {  // the address of v's counter
+        const uint32_t h = cand_hash<ES>(v), b = h >> 23;
+        K k0, k1;
+        sm_pair(keys + 2 * sizeof(K) * b, k0, k1);
+        const uint32_t c = counts + 8 * b;
+        const uint32_t a = k0 == v ? c : k1 == v ? c + 4 : counts + 4 * kBCandSlots + 4 * (h >> 20);
+        return FP && is_nan_bits(v, FO) ? counts + 4 * (kBCandSlots + kBCandCoarse) + 4 * lane : a;
+    };
+    auto nans = [&](K v, uint32_t c) {  // c occurrences of v, if it is a NaN
+        if (FP && is_nan_bits(v, FO))
+            for (uint32_t q = 0; q < c && q < 4; q++)
+                cand_nan((unsigned long long *)(smem + kCandNan), ~(unsigned long long)order_key(v, ES, FO));
+    };
+    const uint64_t step = (uint64_t)blockDim.x * N;
+    // two rounds' loads are in flight while two are counted (fewer for narrow types: registers)
+    constexpr int R = ES == 1 ? 1 : 2;
+    K u[R][N], next[R][N];
+    uint64_t w0 = t0 + (uint64_t)(threadIdx.x - lane) * N;
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        if (w0 + lane * N + r * step < end) load_vec<ES>(vc, in.ptr, w0 + lane * N + r * step, next[r]);
+    for (; w0 < end; w0 += R * step) {
+        const uint64_t b0 = w0 + lane * N;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+#pragma unroll
+            for (int q = 0; q < N; q++) u[r][q] = next[r][q];
+            const uint64_t b = b0 + (R + r) * step;
+            if (b < end) load_vec<ES>(vc, in.ptr, b, next[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const uint64_t base = b0 + r * step;
+            const int cnt = base >= end ? 0 : end - base < (uint64_t)N ? (int)(end - base) : N;  // this lane's values
+            K(&v)[N] = u[r];
+            bool same = cnt == N;
+#pragma unroll
+            for (int q = 1; q < N; q++) same = same && v[q] == v[0];
+            if (__all_sync(0xffffffffu, same)) {  // runs: one addition a thread, or a warp
+                int one;
+                __match_all_sync(0xffffffffu, v[0], &one);
+                if (!one || lane == 0) {
+                    sm_add(place(v[0]), one ? 32 * N : N);
+                    nans(v[0], one ? 32 * N : N);
+                }
+                continue;
+            }
+            uint32_t at[N];
+#pragma unroll
+            for (int q = 0; q < N; q++) at[q] = place(v[q]);
+#pragma unroll
+            for (int q = 0; q < N; q++)
+                if (q < cnt) sm_add(at[q], 1u);
+            if (FP) {
+#pragma unroll
+                for (int q = 0; q < N; q++)
+                    if (q < cnt) nans(v[q], 1u);
+            }
+        }
+    }
+}
+
+template <int ES>
+__device__ __forceinline__ void cand_tile(const BItem &it, uint32_t tile, StreamDesc *S, unsigned char *smem)
+{
+    if (ES >= 4 && it.order != ORD_INT) cand_tile_of<ES, (ES >= 4)>(it, tile, S, smem);
+    else cand_tile_of<ES, false>(it, tile, S, smem);
+}
+
+// one tile on its own (the persistent schedule)
+template <int ES>
+__device__ __forceinline__ void p_hist_count(const BItem &it, uint32_t tile, StreamDesc *S, unsigned char *smem)
+{
+    if ((uint64_t)tile * it.p[3] >= view_len(it, S)) return;
+    cand_load<ES>(it, smem);
+    __syncthreads();
+    cand_tile<ES>(it, tile, S, smem);
+    __syncthreads();
+    cand_flush(it, smem);
+}
+
+// the k most frequent values to where the split reads them: dict after out1's 16-byte header, const at
+// the start of its metadata (which may lie anywhere: bytes)
+template <int ES>
+__device__ __forceinline__ void put_top(const BItem &it, StreamDesc *S, const Cand (&r)[4])
+{
+    const Order o = (Order)it.order;
+    const int k = it.mode;
+    uint8_t *dst = k == 1 ? S[it.out[0]].ptr : S[it.out[1]].ptr + 16;
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        if (j < k) {
+            const uint64_t v = r[j].count ? order_unkey(r[j].key, ES, o) : 0ull;
+            for (int b = 0; b < ES; b++) dst[j * ES + b] = (uint8_t)(v >> (8 * b));
+        }
+}
+
+// one block an item: the k best candidates, or the flag
+template <int ES>
+__device__ __forceinline__ void p_cand_top(const BItem &it, StreamDesc *S)
+{
+    __shared__ uint32_t s_max;
+    const CandArea area(it);
+    const Order o = (Order)it.order;
+    if (threadIdx.x == 0) s_max = 0;
+    __syncthreads();
+    constexpr int PER = (int)(kBCandSlots / kBThreads), COARSE = (int)(kBCandCoarse / kBThreads / 4);
+    uint32_t c[PER], most = 0;
+    word_t<ES> k[PER];
+    uint4 g[COARSE];
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const uint32_t i = threadIdx.x + j * kBThreads;
+        c[j] = ldg(area.counts + i);
+        k[j] = ldg((const word_t<ES> *)area.keys + i);
+    }
+#pragma unroll
+    for (int j = 0; j < COARSE; j++) g[j] = ldg((const uint4 *)area.coarse + threadIdx.x + j * kBThreads);
+    Cand l[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}}, r[4];
+#pragma unroll
+    for (int j = 0; j < COARSE; j++) most = max(max(most, max(g[j].x, g[j].y)), max(g[j].z, g[j].w));
+#pragma unroll
+    for (int j = 0; j < PER; j++)
+        if (c[j]) cpush(l, Cand{order_key(k[j], ES, o), c[j]});
+    if (threadIdx.x < 4 && area.nan[threadIdx.x]) cpush(l, Cand{~area.nan[threadIdx.x], 1u});
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_max, most);
+    block_top4(l, r);  // its barriers publish s_max
+    if (threadIdx.x == 0) {
+        const uint32_t least = it.mode == 1 ? r[0].count : r[3].count;
+        if (s_max == 0 || s_max < least) put_top<ES>(it, S, r);
+        else *area.flag = 1;
+    }
+}
+
+#ifndef GTSC_PERSISTENT_TU
+template <class F>
+__device__ __forceinline__ void each_size(int es, F f)
+{
+    switch (es) {
+    case 1: f(std::integral_constant<int, 1>()); break;
+    case 2: f(std::integral_constant<int, 2>()); break;
+    case 4: f(std::integral_constant<int, 4>()); break;
+    default: f(std::integral_constant<int, 8>()); break;
+    }
+}
+
+// The counting pass's stage launch: as many blocks as are resident, striding over the tiles; a block
+// keeps its counters while its tiles are of one item.
+__global__ void __launch_bounds__(kBThreads, 4)
+k_bcount(const BItem *items, const uint32_t *item_of, StreamDesc *S, uint32_t total_tiles)
+{
+    __shared__ __align__(16) unsigned char smem[kCandSmem];
+    constexpr uint32_t NONE = 0xffffffffu;
+    uint32_t t = blockIdx.x, cur = NONE;
+    while (t < total_tiles) {
+        const uint32_t k = item_of[t];
+        if (k != cur) {
+            __syncthreads();  // the counters are complete, nobody reads the previous descriptor any more
+            if (cur != NONE) cand_flush(shared_item_ref(), smem);
+            __syncthreads();
+            shared_item(items, k);
+            each_size(shared_item_ref().es, [&](auto es) { cand_load<decltype(es)::value>(shared_item_ref(), smem); });
+            __syncthreads();
+            cur = k;
+        }
+        const BItem &it = shared_item_ref();
+        const uint32_t tile = t - (uint32_t)it.tile_base;
+        if ((uint64_t)tile * it.p[3] >= view_len(it, S)) {
+            const uint64_t next = it.tile_base + it.tiles;  // the next item's first tile
+            if (next >= total_tiles) break;
+            t = (uint32_t)(next + (blockIdx.x + gridDim.x - next % gridDim.x) % gridDim.x);
+            continue;
+        }
+        each_size(it.es, [&](auto es) { cand_tile<decltype(es)::value>(shared_item_ref(), tile, S, smem); });
+        t += gridDim.x;
+    }
+    __syncthreads();
+    if (cur != NONE) cand_flush(shared_item_ref(), smem);
+}
+
+// The items of a launch whose flag is set, in order, f(index) for each; the block's threads look at 256
+// or more of them at a time.
+template <class F>
+__device__ __forceinline__ void flagged_items(const BItem *items, int n_items, F f)
+{
+    __shared__ uint32_t s_mask[32];
+    for (int i0 = 0; i0 < n_items; i0 += blockDim.x) {
+        const int i = i0 + threadIdx.x;
+        const bool on = i < n_items && *CandArea(items[i]).flag != 0;
+        const uint32_t m = __ballot_sync(0xffffffffu, on);
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0) s_mask[threadIdx.x >> 5] = m;
+        if (!__syncthreads_or(on)) continue;
+        for (uint32_t w = 0; w < blockDim.x / 32; w++)
+            for (uint32_t rest = s_mask[w]; rest; rest &= rest - 1) f(i0 + 32 * w + __ffs(rest) - 1);
+        __syncthreads();
+    }
+}
+
+// The full histogram's stage launch, over the flagged items: as many blocks as are resident, striding
+// over an item's tiles.  A block keeps its table while it is at most half full.
+__global__ void __launch_bounds__(kBHistThreads, 2)
+k_bhist(const BItem *items, int n_items, StreamDesc *S, uint32_t *status)
+{
+    extern __shared__ __align__(16) unsigned char table[];
+    flagged_items(items, n_items, [&](int k) {
+        __syncthreads();
+        const BItem &it = shared_item(items, k);
+        each_size(it.es, [&](auto es) {
+            constexpr int E = decltype(es)::value;
+            const uint64_t n = view_len(it, S), tiles = (n + it.p[3] - 1) / it.p[3];
+            bool dirty = false;  // the table holds counts, up to tile `last`
+            uint32_t last = 0;
+            for (uint64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+                if (dirty) {  // the tile before went into this table too: its NaN keys are listed with this one's
+                    if (threadIdx.x < 4) htab(it).nan[4ull * last + threadIdx.x] = ~0ull;
+                } else {
+                    hist_clear<E>(table, kBHistBytes);
+                    __syncthreads();
+                }
+                hist_tile<E>(table, kBHistBytes, it, (uint32_t)t, S, status);
+                last = (uint32_t)t;
+                dirty = true;
+                // one decision for the block: the threads' reads lie before the barrier
+                const uint32_t used = *(volatile uint32_t *)&s_hist.used;
+                if (__syncthreads_or(used > (E == 8 ? kBHistBytes / 24 : kBHistBytes / 16))) {
+                    hist_flush<E>(table, kBHistBytes, it, last, status);
+                    dirty = false;
+                    __syncthreads();
+                }
+            }
+            if (dirty) hist_flush<E>(table, kBHistBytes, it, last, status);
+        });
+    });
+}
+
+__global__ void __launch_bounds__(kBThreads, 4) k_btopk(const BItem *items, int n_items, StreamDesc *S)
+{
+    flagged_items(items, n_items, [&](int k) {
+        __syncthreads();
+        const BItem &it = shared_item(items, k);
+        each_size(it.es, [&](auto es) { topk_blocks<decltype(es)::value>(it, blockIdx.x, gridDim.x, S); });
+    });
+}
+#endif
 
 // ------------------------------------------------------------------------------- split
 // the outside variant of patch, beside SplitMode
@@ -1584,8 +2096,9 @@ __device__ void p_vmeta(const BItem &it, StreamDesc *S)
 constexpr size_t stage_smem(int op)
 {
     return op == B_AFL_PACK ? 8 * (kBTile + kBTile / 16 + 8)
-         : op == B_HIST     ? 8 * kBHistPacked + 8 * 4 * (kBThreads / 32)
-         : op == B_TOPK     ? sizeof(Cand) * kBThreads * 4
+         : op == B_HIST     ? kCandSmem
+         : op == B_HIST_SAMPLE ? kSampleSmem
+         : op == B_HIST_FULL ? kBHistBytesPersist
          : op == B_SPLIT    ? kSplitCodes * (kBThreads / 32)  // a dictionary's codes, a byte each
          : op == B_RLE_HEADS ? kXchgBlockBytes
          : op == B_GFC_COMPRESS ? kGfcStage * (kBThreads / 32)
@@ -1700,8 +2213,14 @@ __device__ __forceinline__ void run_stage(const BItem &it, uint32_t tile, Stream
     else if constexpr (OP == B_DELTA_ENC) { GTSC_ES_SWITCH(p_delta_enc<E>(it, tile, S)) }
     else if constexpr (OP == B_SCALE_SUB) { GTSC_ES_SWITCH(p_scale_sub<E>(it, tile, S)) }
     else if constexpr (OP == B_AFL_PACK) { GTSC_ES_SWITCH(p_afl_pack<E>(it, tile, S, (unsigned long long *)smem)) }
-    else if constexpr (OP == B_HIST) { GTSC_ES_SWITCH(p_hist<E>(it, tile, S, status, smem)) }
-    else if constexpr (OP == B_TOPK) { GTSC_ES_SWITCH(p_topk<E>(it, tile, S, smem)) }
+    else if constexpr (OP == B_HIST_SAMPLE) { GTSC_ES_SWITCH(p_hist_sample<E>(it, S, smem)) }
+    else if constexpr (OP == B_HIST) { GTSC_ES_SWITCH(p_hist_count<E>(it, tile, S, smem)) }
+    else if constexpr (OP == B_TOPK) { GTSC_ES_SWITCH(p_cand_top<E>(it, S)) }
+    else if constexpr (OP == B_HIST_FULL) {
+        if (*CandArea(it).flag) { GTSC_ES_SWITCH(p_hist<E>(it, tile, S, status, smem)) }
+    } else if constexpr (OP == B_TOPK_FULL) {
+        if (*CandArea(it).flag) { GTSC_ES_SWITCH(topk_blocks<E>(it, tile, it.tiles, S)) }
+    }
     else if constexpr (OP == B_VMETA) { GTSC_ES_SWITCH(p_vmeta<E>(it, S)) }
     else if constexpr (OP == B_SPLIT_COUNT) { p_split_count(it, tile, S); }
     else if constexpr (OP == B_SPLIT) { GTSC_ES_SWITCH(p_split<E>(it, tile, S, smem)) }
@@ -1727,7 +2246,7 @@ __device__ __forceinline__ void run_stage(const BItem &it, uint32_t tile, Stream
 constexpr size_t persist_smem_c()
 {
     size_t m = 16;
-    for (int op = 0; op <= B_GFC_COMPACT; op++) m = stage_smem(op) > m ? stage_smem(op) : m;
+    for (int op = 0; op < B_NUM_OPS; op++) m = stage_smem(op) > m ? stage_smem(op) : m;
     return m;
 }
 
@@ -1764,8 +2283,11 @@ __global__ void __launch_bounds__(kBThreads, 4) k_bpersist_c(PersistArgs a)
             GTSC_RUN(B_DELTA_ENC)
             GTSC_RUN(B_SCALE_SUB)
             GTSC_RUN(B_AFL_PACK)
+            GTSC_RUN(B_HIST_SAMPLE)
             GTSC_RUN(B_HIST)
             GTSC_RUN(B_TOPK)
+            GTSC_RUN(B_HIST_FULL)
+            GTSC_RUN(B_TOPK_FULL)
             GTSC_RUN(B_SPLIT_COUNT)
             GTSC_RUN(B_SPLIT)
             GTSC_RUN(B_RLE_HEADS)
@@ -1834,7 +2356,28 @@ void launch_batch_stage(int op, const BItem *d_items, const uint32_t *d_item_of,
         GTSC_STAGE(B_DELTA_ENC)
         GTSC_STAGE(B_SCALE_SUB)
         GTSC_STAGE(B_AFL_PACK)
-        GTSC_STAGE(B_HIST)
+        GTSC_STAGE(B_HIST_SAMPLE)
+    case B_HIST: {
+        int per_sm = 0;
+        GTSC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bcount, kBThreads, 0));
+        const uint64_t resident = (uint64_t)std::max(per_sm, 1) * (uint64_t)sm_count();
+        k_bcount<<<(unsigned)std::min<uint64_t>(total_tiles, resident), kBThreads, 0, s>>>(d_items, d_item_of, d_streams,
+                                                                                        (uint32_t)total_tiles);
+        break;
+    }
+    case B_HIST_FULL: {
+        GTSC_CUDA(cudaFuncSetAttribute(k_bhist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBHistBytes));
+        int per_sm = 0;
+        GTSC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bhist, (int)kBHistThreads, kBHistBytes));
+        const uint64_t resident = (uint64_t)std::max(per_sm, 1) * (uint64_t)sm_count();
+        k_bhist<<<(unsigned)std::min<uint64_t>(total_tiles, resident), kBHistThreads, kBHistBytes, s>>>(
+            d_items, n_items, d_streams, d_status);
+        break;
+    }
+    case B_TOPK_FULL:
+        k_btopk<<<(unsigned)std::min<uint64_t>(total_tiles, 4 * (uint64_t)sm_count()), kBThreads, 0, s>>>(d_items, n_items,
+                                                                                                        d_streams);
+        break;
         GTSC_STAGE(B_TOPK)
         GTSC_STAGE(B_SPLIT_COUNT)
         GTSC_STAGE(B_SPLIT)

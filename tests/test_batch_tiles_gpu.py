@@ -54,3 +54,41 @@ def test_split_and_merge_through_views(G, O, rng, dt, path):
             dts.append(dt)
             trees.append(G.tree_from_path(path, dt))
     run_batch(G, O, cols, dts, trees)
+
+
+def frequent(rng, kind, n, npt):
+    """columns whose most frequent values are hard to tell: equal (many values of one frequency), unique,
+    few (fewer than four), marks (the values that the histogram tables use as empty marks), nans (float:
+    NaNs of many payloads beside three values, so that one of them is the fourth)"""
+    bits = {1: np.uint8, 2: np.uint16, 4: np.uint32, 8: np.uint64}[np.dtype(npt).itemsize]
+    if kind == "equal":
+        return (np.arange(n) % 300).astype(npt)
+    if kind == "unique":
+        return rng.permutation(n).astype(npt)
+    if kind == "few":
+        return rng.choice([7, 9], n).astype(npt)
+    if kind == "marks":
+        marks = np.array([0x8f1b5c37a4d96e21, 0xe3779a4d51c2b867, 0xffffffffffffffff, 0, 5], np.uint64)
+        with np.errstate(over="ignore"):
+            return marks.astype(bits)[rng.choice(5, n, p=[.3, .25, .2, .15, .1])].view(npt)
+    x = rng.choice([1, 2, 4], n).astype(npt)
+    if np.issubdtype(npt, np.floating):
+        pos = rng.random(n) < 0.4
+        exp, man = (0x7ff << 52, 52) if bits is np.uint64 else (0xff << 23, 23)
+        pay = rng.integers(1, 1 << man, n, dtype=np.uint64) | np.uint64(exp)
+        sign = rng.integers(0, 2, n, dtype=np.uint64) << np.uint64(8 * np.dtype(npt).itemsize - 1)
+        x.view(bits)[pos] = (pay | sign)[pos].astype(bits)
+    return x
+
+
+@pytest.mark.parametrize("dt", list(IDS), ids=list(IDS.values()))
+def test_most_frequent_values(G, O, rng, dt):
+    """dictionary and const nodes: candidates proven by the bounds, and the full histogram where not"""
+    cols, dts, trees = [], [], []
+    for n in [3, 2047, 2048, 2049, 4097, 40001, 300001]:
+        for kind in ["equal", "unique", "few", "marks", "nans"]:
+            for path in [[OR.DICT, OR.NONE, OR.NONE], [OR.CONST, OR.NONE]]:
+                cols.append(frequent(rng, kind, n, OR.NP_TYPES[dt]))
+                dts.append(dt)
+                trees.append(G.tree_from_path(path, dt))
+    run_batch(G, O, cols, dts, trees, steps=2)
