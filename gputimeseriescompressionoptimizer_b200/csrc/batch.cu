@@ -99,9 +99,11 @@ struct Launch {
 // passes whose tiles chain through a decoupled look-back (claimed in order from a counter)
 bool dyn_pass(int op)
 {
-    return op == B_RLE_HEADS || op == B_GFC_SCAN || op == B_DELTA_DEC || op == B_RLE_SCAN ||
-           op == B_MERGE_COUNT;
+    return op == B_RLE_HEADS || op == B_GFC_SCAN || op == B_RLE_SCAN || op == B_MERGE_COUNT;
 }
+
+// blocks of the passes of a delta decode of n elements
+uint64_t delta_tiles(uint64_t n) { return std::max<uint64_t>(1, cdiv(n, kBDeltaTile)); }
 
 // blocks of the counting pass of a merge over n elements
 uint64_t merge_count_tiles(uint64_t n) { return std::max<uint64_t>(1, cdiv(n, kBCountTile)); }
@@ -339,7 +341,7 @@ void BatchEngine::plan_passes()
         switch (nd.enc) {
         case GTSC_DELTA:
             nd.dlb_off = nd.c_bytes;
-            d = align_up(lookback_bytes(tiles), 256);
+            d = align_up(bdelta_bytes(delta_tiles(n)), 256);
             break;
         case GTSC_PATCH: case GTSC_PATCH_OUTSIDE: case GTSC_DICT: case GTSC_CONST:
             nd.dlb_off = nd.c_bytes;
@@ -590,7 +592,7 @@ void BatchEngine::plan_passes()
             for (size_t j = 0; j < nd.kids.size() && j < 2; j++) it.in[j + 1] = child_out((int)j);
             it.out[0] = nd.dec_out_sid;
             // the passes that read their children element-wise take them through DViews
-            if (op == B_DELTA_DEC || op == B_SCALE_ADD || op == B_MERGE || op == B_RLE_SCAN || op == B_RLE_EXPAND ||
+            if (op == B_DELTA_SUM || op == B_SCALE_ADD || op == B_MERGE || op == B_RLE_SCAN || op == B_RLE_EXPAND ||
                 op == B_F2I_DEC)
                 for (size_t j = 0; j < nd.kids.size() && j < 2; j++) it.dv[j] = nodes[nd.kids[j]].dview;
             return it;
@@ -605,7 +607,14 @@ void BatchEngine::plan_passes()
             }
             break;
         case GTSC_AFL: ps.push_back(ditem(B_AFL_UNPACK, t2k)); break;
-        case GTSC_DELTA: { BItem it = ditem(B_DELTA_DEC, t2k); it.p[0] = nd.dlb_off; ps.push_back(it); break; }
+        case GTSC_DELTA: {
+            BItem it = ditem(B_DELTA_SUM, delta_tiles(n));
+            it.p[0] = nd.dlb_off;
+            ps.push_back(it);
+            it.op = B_DELTA_DEC;
+            ps.push_back(it);
+            break;
+        }
         case GTSC_SCALE: ps.push_back(ditem(B_SCALE_ADD, t2k)); break;
         case GTSC_PATCH: case GTSC_PATCH_OUTSIDE: case GTSC_DICT: case GTSC_CONST: {
             BItem it = ditem(B_MERGE, cdiv(n, kBMergeTile));
@@ -724,7 +733,7 @@ void BatchEngine::layout(cudaStream_t s)
                 if (ps[j].op == B_SPLIT_COUNT)  // the children whose min / max the split accumulates
                     for (int q = 2; q < 4; q++)
                         it.p[q] = it.p[q] ? (uint64_t)(uintptr_t)(A + nodes[it.p[q] - 1].scratch) : 0;
-                if (ps[j].op < B_NONE_COPY || ps[j].op == B_VMETA || ps[j].op >= B_SPLIT_COUNT)  // compress: the view's scale nodes
+                if (ps[j].op < B_NONE_COPY || ps[j].op == B_VMETA || (ps[j].op >= B_SPLIT_COUNT && ps[j].op <= B_TOPK_FULL))  // compress: the view's scale nodes
                     for (int v = 0; v < kMaxViewOps; v++) {
                         const int sn = nodes[ps[j].node].vnode[v];
                         it.vscr[v] = sn >= 0 ? A + nodes[sn].scratch : nullptr;
@@ -783,7 +792,8 @@ void BatchEngine::layout(cudaStream_t s)
         const uint64_t n = nd.in_cap / nd.es;
         const uint64_t t2k = std::max<uint64_t>(1, cdiv(n, kBTile));
         switch (nd.enc) {
-        case GTSC_DELTA: case GTSC_RLE: zr(zero_d, sc + nd.dlb_off, lookback_zero_bytes(t2k)); break;
+        case GTSC_DELTA: zr(zero_d, sc + nd.dlb_off, 8 * bdelta_groups(delta_tiles(n))); break;
+        case GTSC_RLE: zr(zero_d, sc + nd.dlb_off, lookback_zero_bytes(t2k)); break;
         case GTSC_PATCH: case GTSC_PATCH_OUTSIDE: case GTSC_DICT: case GTSC_CONST:
             zr(zero_d, sc + nd.dlb_off, lookback_zero_bytes(merge_count_tiles(n)));
             break;
@@ -1274,6 +1284,7 @@ static uint64_t item_bytes(const BItem &it, const std::vector<StreamDesc> &S)
     case B_GFC_COMPACT: return 2 * L(it.out[2]);
     case B_NONE_COPY: return 2 * in;
     case B_AFL_UNPACK: return L(it.in[1]) + L(it.out[0]);
+    case B_DELTA_SUM: return D(1);
     case B_DELTA_DEC: case B_SCALE_ADD: case B_F2I_DEC: return D(1) + L(it.out[0]);
     case B_MERGE: return in + (it.mode == SPLIT_DICT ? L(it.in[1]) : D(1)) + D(2) + L(it.out[0]);
     case B_RLE_SCAN: return D(1);

@@ -47,6 +47,7 @@ enum BOp : int {
     B_HIST_SAMPLE,     // compress: dict / const: the candidates, from a sample
     B_HIST_FULL,       // compress: dict / const: the full histogram, where the bounds prove nothing
     B_TOPK_FULL,       // compress: its most frequent values
+    B_DELTA_SUM,       // decode: sums of the differences of every unit
     B_NUM_OPS
 };
 
@@ -252,6 +253,12 @@ constexpr uint32_t kBCountTile = 128 * kBMergeUnit;  // ... of a block of the co
 constexpr uint32_t kBSplitUnit = 1024;  // split: values of a warp's unit (32 rows of 32)
 constexpr uint32_t kBSplitTile = 8 * kBSplitUnit;    // ... of a block
 constexpr uint32_t kBSplitGroup = 64;                // tiles whose matches are summed together
+
+constexpr uint32_t kBDeltaUnit = 1024, kBDeltaTile = 8 * kBDeltaUnit, kBDeltaGroup = 64;  // delta decode, alike
+
+// scratch of a delta decode: sums (u64) of the groups, the tiles and the units
+__host__ __device__ inline uint64_t bdelta_groups(uint64_t tiles) { return (tiles + kBDeltaGroup - 1) / kBDeltaGroup; }
+inline uint64_t bdelta_bytes(uint64_t tiles) { return 8 * (bdelta_groups(tiles) + 9 * tiles); }
 
 // scratch of a split: the groups' matches (u64), then per tile its 8 units' matches (u16 each)
 __host__ __device__ inline uint64_t bsplit_group_bytes(uint64_t tiles)

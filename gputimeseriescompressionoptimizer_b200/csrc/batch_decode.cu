@@ -137,50 +137,243 @@ __device__ void p_afl_unpack(const BItem &it, uint32_t tile, StreamDesc *S, uint
 }
 
 // ------------------------------------------------------------------------------- delta decode
+// A decode view from one of its elements: values of b bits (mask) from bit s of the words at w (a plain
+// stream is one of full-width values), `left` values from there to the stream's end, c added to each.
+template <int ES>
+struct UnitSrc {
+    using V = std::conditional_t<ES == 8, uint64_t, uint32_t>;
+    const uint32_t *w = nullptr;
+    uint32_t s = 0, b = 0;
+    V mask = 0, c = 0;
+    uint64_t left = 0;
+    __device__ __forceinline__ void set(const uint8_t *p, uint64_t off_bits, uint32_t width, uint64_t first, uint64_t n,
+                                        uint64_t add)
+    {
+        const uint64_t bit = off_bits + first * width;
+        w = (const uint32_t *)p + (bit >> 5);
+        s = (uint32_t)(bit & 31);
+        b = width;
+        mask = width >= 8 * sizeof(V) ? ~(V)0 : ((V)1 << width) - 1;
+        left = n > first ? n - first : 0;
+        c = (V)add;
+    }
+    __device__ __forceinline__ void set(const DViewCtx &v, uint64_t first)
+    {
+        const uint32_t mis = (uint32_t)((uintptr_t)v.p & 3);
+        if (v.b) set(v.p, v.off_bits, (uint32_t)v.b, first, v.n, v.c0 + v.c1);
+        else set(v.p - mis, 8 * mis, 8 * ES, first, v.n, v.c0 + v.c1);
+    }
+};
+
+// 16 bytes' worth of consecutive values of a view, from value i of its unit (a multiple of them).
+// CHECK: zeros from value `cnt` of the unit on; else all exist and a whole word follows them.
+template <int ES, bool CHECK>
+__device__ __forceinline__ void unit_vec(const UnitSrc<ES> &u, uint32_t i, uint32_t cnt, word_t<ES> (&v)[16 / ES])
+{
+    using V = word_t<ES>;
+    constexpr int N = 16 / ES;
+    const uint32_t bit = u.s + i * u.b;
+    if (!CHECK && u.b == 8 * ES && u.s == 0 && ((uintptr_t)u.w & 15) == 0) {
+        const uint4 q = ldg((const uint4 *)u.w + i / N);
+#pragma unroll
+        for (int k = 0; k < N; k++) v[k] = (V)chunk_elem<ES>(q, k) + u.c;
+    } else if (!CHECK && N * u.b <= 32) {
+        const uint32_t *w = u.w + (bit >> 5);
+        const uint32_t x = __funnelshift_r(ldg(w), ldg(w + 1), bit);
+#pragma unroll
+        for (int k = 0; k < N; k++) v[k] = ((x >> (k * u.b)) & (uint32_t)u.mask) + u.c;
+    } else if (!CHECK && N * u.b <= 64) {
+        const uint32_t *w = u.w + (bit >> 5);
+        const uint32_t w0 = ldg(w), w1 = ldg(w + 1), w2 = (bit & 31) + N * u.b > 64 ? ldg(w + 2) : 0u;
+        const uint64_t x = (uint64_t)__funnelshift_r(w1, w2, bit) << 32 | __funnelshift_r(w0, w1, bit);
+#pragma unroll
+        for (int k = 0; k < N; k++) v[k] = ((V)(x >> (k * u.b)) & u.mask) + u.c;
+    } else {
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            const uint32_t p = bit + k * u.b, s = p & 31;
+            const uint32_t *w = u.w + (p >> 5);
+            const bool in = !CHECK || i + k < cnt;
+            const uint32_t w0 = in ? ldg(w) : 0u, w1 = in && s + u.b > 32 ? ldg(w + 1) : 0u;
+            V x;
+            if constexpr (ES == 8) {
+                const uint32_t w2 = in && s + u.b > 64 ? ldg(w + 2) : 0u;
+                x = (uint64_t)__funnelshift_r(w1, w2, s) << 32 | __funnelshift_r(w0, w1, s);
+            } else {
+                x = __funnelshift_r(w0, w1, s);
+            }
+            v[k] = in ? (x & u.mask) + u.c : (V)0;
+        }
+    }
+}
+
+// The sums of a delta decode (element i = first + the differences before i, wrapping) take two passes
+// over the differences, which are mostly packed, so that no tile waits for another: this one sums every
+// unit of 1024 (one warp), tile of 8 units and group of 64 tiles.
+struct DeltaSums {
+    unsigned long long *groups, *tiles, *units;
+    __device__ __forceinline__ DeltaSums(const BItem &it)
+    {
+        groups = (unsigned long long *)(it.scratch + it.p[0]);
+        tiles = groups + bdelta_groups(it.tiles);
+        units = tiles + it.tiles;
+    }
+};
+
+// the sum of a unit's differences (its low 8 * ES bits), in every lane of the warp
+template <int ES>
+__device__ __forceinline__ unsigned long long delta_unit_sum(const DViewCtx &dv, uint64_t unit)
+{
+    using V = word_t<ES>;
+    constexpr uint32_t N = 16 / ES;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t e0 = unit * kBDeltaUnit;
+    V sum = 0;
+    if (e0 < dv.n) {
+        UnitSrc<ES> u;
+        u.set(dv, e0);
+        V v[N];
+        if (u.left >= kBDeltaUnit + 64) {
+#pragma unroll(ES >= 4 ? 4 : 1)
+            for (uint32_t i = lane * N; i < kBDeltaUnit; i += 32 * N) {
+                unit_vec<ES, false>(u, i, 0, v);
+#pragma unroll
+                for (int k = 0; k < (int)N; k++) sum += v[k];
+            }
+        } else {
+            const uint32_t cnt = (uint32_t)(u.left < kBDeltaUnit ? u.left : kBDeltaUnit);
+#pragma unroll 1
+            for (uint32_t i = lane * N; i < cnt; i += 32 * N) {
+                unit_vec<ES, true>(u, i, cnt, v);
+#pragma unroll
+                for (int k = 0; k < (int)N; k++) sum += v[k];
+            }
+        }
+    }
+    unsigned long long x = sum;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
+    return x;
+}
+
+template <int ES>
+__device__ void p_delta_sum(const BItem &it, uint32_t tile, StreamDesc *S)
+{
+    constexpr uint32_t WARPS = kBThreads / 32;
+    __shared__ unsigned long long s_sum[WARPS];
+    bool ok;
+    DViewCtx dv = dview_ctx<ES>(it, S, 1, ok);
+    if (!ok) dv.n = 0;
+    const uint32_t warp = threadIdx.x >> 5;
+    const uint64_t unit = (uint64_t)tile * WARPS + warp;
+    unsigned long long x = delta_unit_sum<ES>(dv, unit);
+    const DeltaSums ds(it);
+    if ((threadIdx.x & 31) == 0) ds.units[unit] = s_sum[warp] = x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (uint32_t w = 1; w < WARPS; w++) x += s_sum[w];
+        ds.tiles[tile] = x;
+        atomicAdd(ds.groups + tile / kBDeltaGroup, x);
+    }
+}
+
+// The second pass: a warp adds up the sums before its unit and scans the unit in rows of 512 bytes, 16
+// bytes a lane.  CHECK as unit_vec; `end`: elements of the unit to write, `cnt` of them with a difference.
+template <int ES, bool CHECK>
+__device__ __forceinline__ void delta_unit(const UnitSrc<ES> &u, word_t<ES> acc, uint8_t *out, uint32_t cnt, uint32_t end)
+{
+    using V = word_t<ES>;
+    constexpr int N = 16 / ES, R = ES >= 4 ? 4 : 1;  // rows whose loads are in flight together
+    constexpr uint32_t ROW = 32 * N;
+    static_assert(kBDeltaUnit % (ROW * R) == 0, "whole batches of rows");
+    const uint32_t lane = threadIdx.x & 31;
+    const bool vec = ((uintptr_t)out & 15) == 0;
+#pragma unroll 1
+    for (uint32_t r0 = 0; r0 < (CHECK ? end : kBDeltaUnit); r0 += ROW * R) {
+        V v[R][N], t[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) unit_vec<ES, CHECK>(u, r0 + r * ROW + lane * N, cnt, v[r]);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            V s = 0;
+#pragma unroll
+            for (int k = 0; k < N; k++) {  // exclusive sums of the lane's values
+                const V x = v[r][k];
+                v[r][k] = s;
+                s += x;
+            }
+            t[r] = s;
+        }
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            V y[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) y[r] = __shfl_up_sync(0xffffffffu, t[r], d);
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                if (lane >= (uint32_t)d) t[r] += y[r];
+        }
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const V total = __shfl_sync(0xffffffffu, t[r], 31), up = __shfl_up_sync(0xffffffffu, t[r], 1);
+            const V base = acc + (lane ? up : (V)0);
+            acc += total;
+            const uint32_t i = r0 + r * ROW + lane * N;
+            uint64_t o[N];
+#pragma unroll
+            for (int k = 0; k < N; k++) o[k] = wrap_es(base + v[r][k], ES);
+            if (vec && (!CHECK || i + N <= end)) {
+                ((uint4 *)out)[i / N] = make_chunk<ES>(o);
+            } else {
+#pragma unroll
+                for (int k = 0; k < N; k++)
+                    if (!CHECK || i + k < end) st_elem<ES>(out, i + k, o[k]);
+            }
+        }
+    }
+}
+
+// Delta decode, second pass (C bytes of differences read again, n * s written).  Before, one pass kept
+// 16 unpacked values a thread behind a look-back, and its blocked stores touched half sectors.  2^26
+// int32 in 5 bits, both passes: 0.400 -> 0.195 ms (0.115 of it here); the 256 mixed columns' delta decodes
+// 0.84 -> 0.72 ms.  Tried: four tiles a block behind one setup (long columns 3 % faster, short ones twice
+// as slow); blocks of short columns summing what lies before them instead of a pass (no faster).
 template <int ES>
 __device__ void p_delta_dec(const BItem &it, uint32_t tile, StreamDesc *S, uint32_t *status)
 {
-    __shared__ unsigned long long ws[32];
-    __shared__ unsigned long long s_prefix;
+    using V = word_t<ES>;
+    constexpr uint32_t WARPS = kBThreads / 32;
     const StreamDesc meta = S[it.in[0]];
     bool ok;
     const DViewCtx dv = dview_ctx<ES>(it, S, 1, ok);
     StreamDesc &out = S[it.out[0]];
     const uint64_t n = meta.len ? dv.n + 1 : 0;
-    if (!ok || n * ES > out.cap) {  // item-uniform: no tile of this item enters the look-back
+    if (!ok || n * ES > out.cap) {
         if (tile == 0 && threadIdx.x == 0) set_status(status, ok ? GTSC_ERR_CAPACITY : GTSC_ERR_FORMAT);
         return;
     }
     if (tile == 0 && threadIdx.x == 0) out.len = n * ES;
-    // a tile past the output has no successor waiting on its look-back descriptor
-    if (tile > 0 && (uint64_t)tile * kBTile >= n) return;
-    Lookback lb = lookback_at(it.scratch + it.p[0], it.tiles);
-    const uint64_t m = n ? n - 1 : 0;
-    const uint64_t base = (uint64_t)tile * kBTile + (uint64_t)threadIdx.x * kBVPT;
-    uint64_t v[kBVPT];
-    load_dview<ES, kBVPT>(dv, base, v);
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t unit = (uint64_t)tile * WARPS + warp, e0 = unit * kBDeltaUnit;
+    if (e0 >= n) return;
+    const DeltaSums ds(it);
+    const uint32_t g = tile / kBDeltaGroup;
+    unsigned long long part = 0;
+    for (uint32_t k = lane; k < g; k += 32) part += ldg(ds.groups + k);
+    for (uint32_t k = g * kBDeltaGroup + lane; k < tile; k += 32) part += ldg(ds.tiles + k);
+    if (lane < warp) part += ldg(ds.units + (uint64_t)tile * WARPS + lane);
 #pragma unroll
-    for (int j = 0; j < (int)kBVPT; j++)
-        if (base + j >= m) v[j] = 0;
-    unsigned long long local = 0;
-#pragma unroll
-    for (int j = 0; j < (int)kBVPT; j++) local += v[j];
-    unsigned long long total;
-    const unsigned long long excl = block_exclusive_scan<kBThreads>(local, ws, total);
-    if (threadIdx.x < 32) {
-        const unsigned long long e = lookback_exclusive(lb, tile, total);
-        if (threadIdx.x == 0) s_prefix = e;
+    for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(0xffffffffu, part, d);
+    const V acc = (V)(ld_unaligned<ES>(meta.ptr) + part);
+    UnitSrc<ES> u;
+    u.set(dv, e0);
+    uint8_t *dst = out.ptr + e0 * ES;
+    if (u.left >= kBDeltaUnit + 64) {
+        delta_unit<ES, false>(u, acc, dst, kBDeltaUnit, kBDeltaUnit);
+    } else {
+        const uint32_t end = (uint32_t)(n - e0 < kBDeltaUnit ? n - e0 : kBDeltaUnit);
+        delta_unit<ES, true>(u, acc, dst, (uint32_t)(u.left < end ? u.left : end), end);
     }
-    __syncthreads();
-    if (base >= n) return;
-    unsigned long long acc = ld_unaligned<ES>(meta.ptr) + s_prefix + excl;
-    uint64_t o[kBVPT];
-#pragma unroll
-    for (int j = 0; j < (int)kBVPT; j++) {
-        o[j] = wrap_es(acc, ES);
-        acc += v[j];
-    }
-    store_run<ES, kBVPT>(out.ptr, base, n, o);
 }
 
 // ------------------------------------------------------------------------------- scale add
@@ -289,34 +482,6 @@ __device__ void p_merge_count(const BItem &it, uint32_t tile, StreamDesc *S)
     }
 }
 
-// One of a unit's two sources: values of b bits (mask) from bit s of the words at w (a plain stream
-// is one of full-width values), `left` values from there to the stream's end, c added to each.
-template <int ES>
-struct MergeSrc {
-    using V = std::conditional_t<ES == 8, uint64_t, uint32_t>;
-    const uint32_t *w = nullptr;
-    uint32_t s = 0, b = 0;
-    V mask = 0, c = 0;
-    uint64_t left = 0;
-    __device__ __forceinline__ void set(const uint8_t *p, uint64_t off_bits, uint32_t width, uint64_t first, uint64_t n,
-                                        uint64_t add)
-    {
-        const uint64_t bit = off_bits + first * width;
-        w = (const uint32_t *)p + (bit >> 5);
-        s = (uint32_t)(bit & 31);
-        b = width;
-        mask = width >= 8 * sizeof(V) ? ~(V)0 : ((V)1 << width) - 1;
-        left = n > first ? n - first : 0;
-        c = (V)add;
-    }
-    __device__ __forceinline__ void set(const DViewCtx &v, uint64_t first)
-    {
-        const uint32_t mis = (uint32_t)((uintptr_t)v.p & 3);
-        if (v.b) set(v.p, v.off_bits, (uint32_t)v.b, first, v.n, v.c0 + v.c1);
-        else set(v.p - mis, 8 * mis, 8 * ES, first, v.n, v.c0 + v.c1);
-    }
-};
-
 // R rows of 32 elements of one unit, from row j0.  In row j lane l's element is a match when bit l of
 // the row's stencil word is set (lane j holds the word); its rank among the unit's matches is the
 // matches before the row (pre, lane j) plus the word's set bits below l.  So each row's two runs are
@@ -326,10 +491,10 @@ struct MergeSrc {
 // CHECK: a row may pass the unit's end (cnt) or a stream's end; else whole rows whose every value
 // is followed by another whole word of its stream.
 template <int ES, int MODE, bool CHECK, int R>
-__device__ __forceinline__ bool merge_rows(const MergeSrc<ES> &ys, const MergeSrc<ES> &ns, const uint64_t (&top)[4],
+__device__ __forceinline__ bool merge_rows(const UnitSrc<ES> &ys, const UnitSrc<ES> &ns, const uint64_t (&top)[4],
                                            uint32_t word, uint32_t pre, uint32_t j0, uint8_t *dst, uint32_t cnt)
 {
-    using V = typename MergeSrc<ES>::V;
+    using V = typename UnitSrc<ES>::V;
     constexpr bool ONE = MODE == SPLIT_NOT_CONST;  // only matches are read
     const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1;
     uint32_t bit[R], w0[R], w1[R], w2[ES == 8 ? R : 1], yes = 0;
@@ -379,7 +544,7 @@ __device__ __forceinline__ bool merge_rows(const MergeSrc<ES> &ys, const MergeSr
 }
 
 template <int ES, int MODE>
-__device__ __forceinline__ bool merge_unit(const MergeSrc<ES> &ys, const MergeSrc<ES> &ns, const uint64_t (&top)[4],
+__device__ __forceinline__ bool merge_unit(const UnitSrc<ES> &ys, const UnitSrc<ES> &ns, const uint64_t (&top)[4],
                                            uint32_t word, uint8_t *dst, uint32_t cnt)
 {
     constexpr int R = ES == 8 ? 4 : 8;
@@ -462,7 +627,7 @@ __device__ void p_merge(const BItem &it, uint32_t tile, StreamDesc *S, uint32_t 
     const uint32_t cnt = (uint32_t)(n - e0 < kBMergeUnit ? n - e0 : kBMergeUnit);
     uint8_t *dst = out.ptr + e0 * ES;
     uint64_t top[4] = {0, 0, 0, 0};
-    MergeSrc<ES> ys, ns;
+    UnitSrc<ES> ys, ns;
     bool bad;
     if (mode == SPLIT_DICT) {
         // dictionary stream: 16-byte header, 4 values, codes (2 bits a match)
@@ -864,7 +1029,11 @@ __device__ __forceinline__ uint32_t dec_extent(const BItem &it, const StreamDesc
 {
     auto cdiv = [](uint64_t a, uint64_t b) { return (a + b - 1) / b; };
     uint64_t e = it.tiles;
-    if constexpr (OP == B_SCALE_ADD) {
+    if constexpr (OP == B_DELTA_SUM) {
+        e = cdiv(dview_len(it, S, 1, it.es), kBDeltaTile);
+    } else if constexpr (OP == B_DELTA_DEC) {
+        e = cdiv(dview_len(it, S, 1, it.es) + 1, kBDeltaTile);
+    } else if constexpr (OP == B_SCALE_ADD) {
         e = cdiv(dview_len(it, S, 1, it.es), kBTile);
     } else if constexpr (OP == B_AFL_UNPACK) {
         const StreamDesc data = S[it.in[1]], meta = S[it.in[0]];
@@ -895,11 +1064,12 @@ __device__ __forceinline__ void run_dec(const BItem &it, uint32_t tile, StreamDe
 
 constexpr bool dec_persistent(int op)
 {
-    return op == B_AFL_UNPACK || op == B_SCALE_ADD || op == B_F2I_DEC || op == B_RLE_EXPAND;
+    return op == B_AFL_UNPACK || op == B_SCALE_ADD || op == B_F2I_DEC || op == B_RLE_EXPAND ||
+           op == B_DELTA_SUM || op == B_DELTA_DEC;
 }
 
 // resident blocks per SM the compiler keeps registers for: the merge's rows need 64 registers
-constexpr int dec_min_blocks(int op) { return op == B_MERGE ? 4 : 5; }
+constexpr int dec_min_blocks(int op) { return op == B_MERGE || op == B_DELTA_DEC || op == B_DELTA_SUM ? 4 : 5; }
 
 // One launch of a decode pass over every item: look-back passes one tile per block in claim order,
 // the others persistent over the tiles (see k_bstage).
@@ -908,7 +1078,7 @@ __global__ void __launch_bounds__(kBThreads, dec_min_blocks(OP))
 k_bdec(const BItem *items, const uint32_t *item_of, StreamDesc *S, uint32_t *counter, uint32_t *status,
        uint32_t total_tiles)
 {
-    constexpr bool DYN = OP == B_DELTA_DEC || OP == B_RLE_SCAN || OP == B_MERGE_COUNT;
+    constexpr bool DYN = OP == B_RLE_SCAN || OP == B_MERGE_COUNT;
     constexpr int kSmem = OP == B_GFC_DEC                           ? kGfcRing * (kBThreads / 32)
                           : OP == B_RLE_EXPAND                      ? kXchgBlockBytes  // warp exchange
                                                                     : 16;
@@ -957,6 +1127,7 @@ __device__ __forceinline__ void run_dec(const BItem &it, uint32_t tile, StreamDe
     }
     if constexpr (OP == B_NONE_COPY) p_none_copy(it, tile, S, status);
     else if constexpr (OP == B_AFL_UNPACK) { GTSC_ES_SWITCH(p_afl_unpack<E>(it, tile, S, status)) }
+    else if constexpr (OP == B_DELTA_SUM) { GTSC_ES_SWITCH(p_delta_sum<E>(it, tile, S)) }
     else if constexpr (OP == B_DELTA_DEC) { GTSC_ES_SWITCH(p_delta_dec<E>(it, tile, S, status)) }
     else if constexpr (OP == B_SCALE_ADD) { GTSC_ES_SWITCH(p_scale_add<E>(it, tile, S, status)) }
     else if constexpr (OP == B_MERGE) { GTSC_ES_SWITCH(p_merge<E>(it, tile, S, status)) }
@@ -980,6 +1151,8 @@ __device__ __forceinline__ uint32_t persist_extent_d(int op, const BItem &it, co
 {
     switch (op) {
     case B_AFL_UNPACK: return dec_extent<B_AFL_UNPACK>(it, S);
+    case B_DELTA_SUM: return dec_extent<B_DELTA_SUM>(it, S);
+    case B_DELTA_DEC: return dec_extent<B_DELTA_DEC>(it, S);
     case B_SCALE_ADD: return dec_extent<B_SCALE_ADD>(it, S);
     case B_F2I_DEC: return dec_extent<B_F2I_DEC>(it, S);
     case B_RLE_EXPAND: return dec_extent<B_RLE_EXPAND>(it, S);
@@ -1000,6 +1173,7 @@ __global__ void __launch_bounds__(kBThreads, 4) k_bpersist_d(PersistArgs a)
 #define GTSC_RUN(OPC) case OPC: run_dec<OPC>(it, tile, a.S, a.status, smem); break;
                 GTSC_RUN(B_NONE_COPY)
                 GTSC_RUN(B_AFL_UNPACK)
+                GTSC_RUN(B_DELTA_SUM)
                 GTSC_RUN(B_DELTA_DEC)
                 GTSC_RUN(B_SCALE_ADD)
                 GTSC_RUN(B_MERGE)
@@ -1213,6 +1387,7 @@ void launch_batch_decode_stage(int op, const BItem *d_items, const uint32_t *d_i
     }
         GTSC_STAGE(B_NONE_COPY)
         GTSC_STAGE(B_AFL_UNPACK)
+        GTSC_STAGE(B_DELTA_SUM)
         GTSC_STAGE(B_DELTA_DEC)
         GTSC_STAGE(B_SCALE_ADD)
         GTSC_STAGE(B_MERGE)

@@ -92,3 +92,22 @@ def test_most_frequent_values(G, O, rng, dt):
                 dts.append(dt)
                 trees.append(G.tree_from_path(path, dt))
     run_batch(G, O, cols, dts, trees, steps=2)
+
+
+@pytest.mark.parametrize("dt", list(IDS), ids=list(IDS.values()))
+def test_delta_edges(G, O, rng, dt):
+    """delta decode around its 1024-value units, 8192-value tiles and 64-tile groups, from plain and packed
+    differences of several widths"""
+    paths = [[OR.DELTA, OR.NONE], [OR.DELTA, OR.DELTA, OR.NONE]]
+    if dt not in (OR.FLOAT, OR.DOUBLE):
+        paths += [[OR.DELTA, OR.AFL, OR.NONE], [OR.DELTA, OR.SCALE, OR.AFL, OR.NONE]]
+    cols, dts, trees = [], [], []
+    for n in [1, 2, 33, 127, 128, 129, 1023, 1024, 1025, 1026, 8192, 8193, 8194, 70000, 64 * 8192 + 1, 64 * 8192 + 1030]:
+        for bits in [1, 6, 12, 30]:
+            if n > 70000 and bits in (6, 30):
+                continue
+            x = 1000 + np.cumsum(rng.integers(0, 1 << bits, n))
+            cols.append((x % 97 if OR.NP_TYPES[dt] == np.int8 else x).astype(OR.NP_TYPES[dt]))
+            dts.append(dt)
+            trees.append(G.tree_from_path(paths[(n + bits) % len(paths)], dt))
+    run_batch(G, O, cols, dts, trees)
