@@ -254,6 +254,7 @@ constexpr uint32_t kBSplitUnit = 1024;  // split: values of a warp's unit (32 ro
 constexpr uint32_t kBSplitTile = 8 * kBSplitUnit;    // ... of a block
 constexpr uint32_t kBSplitGroup = 64;                // tiles whose matches are summed together
 
+constexpr uint32_t kBPackUnit = 512;    // AFL packing: values of a warp's unit (whole 16-byte pieces at any width)
 constexpr uint32_t kBDeltaUnit = 1024, kBDeltaTile = 8 * kBDeltaUnit, kBDeltaGroup = 64;  // delta decode, alike
 
 // scratch of a delta decode: sums (u64) of the groups, the tiles and the units

@@ -189,9 +189,75 @@ __device__ void p_scale_sub(const BItem &it, uint32_t tile, StreamDesc *S)
 }
 
 // ------------------------------------------------------------------------------- AFL pack
+__device__ __forceinline__ void sm_or(uint32_t a, uint32_t v) { asm volatile("red.shared.or.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+
 __device__ __forceinline__ uint32_t afl_slot(uint32_t i) { return i + (i >> 4); }
+// Packs the rows of a unit (16 bytes of values a lane and row) into the warp's words of shared memory,
+// which are zero: a lane's values become up to 5 words from bit i * b on, or-ed in (a word is shared by
+// the lanes whose bits it holds).  SMALL: they fit one word.
+template <int ES, bool SMALL>
+__device__ __forceinline__ void pack_rows(const ViewCtx &vc, const uint8_t *src, uint64_t u0, uint32_t cnt, uint32_t b,
+                                          uint32_t words)
+{
+    using V = word_t<ES>;
+    constexpr uint32_t N = 16 / ES, ROW = 32 * N, R = ES == 4 ? 4 : 1;
+    const V mask = b >= 8 * sizeof(V) ? ~(V)0 : ((V)1 << b) - 1;
+    const uint32_t lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (uint32_t r0 = 0; r0 * ROW < cnt; r0 += R) {
+        V v[R][N];
+#pragma unroll
+        for (uint32_t r = 0; r < R; r++) {
+            const uint32_t i = (r0 + r) * ROW + lane * N;
+            if (i < cnt) load_vec<ES>(vc, src, u0 + i, v[r]);  // zeros past the view
+        }
+#pragma unroll
+        for (uint32_t r = 0; r < R; r++) {
+            const uint32_t i = (r0 + r) * ROW + lane * N, bit = i * b;
+            if (i >= cnt) continue;
+            uint32_t at = words + 4 * (bit >> 5);
+            if constexpr (SMALL) {
+                uint32_t x = 0;
+#pragma unroll
+                for (int k = (int)N - 1; k >= 0; k--) x = x << b | (uint32_t)(v[r][k] & mask);
+                const uint32_t s = bit & 31;
+                sm_or(at, x << s);
+                const uint32_t hi = __funnelshift_l(x, 0u, s);
+                if (hi) sm_or(at + 4, hi);
+            } else {
+                uint64_t acc = 0;
+                uint32_t fill = bit & 31;
+                auto put = [&](uint32_t x, uint32_t w) {  // w <= 32 bits
+                    acc |= (uint64_t)x << fill;
+                    fill += w;
+                    if (fill >= 32) {
+                        sm_or(at, (uint32_t)acc);
+                        at += 4;
+                        acc >>= 32;
+                        fill -= 32;
+                    }
+                };
+#pragma unroll
+                for (int k = 0; k < (int)N; k++) {
+                    const V x = v[r][k] & mask;
+                    put(x, b);
+                }
+                if (fill) sm_or(at, (uint32_t)acc);
+            }
+        }
+    }
+}
+
+// AFL packing (n * s read, n * b / 8 written).  Values of up to 4 bytes read plainly: a warp packs a unit
+// whose packed words no other unit shares, in its own part of shared memory, and stores them whole; no
+// barrier lies between units.  Views (a delta's neighbours, a scale's constant) and 8-byte values: a
+// thread packs 16 consecutive values between two barriers.  That form's 16-byte loads lie 64 bytes
+// apart, which binds it by L1 where nothing else does, but it shares the neighbours of a view in
+// registers.  2^26 int32: 31 bits, plain 0.219 -> 0.113 ms (4.7 TB/s); a scaled delta in 5 bits 0.139 ->
+// 0.107, by the setup done once for a block's tiles of an item (as units 0.164); the 256 mixed columns
+// 0.69 -> 0.56.  64 registers, four blocks an SM: with 48 and five the units took 0.167.
 template <int ES>
-__device__ void p_afl_pack(const BItem &it, uint32_t tile, StreamDesc *S, unsigned long long *sv)
+__device__ void p_afl_pack(const BItem &it, uint32_t tile, uint32_t step, uint32_t end, StreamDesc *S, unsigned char *sm)
 {
     const StreamDesc in = S[it.in[0]];
     const ViewCtx vc = view_ctx<ES>(it, in);
@@ -239,9 +305,45 @@ __device__ void p_afl_pack(const BItem &it, uint32_t tile, StreamDesc *S, unsign
         }
         S[it.out[1]].len = out_bytes;
     }
+    if constexpr (ES <= 4) {
+    if (vc.plain) {
+    constexpr uint32_t UNIT = kBPackUnit;
+    const uint32_t lane = threadIdx.x & 31, pieces = UNIT / 128 * (uint32_t)b;  // of 16 bytes, of a unit's output
+    uint8_t *const out0 = S[it.out[1]].ptr;
+    uint4 *wq = (uint4 *)(sm + (threadIdx.x >> 5) * (UNIT * ES));
+    const uint32_t words = (uint32_t)__cvta_generic_to_shared(wq);
+#pragma unroll 1
+    for (; tile < end; tile += step) {
+        const uint64_t u0 = (uint64_t)tile * kBTile + (threadIdx.x >> 5) * UNIT;
+        if (u0 >= n) break;
+        const uint32_t cnt = (uint32_t)(n - u0 < UNIT ? n - u0 : UNIT);
+        __syncwarp();  // the warp's words of the tile before are stored
+        for (uint32_t i = lane; i < pieces; i += 32) wq[i] = make_uint4(0, 0, 0, 0);
+        __syncwarp();
+        if (16 / ES * b <= 32) pack_rows<ES, true>(vc, in.ptr, u0, cnt, (uint32_t)b, words);
+        else pack_rows<ES, false>(vc, in.ptr, u0, cnt, (uint32_t)b, words);
+        __syncwarp();
+        const uint64_t o0 = u0 / 8 * (uint64_t)b;  // the unit's first byte of the output
+        uint8_t *out = out0 + o0;
+        const uint64_t left = out_bytes - o0;
+        for (uint32_t i = lane; i < pieces; i += 32) {
+            if (16ull * i + 16 <= left) {
+                ((uint4 *)out)[i] = wq[i];
+            } else {
+                for (uint32_t k = 16 * i; k < 16 * i + 16 && k < left; k++) out[k] = ((const uint8_t *)wq)[k];
+            }
+        }
+    }
+    return;
+    }
+    }
+    uint8_t *const out = S[it.out[1]].ptr;
+    unsigned long long *sv = (unsigned long long *)sm;
+#pragma unroll 1
+    for (; tile < end; tile += step) {
     const uint64_t t0 = (uint64_t)tile * kBTile;
     if (t0 >= n) return;
-    uint8_t *out = S[it.out[1]].ptr;
+    __syncthreads();  // the tile before is stored
     if constexpr (ES <= 4) {
         // b <= 32.  Thread t packs its 16 values (tile bits [16 b t, 16 b (t + 1))) into a register
         // and stores whole words to the tile's words in shared memory; the word it shares with the
@@ -289,7 +391,7 @@ __device__ void p_afl_pack(const BItem &it, uint32_t tile, StreamDesc *S, unsign
                     if (4 * w + k < out_bytes) out[4 * w + k] = (uint8_t)(word >> (8 * k));
             }
         }
-        return;
+        continue;
     }
     const uint64_t vmask = b >= 64 ? ~0ull : ((1ull << b) - 1);
     const uint64_t cnt = n - t0 < kBTile ? n - t0 : kBTile;
@@ -338,6 +440,7 @@ __device__ void p_afl_pack(const BItem &it, uint32_t tile, StreamDesc *S, unsign
             for (int k = 0; k < 4; k++)
                 if (4 * w + k < out_bytes) out[4 * w + k] = (uint8_t)(word >> (8 * k));
         }
+    }
     }
 }
 
@@ -1368,7 +1471,7 @@ __device__ __forceinline__ void split_ballots(const ViewCtx &vc, const uint8_t *
 // 1024 values, in rows of 32: a row's ballot is its stencil word.  Also the min / max of the classes
 // that an AFL child packs (integer order, as its own min/max pass would compute it).
 template <int ES, int MODE, bool FP>
-__device__ __forceinline__ void split_count(const BItem &it, uint32_t tile, StreamDesc *S)
+__device__ __forceinline__ void split_count(const BItem &it, uint32_t tile, uint32_t step, uint32_t end, StreamDesc *S)
 {
     using V = word_t<ES>;
     using SV = sword_t<ES>;
@@ -1389,8 +1492,6 @@ __device__ __forceinline__ void split_count(const BItem &it, uint32_t tile, Stre
         }
     }
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t w0 = (uint64_t)tile * kBSplitTile + warp * kBSplitUnit;  // the warp's first value
-    const uint32_t cnt = w0 >= n ? 0u : (uint32_t)(n - w0 < kBSplitUnit ? n - w0 : kBSplitUnit);
     SplitArgs<ES> a{};
     if constexpr (CONST || DICT) {
         const uint8_t *tp = CONST ? meta : S[it.out[1]].ptr + 16;
@@ -1418,6 +1519,12 @@ __device__ __forceinline__ void split_count(const BItem &it, uint32_t tile, Stre
     }
     const bool fold_y = it.p[2] != 0, fold_n = it.p[3] != 0;
     constexpr SV LO = ES == 8 ? (SV)INT64_MIN : (SV)INT32_MIN, HI = ~LO;
+    __shared__ uint32_t s_tot[WARPS];
+    __shared__ unsigned long long s_fold[WARPS][4];
+#pragma unroll 1
+    for (; tile < end; tile += step) {
+    const uint64_t w0 = (uint64_t)tile * kBSplitTile + warp * kBSplitUnit;  // the warp's first value
+    const uint32_t cnt = w0 >= n ? 0u : (uint32_t)(n - w0 < kBSplitUnit ? n - w0 : kBSplitUnit);
     SV mm[4] = {HI, LO, HI, LO};
     uint32_t mine = 0;
     if (fold_y || fold_n) {
@@ -1440,8 +1547,6 @@ __device__ __forceinline__ void split_count(const BItem &it, uint32_t tile, Stre
         if (left < 32 && ((word >> (left - 1)) & 1u)) word |= ~0u << left;
         ((uint32_t *)(meta + (CONST ? ES + 1 : 1)))[w0 / 32 + lane] = word;  // 4-byte aligned (layout)
     }
-    __shared__ uint32_t s_tot[WARPS];
-    __shared__ unsigned long long s_fold[WARPS][4];
     if (lane == 0) s_tot[warp] = total;
     if (fold_y || fold_n) {
         warp_min_max<ES>(mm[0], mm[1]);
@@ -1471,20 +1576,22 @@ __device__ __forceinline__ void split_count(const BItem &it, uint32_t tile, Stre
         unsigned long long *dst = lane & 1 ? &acc->kmax : &acc->nkmin;
         if (x > *(volatile unsigned long long *)dst) atomicMax(dst, x);  // most tiles do not move it
     }
+    __syncthreads();  // the next tile's counts
+    }
 }
 
-__device__ __forceinline__ void p_split_count(const BItem &it, uint32_t tile, StreamDesc *S)
+__device__ __forceinline__ void p_split_count(const BItem &it, uint32_t tile, uint32_t step, uint32_t end, StreamDesc *S)
 {
     with_size(it.es, [&](auto es) {
         constexpr int E = decltype(es)::value;
-        if (it.mode == SPLIT_DICT) split_count<E, SPLIT_DICT, false>(it, tile, S);
-        else if (it.mode == SPLIT_NOT_CONST) split_count<E, SPLIT_NOT_CONST, false>(it, tile, S);
+        if (it.mode == SPLIT_DICT) split_count<E, SPLIT_DICT, false>(it, tile, step, end, S);
+        else if (it.mode == SPLIT_NOT_CONST) split_count<E, SPLIT_NOT_CONST, false>(it, tile, step, end, S);
         else if (E >= 4 && it.order != ORD_INT) {
-            if (it.p[1]) split_count<E, kSplitOutside, (E >= 4)>(it, tile, S);
-            else split_count<E, SPLIT_LOWER, (E >= 4)>(it, tile, S);
+            if (it.p[1]) split_count<E, kSplitOutside, (E >= 4)>(it, tile, step, end, S);
+            else split_count<E, SPLIT_LOWER, (E >= 4)>(it, tile, step, end, S);
         } else {
-            if (it.p[1]) split_count<E, kSplitOutside, false>(it, tile, S);
-            else split_count<E, SPLIT_LOWER, false>(it, tile, S);
+            if (it.p[1]) split_count<E, kSplitOutside, false>(it, tile, step, end, S);
+            else split_count<E, SPLIT_LOWER, false>(it, tile, step, end, S);
         }
     });
 }
@@ -1522,11 +1629,13 @@ __device__ __forceinline__ void split_rows(const ViewCtx &vc, const uint8_t *src
 // before its tile's, of the tiles before it in the group and of the units before it in the tile; a
 // value's rank in its unit comes from the stencil words.  Rows are stored straight to the two runs;
 // only a dictionary's 2-bit codes pass through shared memory, to be packed 16 a word.
-// 2^26 int32, both passes: patch 0.430 -> 0.206 ms, Zipf(1.1) dictionary 0.506 -> 0.247 ms.  One pass with
+// 2^26 int32, both passes: patch 0.430 -> 0.182 ms, Zipf(1.1) dictionary 0.506 -> 0.233 ms (0.206 and
+// 0.247 with the setup done for every tile).  One pass with
 // the rows held in registers behind a look-back took 0.26 and 0.29 ms (its warps wait at the barrier of
 // the look-back); the same with two tiles in flight a block 0.27 and 0.33 ms (too few warps).
 template <int ES, int MODE>
-__device__ __forceinline__ void split_move(const BItem &it, uint32_t tile, StreamDesc *S, unsigned char *sm)
+__device__ __forceinline__ void split_move(const BItem &it, uint32_t tile, uint32_t step, uint32_t end, StreamDesc *S,
+                                           unsigned char *sm)
 {
     using V = word_t<ES>;
     constexpr int R = 8;
@@ -1535,10 +1644,16 @@ __device__ __forceinline__ void split_move(const BItem &it, uint32_t tile, Strea
     const ViewCtx vc = view_ctx<ES>(it, in);
     const uint64_t n = vc.n;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t w0 = (uint64_t)tile * kBSplitTile + warp * kBSplitUnit;  // the warp's first value
-    if (w0 >= n) return;
-    const uint32_t cnt = (uint32_t)(n - w0 < kBSplitUnit ? n - w0 : kBSplitUnit);
     const uint8_t *meta = S[it.out[0]].ptr;
+    uint8_t *const out1 = S[it.out[1]].ptr, *const out2 = CONST ? nullptr : S[it.out[2]].ptr;
+    V top[4] = {0, 0, 0, 0};
+    if constexpr (DICT)
+        for (int k = 1; k < 4; k++) top[k] = (V)ld_elem<ES>(out1 + 16, k);
+#pragma unroll 1
+    for (; tile < end; tile += step) {
+    const uint64_t w0 = (uint64_t)tile * kBSplitTile + warp * kBSplitUnit;  // the warp's first value
+    if (w0 >= n) break;
+    const uint32_t cnt = (uint32_t)(n - w0 < kBSplitUnit ? n - w0 : kBSplitUnit);
     uint32_t word = 32 * lane < cnt ? ldg((const uint32_t *)(meta + (CONST ? ES + 1 : 1)) + w0 / 32 + lane) : 0u;
     if (cnt < 32 * lane + 32 && cnt > 32 * lane) word &= (1u << (cnt - 32 * lane)) - 1;
     // the matches before the unit
@@ -1564,11 +1679,8 @@ __device__ __forceinline__ void split_move(const BItem &it, uint32_t tile, Strea
     }
     const uint32_t total = __shfl_sync(0xffffffffu, pre, 31);
     pre -= __popc(word);
-    V top[4] = {0, 0, 0, 0};
-    if constexpr (DICT)
-        for (int k = 1; k < 4; k++) top[k] = (V)ld_elem<ES>(S[it.out[1]].ptr + 16, k);
-    elem_t<ES> *yes = DICT ? nullptr : (elem_t<ES> *)S[it.out[1]].ptr + yes0;
-    elem_t<ES> *no = CONST ? nullptr : (elem_t<ES> *)S[it.out[2]].ptr + no0 + lane;
+    elem_t<ES> *yes = DICT ? nullptr : (elem_t<ES> *)out1 + yes0;
+    elem_t<ES> *no = CONST ? nullptr : (elem_t<ES> *)out2 + no0 + lane;
     unsigned char *codes = sm + warp * kSplitCodes;
     const uint32_t c0 = (uint32_t)(yes0 & 15);  // the unit's first code inside its code word
 #pragma unroll 1
@@ -1582,11 +1694,11 @@ __device__ __forceinline__ void split_move(const BItem &it, uint32_t tile, Strea
         // the unit's codes, 16 a word; the first and the last word may be shared with the neighbour
         // units and are or-ed in (the words start zeroed)
         __syncwarp();
-        uint32_t *words = (uint32_t *)(S[it.out[1]].ptr + 16 + 4 * ES) + (yes0 >> 4);
-        const uint32_t end = total ? c0 + total : 0;
-        for (uint32_t k = lane; 16 * k < end; k += 32) {
+        uint32_t *words = (uint32_t *)(out1 + 16 + 4 * ES) + (yes0 >> 4);
+        const uint32_t codes_end = total ? c0 + total : 0;
+        for (uint32_t k = lane; 16 * k < codes_end; k += 32) {
             uint32_t x = pack_codes(((const uint4 *)codes)[k]);
-            const uint32_t lo = 16 * k < c0 ? c0 - 16 * k : 0, hi = end - 16 * k < 16 ? end - 16 * k : 16;
+            const uint32_t lo = 16 * k < c0 ? c0 - 16 * k : 0, hi = codes_end - 16 * k < 16 ? codes_end - 16 * k : 16;
             if (lo == 0 && hi == 16) {
                 words[k] = x;
             } else {  // bytes outside [lo, hi) are of an earlier unit
@@ -1614,14 +1726,16 @@ __device__ __forceinline__ void split_move(const BItem &it, uint32_t tile, Strea
             S[it.out[2]].len = (n - m) * ES;
         }
     }
+    }
 }
 
 template <int ES>
-__device__ __forceinline__ void p_split(const BItem &it, uint32_t tile, StreamDesc *S, unsigned char *sm)
+__device__ __forceinline__ void p_split(const BItem &it, uint32_t tile, uint32_t step, uint32_t end, StreamDesc *S,
+                                        unsigned char *sm)
 {
-    if (it.mode == SPLIT_DICT) split_move<ES, SPLIT_DICT>(it, tile, S, sm);
-    else if (it.mode == SPLIT_NOT_CONST) split_move<ES, SPLIT_NOT_CONST>(it, tile, S, sm);
-    else split_move<ES, SPLIT_LOWER>(it, tile, S, sm);
+    if (it.mode == SPLIT_DICT) split_move<ES, SPLIT_DICT>(it, tile, step, end, S, sm);
+    else if (it.mode == SPLIT_NOT_CONST) split_move<ES, SPLIT_NOT_CONST>(it, tile, step, end, S, sm);
+    else split_move<ES, SPLIT_LOWER>(it, tile, step, end, S, sm);
 }
 
 // ------------------------------------------------------------------------------- RLE
@@ -2140,9 +2254,15 @@ __device__ __forceinline__ uint32_t stage_extent(const BItem &it, const StreamDe
     return (uint32_t)(e < it.tiles ? e : it.tiles);
 }
 
+// `step`, `end`: passes that loop over an item's tiles themselves (stage_item_loop) run tile, tile + step,
+// ... below end; the others run `tile`
 template <int OP>
-__device__ __forceinline__ void run_stage(const BItem &it, uint32_t tile, StreamDesc *S, uint32_t *status,
-                                          unsigned char *smem);
+__device__ __forceinline__ void run_stage(const BItem &it, uint32_t tile, uint32_t step, uint32_t end, StreamDesc *S,
+                                          uint32_t *status, unsigned char *smem);
+
+// passes that set up (stream pointers, view, widths, classes: a chain of dependent loads) once for all of
+// a block's tiles of an item
+constexpr bool stage_item_loop(int op) { return op == B_AFL_PACK || op == B_SPLIT_COUNT || op == B_SPLIT; }
 
 // passes whose tiles all do the same streaming work run persistent grids (see stage_grid)
 constexpr bool stage_persistent(int op)
@@ -2158,7 +2278,7 @@ constexpr bool stage_persistent(int op)
 constexpr int stage_min_blocks(int op)
 {
     // the histogram at 4 (64 registers, no spills) measured 6 % faster than at 5 (48 registers, spilling)
-    return op == B_GFC_COMPRESS || op == B_TOPK || op == B_HIST ? 4 : 5;
+    return op == B_AFL_PACK || op == B_GFC_COMPRESS || op == B_TOPK || op == B_HIST ? 4 : 5;
 }
 
 template <int OP>
@@ -2172,7 +2292,7 @@ k_bstage(const BItem *items, const uint32_t *item_of, StreamDesc *S, uint32_t *c
         uint32_t tile;
         const BItem &it = locate<DYN>(items, item_of, counter, tile);
         if (tile >= it.tiles) return;
-        run_stage<OP>(it, tile, S, status, smem);
+        run_stage<OP>(it, tile, 1, tile + 1, S, status, smem);
     } else {
         uint32_t t = blockIdx.x;
         uint32_t cur = 0xffffffffu;  // the item in the shared descriptor
@@ -2185,13 +2305,15 @@ k_bstage(const BItem *items, const uint32_t *item_of, StreamDesc *S, uint32_t *c
             }
             const BItem &it = shared_item_ref();
             const uint32_t tile = t - (uint32_t)it.tile_base;
-            if (tile >= stage_extent<OP>(it, S)) {
+            const uint32_t extent = stage_extent<OP>(it, S);
+            if (tile >= extent) {
                 const uint64_t next = it.tile_base + it.tiles;  // the next item's first tile
                 if (next >= total_tiles) break;
                 t = (uint32_t)(next + (blockIdx.x + gridDim.x - next % gridDim.x) % gridDim.x);
                 continue;
             }
-            run_stage<OP>(it, tile, S, status, smem);
+            run_stage<OP>(it, tile, gridDim.x, extent, S, status, smem);
+            if constexpr (stage_item_loop(OP)) t += (extent - 1 - tile) / gridDim.x * gridDim.x;
             __syncthreads();  // the next tile reuses the shared memory
             t += gridDim.x;
         }
@@ -2199,8 +2321,8 @@ k_bstage(const BItem *items, const uint32_t *item_of, StreamDesc *S, uint32_t *c
 }
 
 template <int OP>
-__device__ __forceinline__ void run_stage(const BItem &it, uint32_t tile, StreamDesc *S, uint32_t *status,
-                                          unsigned char *smem)
+__device__ __forceinline__ void run_stage(const BItem &it, uint32_t tile, uint32_t step, uint32_t end, StreamDesc *S,
+                                          uint32_t *status, unsigned char *smem)
 {
 #define GTSC_ES_SWITCH(CALL)                       \
     switch (it.es) {                               \
@@ -2212,7 +2334,7 @@ __device__ __forceinline__ void run_stage(const BItem &it, uint32_t tile, Stream
     if constexpr (OP == B_MINMAX) { GTSC_ES_SWITCH(p_minmax<E>(it, tile, S)) }
     else if constexpr (OP == B_DELTA_ENC) { GTSC_ES_SWITCH(p_delta_enc<E>(it, tile, S)) }
     else if constexpr (OP == B_SCALE_SUB) { GTSC_ES_SWITCH(p_scale_sub<E>(it, tile, S)) }
-    else if constexpr (OP == B_AFL_PACK) { GTSC_ES_SWITCH(p_afl_pack<E>(it, tile, S, (unsigned long long *)smem)) }
+    else if constexpr (OP == B_AFL_PACK) { GTSC_ES_SWITCH(p_afl_pack<E>(it, tile, step, end, S, smem)) }
     else if constexpr (OP == B_HIST_SAMPLE) { GTSC_ES_SWITCH(p_hist_sample<E>(it, S, smem)) }
     else if constexpr (OP == B_HIST) { GTSC_ES_SWITCH(p_hist_count<E>(it, tile, S, smem)) }
     else if constexpr (OP == B_TOPK) { GTSC_ES_SWITCH(p_cand_top<E>(it, S)) }
@@ -2222,8 +2344,8 @@ __device__ __forceinline__ void run_stage(const BItem &it, uint32_t tile, Stream
         if (*CandArea(it).flag) { GTSC_ES_SWITCH(topk_blocks<E>(it, tile, it.tiles, S)) }
     }
     else if constexpr (OP == B_VMETA) { GTSC_ES_SWITCH(p_vmeta<E>(it, S)) }
-    else if constexpr (OP == B_SPLIT_COUNT) { p_split_count(it, tile, S); }
-    else if constexpr (OP == B_SPLIT) { GTSC_ES_SWITCH(p_split<E>(it, tile, S, smem)) }
+    else if constexpr (OP == B_SPLIT_COUNT) { p_split_count(it, tile, step, end, S); }
+    else if constexpr (OP == B_SPLIT) { GTSC_ES_SWITCH(p_split<E>(it, tile, step, end, S, smem)) }
     else if constexpr (OP == B_RLE_HEADS) { GTSC_ES_SWITCH(p_rle_heads<E>(it, tile, S, smem)) }
     else if constexpr (OP == B_RLE_LENGTHS) { p_rle_lengths(it, tile, S); }
     else if constexpr (OP == B_F2I_STATS) { GTSC_ES_SWITCH(p_f2i_stats<E>(it, tile, S)) }
@@ -2278,7 +2400,7 @@ __global__ void __launch_bounds__(kBThreads, 4) k_bpersist_c(PersistArgs a)
         a, [](int op, const BItem &it, const StreamDesc *S) { return persist_extent_c(op, it, S); },
         [&](int op, const BItem &it, uint32_t tile) {
         switch (op) {
-#define GTSC_RUN(OPC) case OPC: run_stage<OPC>(it, tile, a.S, a.status, smem); break;
+#define GTSC_RUN(OPC) case OPC: run_stage<OPC>(it, tile, 1, tile + 1, a.S, a.status, smem); break;
             GTSC_RUN(B_MINMAX)
             GTSC_RUN(B_DELTA_ENC)
             GTSC_RUN(B_SCALE_SUB)

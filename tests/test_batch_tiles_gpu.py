@@ -111,3 +111,21 @@ def test_delta_edges(G, O, rng, dt):
             dts.append(dt)
             trees.append(G.tree_from_path(paths[(n + bits) % len(paths)], dt))
     run_batch(G, O, cols, dts, trees)
+
+
+@pytest.mark.parametrize("dt", [OR.CHAR, OR.SHORT, OR.INT, OR.TIME], ids=["char", "short", "int", "time"])
+def test_pack_edges(G, O, rng, dt):
+    """AFL packing around its 512-value units and 4096-value tiles, of every kind of width, read plainly and
+    through views"""
+    w = 8 * np.dtype(OR.NP_TYPES[dt]).itemsize
+    cols, dts, trees = [], [], []
+    for n in [1, 31, 511, 512, 513, 4095, 4096, 4097, 12289, 50001]:
+        for bits in sorted({1, 2, 3, 5, 7, w // 4, w // 4 + 1, w // 2, w // 2 + 1, w - 1, w}):
+            for path in [[OR.AFL, OR.NONE], [OR.SCALE, OR.AFL, OR.NONE], [OR.DELTA, OR.AFL, OR.NONE]]:
+                if n > 5000 and bits not in (1, 5, w // 2 + 1, w):
+                    continue
+                x = rng.integers(0, 1 << min(bits, 62), n, dtype=np.int64)
+                cols.append((-x if bits == w else x).astype(OR.NP_TYPES[dt]))
+                dts.append(dt)
+                trees.append(G.tree_from_path(path, dt))
+    run_batch(G, O, cols, dts, trees)
