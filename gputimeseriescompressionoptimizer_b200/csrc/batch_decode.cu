@@ -257,7 +257,7 @@ __device__ __forceinline__ unsigned long long delta_unit_sum(const DViewCtx &dv,
 }
 
 template <int ES>
-__device__ void p_delta_sum(const BItem &it, uint32_t tile, StreamDesc *S)
+__device__ void p_delta_sum(const BItem &it, uint32_t tile, uint32_t step, uint32_t end, StreamDesc *S)
 {
     constexpr uint32_t WARPS = kBThreads / 32;
     __shared__ unsigned long long s_sum[WARPS];
@@ -265,15 +265,19 @@ __device__ void p_delta_sum(const BItem &it, uint32_t tile, StreamDesc *S)
     DViewCtx dv = dview_ctx<ES>(it, S, 1, ok);
     if (!ok) dv.n = 0;
     const uint32_t warp = threadIdx.x >> 5;
-    const uint64_t unit = (uint64_t)tile * WARPS + warp;
-    unsigned long long x = delta_unit_sum<ES>(dv, unit);
     const DeltaSums ds(it);
-    if ((threadIdx.x & 31) == 0) ds.units[unit] = s_sum[warp] = x;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (uint32_t w = 1; w < WARPS; w++) x += s_sum[w];
-        ds.tiles[tile] = x;
-        atomicAdd(ds.groups + tile / kBDeltaGroup, x);
+#pragma unroll 1
+    for (; tile < end; tile += step) {
+        const uint64_t unit = (uint64_t)tile * WARPS + warp;
+        unsigned long long x = delta_unit_sum<ES>(dv, unit);
+        __syncthreads();  // the sums of the tile before are read
+        if ((threadIdx.x & 31) == 0) ds.units[unit] = s_sum[warp] = x;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (uint32_t w = 1; w < WARPS; w++) x += s_sum[w];
+            ds.tiles[tile] = x;
+            atomicAdd(ds.groups + tile / kBDeltaGroup, x);
+        }
     }
 }
 
@@ -335,7 +339,7 @@ __device__ __forceinline__ void delta_unit(const UnitSrc<ES> &u, word_t<ES> acc,
 
 // Delta decode, second pass (C bytes of differences read again, n * s written).  Before, one pass kept
 // 16 unpacked values a thread behind a look-back, and its blocked stores touched half sectors.  2^26
-// int32 in 5 bits, both passes: 0.400 -> 0.195 ms (0.115 of it here); the 256 mixed columns' delta decodes
+// int32 in 5 bits, both passes: 0.400 -> 0.178 ms (0.115 of it here); the 256 mixed columns' delta decodes
 // 0.84 -> 0.72 ms.  Tried: four tiles a block behind one setup (long columns 3 % faster, short ones twice
 // as slow); blocks of short columns summing what lies before them instead of a pass (no faster).
 template <int ES>
@@ -1058,9 +1062,16 @@ __device__ __forceinline__ uint32_t dec_extent(const BItem &it, const StreamDesc
     return (uint32_t)(e < it.tiles ? e : it.tiles);
 }
 
+// `step`, `end`: passes that loop over an item's tiles themselves (dec_item_loop) run tile, tile + step, ...
+// below end; the others run `tile`
 template <int OP>
-__device__ __forceinline__ void run_dec(const BItem &it, uint32_t tile, StreamDesc *S, uint32_t *status,
-                                        unsigned char *smem);
+__device__ __forceinline__ void run_dec(const BItem &it, uint32_t tile, uint32_t step, uint32_t end, StreamDesc *S,
+                                        uint32_t *status, unsigned char *smem);
+
+// passes that set up (streams, views, widths: a chain of dependent loads) once for all of a block's tiles of
+// an item: the sums of 2^26 packed differences 0.079 -> 0.063 ms.  (The delta decode and the merge lost by
+// it on tables of many columns: 0.397 -> 0.418 and, with spills, 0.63 -> 0.78 ms.)
+constexpr bool dec_item_loop(int op) { return op == B_DELTA_SUM; }
 
 constexpr bool dec_persistent(int op)
 {
@@ -1088,7 +1099,7 @@ k_bdec(const BItem *items, const uint32_t *item_of, StreamDesc *S, uint32_t *cou
         uint32_t tile;
         const BItem &it = locate<DYN>(items, item_of, counter, tile);
         if (tile >= it.tiles) return;
-        run_dec<OP>(it, tile, S, status, smem);
+        run_dec<OP>(it, tile, 1, tile + 1, S, status, smem);
     } else {
         uint32_t t = blockIdx.x;
         uint32_t cur = 0xffffffffu;  // the item in the shared descriptor
@@ -1101,13 +1112,15 @@ k_bdec(const BItem *items, const uint32_t *item_of, StreamDesc *S, uint32_t *cou
             }
             const BItem &it = shared_item_ref();
             const uint32_t tile = t - (uint32_t)it.tile_base;
-            if (tile >= dec_extent<OP>(it, S)) {
+            const uint32_t extent = dec_extent<OP>(it, S);
+            if (tile >= extent) {
                 const uint64_t next = it.tile_base + it.tiles;
                 if (next >= total_tiles) break;
                 t = (uint32_t)(next + (blockIdx.x + gridDim.x - next % gridDim.x) % gridDim.x);
                 continue;
             }
-            run_dec<OP>(it, tile, S, status, smem);
+            run_dec<OP>(it, tile, gridDim.x, extent, S, status, smem);
+            if constexpr (dec_item_loop(OP)) t += (extent - 1 - tile) / gridDim.x * gridDim.x;
             __syncthreads();
             t += gridDim.x;
         }
@@ -1115,8 +1128,8 @@ k_bdec(const BItem *items, const uint32_t *item_of, StreamDesc *S, uint32_t *cou
 }
 
 template <int OP>
-__device__ __forceinline__ void run_dec(const BItem &it, uint32_t tile, StreamDesc *S, uint32_t *status,
-                                        unsigned char *smem)
+__device__ __forceinline__ void run_dec(const BItem &it, uint32_t tile, uint32_t step, uint32_t end, StreamDesc *S,
+                                        uint32_t *status, unsigned char *smem)
 {
 #define GTSC_ES_SWITCH(CALL)                       \
     switch (it.es) {                               \
@@ -1127,7 +1140,7 @@ __device__ __forceinline__ void run_dec(const BItem &it, uint32_t tile, StreamDe
     }
     if constexpr (OP == B_NONE_COPY) p_none_copy(it, tile, S, status);
     else if constexpr (OP == B_AFL_UNPACK) { GTSC_ES_SWITCH(p_afl_unpack<E>(it, tile, S, status)) }
-    else if constexpr (OP == B_DELTA_SUM) { GTSC_ES_SWITCH(p_delta_sum<E>(it, tile, S)) }
+    else if constexpr (OP == B_DELTA_SUM) { GTSC_ES_SWITCH(p_delta_sum<E>(it, tile, step, end, S)) }
     else if constexpr (OP == B_DELTA_DEC) { GTSC_ES_SWITCH(p_delta_dec<E>(it, tile, S, status)) }
     else if constexpr (OP == B_SCALE_ADD) { GTSC_ES_SWITCH(p_scale_add<E>(it, tile, S, status)) }
     else if constexpr (OP == B_MERGE) { GTSC_ES_SWITCH(p_merge<E>(it, tile, S, status)) }
@@ -1170,7 +1183,7 @@ __global__ void __launch_bounds__(kBThreads, 4) k_bpersist_d(PersistArgs a)
         a, [](int op, const BItem &it, const StreamDesc *S) { return persist_extent_d(op, it, S); },
         [&](int op, const BItem &it, uint32_t tile) {
             switch (op) {
-#define GTSC_RUN(OPC) case OPC: run_dec<OPC>(it, tile, a.S, a.status, smem); break;
+#define GTSC_RUN(OPC) case OPC: run_dec<OPC>(it, tile, 1, tile + 1, a.S, a.status, smem); break;
                 GTSC_RUN(B_NONE_COPY)
                 GTSC_RUN(B_AFL_UNPACK)
                 GTSC_RUN(B_DELTA_SUM)
