@@ -30,6 +30,44 @@ __global__ void k_set_streams(const unsigned long long *vals, const int *sids, i
     S[sids[i]].len = vals[2 * i + 1];
 }
 
+// a run of equal entries of a tile -> item table
+struct TileRun {
+    uint64_t at;  // in d_item_of
+    uint32_t tiles, item;
+};
+
+// bytes to set to one value (multiples of 16, 16-byte aligned)
+struct FillRange {
+    uint64_t at, bytes;
+    uint64_t value;  // 0 or all ones
+};
+
+constexpr uint64_t kLongFill = 16 << 20;  // ranges from here on by memset
+
+// any grid: pieces of 16 KB, the ranges' first pieces on blocks in turn
+__global__ void __launch_bounds__(256) k_fill_ranges(const FillRange *ranges, int n, uint8_t *base)
+{
+    for (int k = 0; k < n; k++) {
+        const FillRange r = ranges[k];
+        const uint4 v = make_uint4((uint32_t)r.value, (uint32_t)r.value, (uint32_t)r.value, (uint32_t)r.value);
+        const uint64_t q = r.bytes / 16;
+        uint4 *p = (uint4 *)(base + r.at);
+        for (uint64_t i = (blockIdx.x + k) % gridDim.x * 1024ull; i < q; i += gridDim.x * 1024ull)
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const uint64_t at = i + j * 256 + threadIdx.x;
+                if (at < q) p[at] = v;
+            }
+    }
+}
+
+// one block a run
+__global__ void k_fill_tiles(const TileRun *runs, uint32_t *item_of)
+{
+    const TileRun r = runs[blockIdx.x];
+    for (uint32_t t = threadIdx.x; t < r.tiles; t += blockDim.x) item_of[r.at + t] = r.item;
+}
+
 uint64_t align_up(uint64_t x, uint64_t a) { return (x + a - 1) / a * a; }
 uint64_t cdiv(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
 bool aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
@@ -90,7 +128,7 @@ struct Launch {
     int op;
     int first, count;
     uint64_t tiles;
-    uint64_t map_off;  // this launch's tile -> item table in the item_of array
+    uint64_t map_off;  // this launch's tile -> item table (look-back passes: claim table) in d_item_of
     int level;
     std::vector<int> after;  // the launches of this one's columns at each column's level before
     bool last = true;        // no launch comes after it
@@ -132,7 +170,7 @@ public:
     std::vector<BItem> items_c, items_d, items_copy;
     std::vector<int> item_col_c, item_col_d;  // each item's column
     std::vector<Launch> launch_c, launch_d;
-    // the persistent schedule (batch.hpp, PUnit) of each phase
+    // the persistent schedule (batch.hpp, PUnit) of each phase, once it is asked for
     std::vector<PUnit> punit_c, punit_d;
     std::vector<PItem> pitem_c, pitem_d;
     uint32_t q_total_c = 0, q_total_d = 0;
@@ -144,14 +182,16 @@ public:
     uint32_t hist_tile = 0;       // the histogram tile in use
     std::vector<BatchColumn> src_cols;  // the columns (current inputs) and trees, for re-tuning
     std::vector<Tree> src_trees;
-    std::vector<uint32_t> item_of;           // tile -> item tables of every launch, back to back
+    std::vector<uint32_t> claims;            // (item, tile) of every claim of the look-back launches
     uint64_t copy_map_off = 0;
     uint32_t *d_item_of = nullptr;
     uint64_t copy_tiles = 0, framed_cap = 0;
     std::vector<unsigned long long> zero_c, zero_d;  // (ptr, bytes) pairs
-    std::vector<std::pair<uint64_t, uint64_t>> hist_tables;  // (offset, cap) to initialise
 
-    DevBuf arena, tables;
+    DevBuf arena, tables, persist_tables;
+    std::vector<FillRange> long_clear;
+    FillRange *d_clear = nullptr;
+    int n_clear = 0, device = 0;
     StreamDesc *d_streams = nullptr;
     BItem *d_items_c = nullptr, *d_items_d = nullptr, *d_items_copy = nullptr;
     BColumnDev *d_cols = nullptr;
@@ -177,7 +217,10 @@ public:
     int folded_minmax(int id) const;
     void plan_passes();
     void layout(cudaStream_t s);
-    void capture(cudaStream_t s);
+    void plan_clear(std::vector<FillRange> &ranges, uint64_t bytes);
+    void clear_arena(cudaStream_t s) const;
+    void capture(cudaStream_t s, bool pers);
+    void prepare_persistent();
     void record_compress(cudaStream_t s, const std::function<void(int)> &mark, bool pers);
     void record_decompress(cudaStream_t s, const std::function<void(int)> &mark, bool pers);
     void plan_persistent(const std::vector<Launch> &launches, const std::vector<BItem> &items,
@@ -539,6 +582,15 @@ void BatchEngine::plan_passes()
         nd.last_c_level = ps.empty() ? start - 1 : lvl - 1;
     }
 
+    // The metadata of every node read through a view in one launch, at the last of their levels: no pass
+    // waits for it, and each launch on its own is a branch of the step's graph, which costs its creation
+    // about as much as five launches in a row.
+    int vmeta_level = 0;
+    for (const Pass &p : pass_c)
+        if (p.op == B_VMETA) vmeta_level = std::max(vmeta_level, p.level);
+    for (Pass &p : pass_c)
+        if (p.op == B_VMETA) p.level = vmeta_level;
+
     // ---------------- decode passes (children before parents)
     std::vector<int> order(nodes.size());
     for (size_t i = 0; i < nodes.size(); i++) order[i] = (int)i;
@@ -696,7 +748,6 @@ void BatchEngine::layout(cudaStream_t s)
     const uint64_t framed_off = off;
     off += align_up(framed_cap + 64, 256);
     arena = dev_alloc(off, s);
-    GTSC_CUDA(cudaMemsetAsync(arena.get(), 0, off, s));
     uint8_t *A = arena.get();
     d_framed = A + framed_off;
     for (size_t i = 0; i < streams.size(); i++)
@@ -712,12 +763,15 @@ void BatchEngine::layout(cudaStream_t s)
         streams[col_in_sid[c]].len = col_bytes[c];
         streams[col_out_sid[c]].cap = col_bytes[c];
     }
-    // hash tables start empty: keys all ones
-    for (auto &nd : nodes)
-        if (nd.tab_cap) {
-            GTSC_CUDA(cudaMemsetAsync(A + nd.scratch + nd.tab_off + 16, 0xff, 8 * nd.tab_cap, s));
-        }
-
+    // The tile -> item tables of the launches, back to back: a number a tile, millions for a large table,
+    // so the device writes them (k_fill_tiles).  Built and uploaded by the host they took a third of the
+    // creation of 256 columns up to 16 Mi values.
+    std::vector<TileRun> runs;
+    uint64_t map_tiles = 0;
+    auto add_map = [&](uint32_t tiles, int k) {
+        runs.push_back(TileRun{map_tiles, tiles, (uint32_t)k});
+        map_tiles += tiles;
+    };
     // items: patch scratch offsets into device addresses, group into launches
     auto build = [&](std::vector<Pass> &ps, std::vector<BItem> &items, std::vector<Launch> &launches,
                      std::vector<int> &item_col) {
@@ -745,11 +799,10 @@ void BatchEngine::layout(cudaStream_t s)
                 j++;
             }
             L.count = (int)items.size() - L.first;
-            L.map_off = item_of.size();
-            for (int k = 0; k < L.count; k++) item_of.insert(item_of.end(), items[L.first + k].tiles, (uint32_t)k);
             if (dyn_pass(L.op)) {
                 // claim order: tile j of every item before tile j + 1 of any, so the tiles in flight
                 // spread over the items' look-back chains instead of queueing on one
+                L.map_off = claims.size();
                 std::vector<int> live(L.count);
                 for (int k = 0; k < L.count; k++) live[k] = k;
                 for (uint32_t j = 0; !live.empty(); j++) {
@@ -757,13 +810,16 @@ void BatchEngine::layout(cudaStream_t s)
                     for (int k : live) {
                         const BItem &b = items[L.first + k];
                         if (j < b.tiles) {
-                            item_of.push_back((uint32_t)k);
-                            item_of.push_back(j);
+                            claims.push_back((uint32_t)k);
+                            claims.push_back(j);
                             live[w++] = k;
                         }
                     }
                     live.resize(w);
                 }
+            } else {
+                L.map_off = map_tiles;
+                for (int k = 0; k < L.count; k++) add_map(items[L.first + k].tiles, k);
             }
             launches.push_back(L);
             i = j;
@@ -773,8 +829,6 @@ void BatchEngine::layout(cudaStream_t s)
     build(pass_d, items_d, launch_d, item_col_d);
     plan_order(launch_c, item_col_c);
     plan_order(launch_d, item_col_d);
-    plan_persistent(launch_c, items_c, item_col_c, punit_c, pitem_c, q_total_c);
-    plan_persistent(launch_d, items_d, item_col_d, punit_d, pitem_d, q_total_d);
 
     // zero ranges per step
     auto zr = [](std::vector<unsigned long long> &z, uint8_t *p, uint64_t bytes) {
@@ -839,8 +893,14 @@ void BatchEngine::layout(cudaStream_t s)
             items_copy.push_back(it);
         }
     }
-    copy_map_off = item_of.size();
-    for (size_t k = 0; k < items_copy.size(); k++) item_of.insert(item_of.end(), items_copy[k].tiles, (uint32_t)k);
+    copy_map_off = map_tiles;
+    for (size_t k = 0; k < items_copy.size(); k++) add_map(items_copy[k].tiles, (int)k);
+    // the claim tables lie before the tile tables
+    copy_map_off += claims.size();
+    for (auto *v : {&launch_c, &launch_d})
+        for (Launch &L : *v)
+            if (!dyn_pass(L.op)) L.map_off += claims.size();
+    for (TileRun &r : runs) r.at += claims.size();
     // counters: one per launch
     n_counters = (int)(launch_c.size() + launch_d.size()) + 4;
 
@@ -865,12 +925,13 @@ void BatchEngine::layout(cudaStream_t s)
     const uint64_t o_frame = t_off; t_off += 256;
     const uint64_t o_status = t_off; t_off += 256;
     const uint64_t o_counters = t_off; t_off += sz(n_counters, 4);
-    const uint64_t o_item_of = t_off; t_off += sz(item_of.size(), 4);
+    const uint64_t o_item_of = t_off; t_off += sz(claims.size() + map_tiles, 4);
+    const uint64_t o_runs = t_off; t_off += sz(runs.size(), sizeof(TileRun));
+    std::vector<FillRange> clear;
+    plan_clear(clear, arena.bytes);
+    n_clear = (int)clear.size();
+    const uint64_t o_clear = t_off; t_off += sz(clear.size(), sizeof(FillRange));
     const uint64_t ncol = col_root.size();
-    const uint64_t o_plc = t_off; t_off += sz(punit_c.size(), sizeof(PUnit));
-    const uint64_t o_pld = t_off; t_off += sz(punit_d.size(), sizeof(PUnit));
-    const uint64_t o_pic = t_off; t_off += sz(pitem_c.size(), sizeof(PItem));
-    const uint64_t o_pid = t_off; t_off += sz(pitem_d.size(), sizeof(PItem));
     const uint64_t o_done_c = t_off; t_off += sz(ncol, 4);
     const uint64_t o_done_d = t_off; t_off += sz(ncol, 4);
     const uint64_t o_ext_c = t_off; t_off += sz(items_c.size(), 4);
@@ -898,10 +959,6 @@ void BatchEngine::layout(cudaStream_t s)
     d_status = (uint32_t *)(T + o_status);
     d_counters = (uint32_t *)(T + o_counters);
     d_item_of = (uint32_t *)(T + o_item_of);
-    d_punit_c = (PUnit *)(T + o_plc);
-    d_punit_d = (PUnit *)(T + o_pld);
-    d_pitem_c = (PItem *)(T + o_pic);
-    d_pitem_d = (PItem *)(T + o_pid);
     d_done_c = (uint32_t *)(T + o_done_c);
     d_done_d = (uint32_t *)(T + o_done_d);
     d_ext_c = (uint32_t *)(T + o_ext_c);
@@ -931,12 +988,41 @@ void BatchEngine::layout(cudaStream_t s)
     h2d(d_nodes_d, nodes_d.data(), nodes_d.size() * sizeof(BNodeDev));
     h2d(d_zero_c, zero_c.data(), zero_c.size() * 8);
     h2d(d_zero_d, zero_d.data(), zero_d.size() * 8);
-    h2d(d_item_of, item_of.data(), item_of.size() * 4);
-    h2d(d_punit_c, punit_c.data(), punit_c.size() * sizeof(PUnit));
-    h2d(d_punit_d, punit_d.data(), punit_d.size() * sizeof(PUnit));
-    h2d(d_pitem_c, pitem_c.data(), pitem_c.size() * sizeof(PItem));
-    h2d(d_pitem_d, pitem_d.data(), pitem_d.size() * sizeof(PItem));
+    h2d(d_item_of, claims.data(), claims.size() * 4);
+    h2d(T + o_runs, runs.data(), runs.size() * sizeof(TileRun));
+    d_clear = (FillRange *)(T + o_clear);
+    h2d(d_clear, clear.data(), clear.size() * sizeof(FillRange));
+    k_fill_tiles<<<(unsigned)runs.size(), 256, 0, s>>>((const TileRun *)(T + o_runs), d_item_of);
+    GTSC_CUDA(cudaGetLastError());
     GTSC_CUDA(cudaStreamSynchronize(s));
+}
+
+// The arena's first contents: zeros, and empty hash tables (keys all ones).  Each byte is set once, and a
+// table's list of used slots is not.  Long ranges by memset (7.3 TB/s, the kernel 4.9), the others in one
+// launch, as a table of many dict / const nodes has hundreds (as memsets 0.3 ms of the host's time for 64
+// short columns).
+void BatchEngine::plan_clear(std::vector<FillRange> &ranges, uint64_t bytes)
+{
+    uint64_t done = 0;
+    auto fill = [&](uint64_t from, uint64_t to, uint64_t value) {
+        if (to > from) (to - from >= kLongFill ? long_clear : ranges).push_back(FillRange{from, to - from, value});
+    };
+    for (auto &nd : nodes)  // in scratch order
+        if (nd.tab_cap) {
+            const uint64_t keys = nd.scratch + nd.tab_off + 16, counts = keys + 8 * nd.tab_cap;
+            fill(done, keys, 0);
+            fill(keys, counts, ~0ull);
+            fill(counts, counts + 4 * nd.tab_cap, 0);
+            done = counts + 8 * nd.tab_cap;
+        }
+    fill(done, bytes, 0);
+}
+
+void BatchEngine::clear_arena(cudaStream_t s) const
+{
+    for (const FillRange &r : long_clear) GTSC_CUDA(cudaMemsetAsync(arena.get() + r.at, (int)(r.value & 0xff), r.bytes, s));
+    if (n_clear) k_fill_ranges<<<8 * sm_count(), 256, 0, s>>>(d_clear, n_clear, arena.get());
+    GTSC_CUDA(cudaGetLastError());
 }
 
 // What each launch of a phase waits for: a pass depends only on passes of its own column at lower
@@ -953,6 +1039,11 @@ void BatchEngine::plan_order(std::vector<Launch> &launches, const std::vector<in
         Launch &L = launches[i];
         for (int k = L.first; k < L.first + L.count; k++) {
             Seen &c = seen[item_col[k]];
+            if (L.op == B_VMETA) {  // after what the column ran at lower levels; nothing waits for it
+                const std::vector<int> &b = c.level != L.level ? c.now : c.before;
+                L.after.insert(L.after.end(), b.begin(), b.end());
+                continue;
+            }
             if (c.level != L.level) {  // launches are sorted by level
                 c.before.swap(c.now);
                 c.now.clear();
@@ -1039,11 +1130,12 @@ void BatchEngine::plan_persistent(const std::vector<Launch> &launches, const std
         }
         const bool dyn = dyn_pass(L.op);
         const uint32_t per = dyn ? 1u : kPersistChunk;
+        int at = L.first;  // the item of tile t
         for (uint64_t t = 0; t < L.tiles; t += per) {
-            // the unit's first tile: look-back passes in the launch's claim order (the claim table
-            // behind its tile table), the others in tile order
-            const int gi = L.first + (int)item_of[L.map_off + (dyn ? L.tiles + 2 * t : t)];
-            const uint64_t tile = dyn ? item_of[L.map_off + L.tiles + 2 * t + 1] : t - items[gi].tile_base;
+            // the unit's first tile: look-back passes in the launch's claim order, the others in tile order
+            while (!dyn && t >= items[at].tile_base + items[at].tiles) ++at;
+            const int gi = dyn ? L.first + (int)claims[L.map_off + 2 * t] : at;
+            const uint64_t tile = dyn ? claims[L.map_off + 2 * t + 1] : t - items[gi].tile_base;
             const uint32_t cnt = (uint32_t)std::min<uint64_t>(per, L.tiles - t);
             if (tile >= (1u << 28)) fail(GTSC_ERR_CAPACITY, "batch: an item has too many tiles for the persistent schedule");
             units.push_back(PUnit{(uint32_t)gi, (uint32_t)tile | (cnt << 28)});
@@ -1114,10 +1206,9 @@ void BatchEngine::record_decompress(cudaStream_t s, const std::function<void(int
     record_launches(launch_d, d_items_d, (int)launch_c.size(), s, mark);
 }
 
-void BatchEngine::capture(cudaStream_t s)
+void BatchEngine::capture(cudaStream_t s, bool pers)
 {
-    for (int which = 0; which < 4; which++) {
-        const bool comp = which % 2 == 0, pers = which >= 2;
+    for (const bool comp : {true, false}) {
         cudaGraph_t g;
         GTSC_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         try {
@@ -1131,10 +1222,62 @@ void BatchEngine::capture(cudaStream_t s)
         }
         GTSC_CUDA(cudaStreamEndCapture(s, &g));
         cudaGraphExec_t ex;
-        GTSC_CUDA(cudaGraphInstantiate(&ex, g, 0));
+        const cudaError_t made = cudaGraphInstantiate(&ex, g, 0);
         cudaGraphDestroy(g);
+        GTSC_CUDA(made);
         (comp ? graph_c : graph_d)[pers ? 1 : 0] = ex;
     }
+}
+
+// The persistent schedule's tables and graphs, when it is first asked for: most batches never replay it, and
+// it took a fifth of the creation of 256 columns up to 16 Mi values.  On the batch's device and a stream of
+// its own, and out of the way of a capture that the calling thread may have under way.
+void BatchEngine::prepare_persistent()
+{
+    if (graph_d[1]) return;
+    struct Guard {
+        int device = 0;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaStream_t s = nullptr;
+        ~Guard()
+        {
+            if (s) cudaStreamDestroy(s);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            cudaSetDevice(device);
+        }
+    } guard;
+    GTSC_CUDA(cudaGetDevice(&guard.device));
+    GTSC_CUDA(cudaThreadExchangeStreamCaptureMode(&guard.mode));
+    GTSC_CUDA(cudaSetDevice(device));
+    GTSC_CUDA(cudaStreamCreateWithFlags(&guard.s, cudaStreamNonBlocking));
+    const cudaStream_t s = guard.s;
+    if (graph_c[1]) cudaGraphExecDestroy(graph_c[1]);  // of a call that failed on its way
+    graph_c[1] = nullptr;
+    plan_persistent(launch_c, items_c, item_col_c, punit_c, pitem_c, q_total_c);
+    plan_persistent(launch_d, items_d, item_col_d, punit_d, pitem_d, q_total_d);
+    struct Part {
+        const void *src;
+        uint64_t bytes;
+        void **dst;
+    };
+    const Part parts[4] = {{punit_c.data(), punit_c.size() * sizeof(PUnit), (void **)&d_punit_c},
+                           {punit_d.data(), punit_d.size() * sizeof(PUnit), (void **)&d_punit_d},
+                           {pitem_c.data(), pitem_c.size() * sizeof(PItem), (void **)&d_pitem_c},
+                           {pitem_d.data(), pitem_d.size() * sizeof(PItem), (void **)&d_pitem_d}};
+    uint64_t bytes = 0;
+    for (const Part &q : parts) bytes += align_up(q.bytes + 16, 256);
+    persist_tables = dev_alloc(bytes, s);
+    persist_tables.release_on_default_stream();  // the stream ends with this call
+    uint8_t *p = persist_tables.get();
+    for (const Part &q : parts) {
+        *q.dst = p;
+        if (q.bytes) GTSC_CUDA(cudaMemcpyAsync(p, q.src, q.bytes, cudaMemcpyHostToDevice, s));
+        p += align_up(q.bytes + 16, 256);
+    }
+    GTSC_CUDA(cudaStreamSynchronize(s));
+    for (auto *v : {&punit_c, &punit_d}) std::vector<PUnit>().swap(*v);
+    for (auto *v : {&pitem_c, &pitem_d}) std::vector<PItem>().swap(*v);
+    capture(s, true);
 }
 
 // ---------------------------------------------------------------------------------- public
@@ -1156,6 +1299,7 @@ BatchEngine *batch_create(const std::vector<BatchColumn> &cols, const std::vecto
     if (tuning.hist_tile < 256 || tuning.hist_tile % 256 || tuning.hist_tile > kBHistTileMax)
         fail(GTSC_ERR_ARG, "batch: the histogram tile must be a multiple of 256");
     std::unique_ptr<BatchEngine> e(new BatchEngine());
+    GTSC_CUDA(cudaGetDevice(&e->device));
     e->tune = tuning;
     e->src_cols = cols;
     e->src_trees = trees;
@@ -1186,8 +1330,12 @@ BatchEngine *batch_create(const std::vector<BatchColumn> &cols, const std::vecto
     for (size_t c = 0; c < cols.size(); c++) sids.push_back(e->col_out_sid[c]);
     GTSC_CUDA(cudaMemcpyAsync(e->d_set_vals, vals.data(), vals.size() * 8, cudaMemcpyHostToDevice, s));
     GTSC_CUDA(cudaMemcpyAsync(e->d_set_sids, sids.data(), sids.size() * 4, cudaMemcpyHostToDevice, s));
+    // the arena is cleared (milliseconds for a large table) while the host instantiates the graphs; after the
+    // uploads, as a copy from pageable memory waits for what its stream has to do before it
+    e->clear_arena(s);
+    e->capture(s, false);
+    if (tuning.persistent_c || tuning.persistent_d) e->prepare_persistent();
     GTSC_CUDA(cudaStreamSynchronize(s));
-    e->capture(s);
     return e.release();
 }
 
@@ -1199,6 +1347,7 @@ void batch_destroy(BatchEngine *e)
     cudaDeviceSynchronize();
     e->arena.release_on_default_stream();
     e->tables.release_on_default_stream();
+    e->persist_tables.release_on_default_stream();
     for (int k = 0; k < 2; k++) {
         if (e->graph_c[k]) cudaGraphExecDestroy(e->graph_c[k]);
         if (e->graph_d[k]) cudaGraphExecDestroy(e->graph_d[k]);
@@ -1208,7 +1357,11 @@ void batch_destroy(BatchEngine *e)
 
 void batch_compress(BatchEngine *e, cudaStream_t s) { GTSC_CUDA(cudaGraphLaunch(e->graph_c[e->tune.persistent_c], s)); }
 
-void batch_set_schedule(BatchEngine *e, bool persistent) { e->tune.persistent_c = e->tune.persistent_d = persistent; }
+void batch_set_schedule(BatchEngine *e, bool persistent)
+{
+    if (persistent) e->prepare_persistent();
+    e->tune.persistent_c = e->tune.persistent_d = persistent;
+}
 bool batch_schedule(const BatchEngine *e) { return e->tune.persistent_c && e->tune.persistent_d; }
 BatchTuning batch_tuning(const BatchEngine *e) { return e->tune; }
 
@@ -1436,12 +1589,12 @@ BatchEngine *batch_autotune(BatchEngine *e, cudaStream_t s, TuneReport *report)
         ms[1] = time_step(x, false, batch_output(x), fb, outs, s, 5);
         if (batch_status(x, s) != GTSC_OK) fail(GTSC_ERR_FORMAT, "autotune: a candidate step failed");
     };
-    // 1. the schedule of each step (both recorded in every batch: no rebuild)
+    // 1. the schedule of each step (no rebuild)
     BatchTuning best = e->tune;
     best.persistent_c = best.persistent_d = false;
     e->tune.persistent_c = e->tune.persistent_d = false;
     measure(e, rep.ms_default);
-    e->tune.persistent_c = e->tune.persistent_d = true;
+    batch_set_schedule(e, true);
     float pers[2];
     measure(e, pers);
     cands += 2;

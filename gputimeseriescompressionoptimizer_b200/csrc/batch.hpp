@@ -174,7 +174,7 @@ gtsc_status batch_status(BatchEngine *e, cudaStream_t s);
 // number of kernel launches in one compress / decompress step
 int batch_launches(BatchEngine *e, bool compress);
 // the schedule the steps replay: a launch per (level, pass kind), or one persistent launch per step
-// pulling tiles from a device queue (both are captured at creation; the default is the levels)
+// pulling tiles from a device queue (prepared when it is first chosen; the default is the levels)
 void batch_set_schedule(BatchEngine *e, bool persistent);
 bool batch_schedule(const BatchEngine *e);
 // one step run launch by launch with events between launches: per launch its pass kind (a BOp, or

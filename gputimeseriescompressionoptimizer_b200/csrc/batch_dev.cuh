@@ -646,10 +646,6 @@ __device__ __forceinline__ void load_dview(const DViewCtx &v, uint64_t base, uin
     for (int j = 0; j < VPT; j++) out[j] = base + j < v.n ? dview_elem<ES>(v, base + j) : 0;
 }
 
-// the stage kernel skeleton: finds this block's (item, tile).  DYN passes take tiles in claim
-// order from a counter (look-back needs every predecessor claimed first), the others use the
-// block index; item_of[t] is the item of global tile t (one table per launch), and for DYN launches
-// item_of[grid + c] is the tile taken by the c-th claim.
 // copies items[k] into the block's shared descriptor (every thread of the block calls it; the
 // caller makes sure no thread still reads the previous one); fields are then read from shared
 // memory instead of every thread loading the whole descriptor into registers
@@ -832,9 +828,11 @@ __device__ __forceinline__ void persist_loop(const PersistArgs &a, Extent extent
     if (threadIdx.x == 0) persist_flush(a, cur, pend);
 }
 
-// DYN launches: after the launch's tile -> item table (gridDim.x entries) comes its claim table, the
-// (item, tile) of every claim (items interleaved round-robin, each item's tiles in order): one load
-// behind the claim's atomic, as every dependent access before a tile's data delays its look-back chain.
+// The item and the tile of a block of a stage launch with a block a tile; item_of[t] is the item of the
+// launch's tile t.  Look-back launches (DYN) take tiles in claim order from a counter, as a tile waits for
+// its predecessors; their table holds the (item, tile) of every claim instead (items interleaved
+// round-robin, each item's tiles in order): one load behind the claim's atomic, as every dependent access
+// before a tile's data delays its look-back chain.
 template <bool DYN>
 __device__ __forceinline__ const BItem &locate(const BItem *items, const uint32_t *item_of, uint32_t *counter,
                                                uint32_t &tile)
@@ -843,7 +841,7 @@ __device__ __forceinline__ const BItem &locate(const BItem *items, const uint32_
     __shared__ uint32_t s_idx;
     if (threadIdx.x == 0) {
         if constexpr (DYN) {
-            const uint32_t *claim = item_of + gridDim.x + 2ull * atomicAdd(counter, 1u);
+            const uint32_t *claim = item_of + 2ull * atomicAdd(counter, 1u);
             s_idx = ldg(claim);
             s_tile = ldg(claim + 1);
         } else {

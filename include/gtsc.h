@@ -194,8 +194,9 @@ gtsc_status gtsc_batch_status(gtsc_batch *b, void *stream);
 /* kernel launches in one step (compress != 0: compress step) */
 int32_t gtsc_batch_launches(gtsc_batch *b, int32_t compress);
 /*
- * The schedule later steps replay (both are recorded at creation): GTSC_SCHEDULE_LEVELS = one launch
- * per (tree level, pass kind) over all columns; GTSC_SCHEDULE_PERSISTENT = one persistent launch per
+ * The schedule later steps replay: GTSC_SCHEDULE_LEVELS (recorded at creation) = one launch
+ * per (tree level, pass kind) over all columns; GTSC_SCHEDULE_PERSISTENT (recorded when it is first
+ * chosen) = one persistent launch per
  * step whose blocks pull (pass, tile) work from a device queue, each column's levels waiting only for
  * that column's earlier levels (then a compress step is 6 launches and a decompress step 4).  Both
  * give the same bytes.  The default is the levels; gtsc_batch_autotune picks by measurement.

@@ -19,7 +19,8 @@ def frame(blobs):
 
 
 def compressed(G, cols, trees):
-    b = G.Batch([G.to_device(x) for x in cols], [OR.INT] * len(cols), trees, G.Stream())
+    b = G.Batch(devs := [G.to_device(x) for x in cols], [OR.INT] * len(cols), trees, G.Stream())
+    b.keep = devs  # the batch reads its columns where they are
     b.compress()
     b.status()
     return b, framed_blobs(G, b)[3]
