@@ -330,14 +330,14 @@ int BatchEngine::folded_minmax(int id) const
 
 void BatchEngine::plan_passes()
 {
-    // The histogram tile: what leaves a few tiles for each of four resident blocks per SM, between
-    // kBHistTileMin (a smaller tile spends its time on its 5120 counters) and the tuned tile.  64 columns
+    // The histogram tile, where none is given: what leaves a few tiles for each of four resident blocks per
+    // SM, between kBHistTileMin (a smaller tile spends its time on its 5120 counters) and 32K.  64 columns
     // of 4 Ki to 64 Ki values: 32K tiles leave all but a few SMs idle (a launch takes 0.2 ms, 15 us at 4K).
     uint64_t hist_values = 0;
     for (auto &nd : nodes)
         if (nd.enc == GTSC_DICT || nd.enc == GTSC_CONST) hist_values += nd.in_cap / nd.es;
     const uint64_t share = align_up(cdiv(hist_values, 24 * (uint64_t)sm_count()), 1024);
-    hist_tile = (uint32_t)std::min<uint64_t>(tune.hist_tile, std::max<uint64_t>(share, kBHistTileMin));
+    hist_tile = tune.hist_tile ? tune.hist_tile : (uint32_t)std::clamp<uint64_t>(share, kBHistTileMin, kBHistTileMax);
     // scratch sizes
     for (auto &nd : nodes) {
         const uint64_t n = nd.in_cap / nd.es;
@@ -1296,7 +1296,7 @@ BatchEngine *batch_create(const std::vector<BatchColumn> &cols, const std::vecto
     if (tuning.minmax_tile < kMinMaxTileMin || tuning.minmax_tile % (256 * tuning.minmax_vpt) ||
         tuning.minmax_tile > (1u << 20))
         fail(GTSC_ERR_ARG, "batch: the min/max tile must be a multiple of 256 x its values per thread, 1K .. 1M");
-    if (tuning.hist_tile < 256 || tuning.hist_tile % 256 || tuning.hist_tile > kBHistTileMax)
+    if (tuning.hist_tile % 256 || tuning.hist_tile > kBHistTileMax)
         fail(GTSC_ERR_ARG, "batch: the histogram tile must be a multiple of 256");
     std::unique_ptr<BatchEngine> e(new BatchEngine());
     GTSC_CUDA(cudaGetDevice(&e->device));
@@ -1363,7 +1363,12 @@ void batch_set_schedule(BatchEngine *e, bool persistent)
     e->tune.persistent_c = e->tune.persistent_d = persistent;
 }
 bool batch_schedule(const BatchEngine *e) { return e->tune.persistent_c && e->tune.persistent_d; }
-BatchTuning batch_tuning(const BatchEngine *e) { return e->tune; }
+BatchTuning batch_tuning(const BatchEngine *e)
+{
+    BatchTuning t = e->tune;
+    t.hist_tile = e->hist_tile;  // the one in use
+    return t;
+}
 
 void batch_set_inputs(BatchEngine *e, const std::vector<const void *> &inputs, cudaStream_t s)
 {
@@ -1427,7 +1432,7 @@ static uint64_t item_bytes(const BItem &it, const std::vector<StreamDesc> &S)
     const uint64_t in = L(it.in[0]);
     switch (it.op) {
     case B_MINMAX: case B_HIST: case B_F2I_STATS: return in;
-    case B_TOPK: case B_HIST_SAMPLE: case B_HIST_FULL: case B_TOPK_FULL: case B_F2I_RAW: case B_GFC_SCAN: return 0;
+    case B_TOPK: case B_HIST_SAMPLE: case B_TOPK_FULL: case B_F2I_RAW: case B_GFC_SCAN: return 0;
     case B_DELTA_ENC: case B_SCALE_SUB: case B_AFL_PACK: case B_F2I_ENC: return in + L(it.out[0]) + L(it.out[1]);
     case B_SPLIT_COUNT: return in + L(it.out[0]);
     case B_SPLIT: return in + L(it.out[0]) + L(it.out[1]) + L(it.out[2]);
@@ -1473,6 +1478,12 @@ std::vector<BatchLaunchProfile> batch_profile(BatchEngine *e, bool compress, cud
         d2h(S.data(), e->d_streams, S.size() * sizeof(StreamDesc), s);
         unsigned long long total = 0;
         d2h(&total, e->d_total, 8, s);
+        auto bytes_of = [&](const BItem &it) -> uint64_t {
+            if (it.op != B_HIST_FULL) return item_bytes(it, S);
+            uint32_t flag = 0;  // the input is read where the candidates proved nothing
+            d2h(&flag, it.scratch + it.cand, 4, s);
+            return flag && it.in[0] >= 0 ? S[it.in[0]].len : 0;
+        };
         int li = 0;
         for (size_t k = 0; k < marks.size(); k++) {
             BatchLaunchProfile p{};
@@ -1481,14 +1492,14 @@ std::vector<BatchLaunchProfile> batch_profile(BatchEngine *e, bool compress, cud
             if (marks[k] >= 0) {
                 const Launch &L = compress ? e->launch_c[li] : e->launch_d[li];
                 const BItem *items = compress ? &e->items_c[L.first] : &e->items_d[L.first];
-                for (int j = 0; j < L.count; j++) p.bytes += item_bytes(items[j], S);
+                for (int j = 0; j < L.count; j++) p.bytes += bytes_of(items[j]);
                 p.blocks = L.tiles;
                 ++li;
             } else if (marks[k] == M_FRAME_COPY) {
                 p.bytes = 2 * total;
                 p.blocks = e->copy_tiles;
             } else if (marks[k] == M_PERSIST) {  // every pass of the step in one launch
-                for (const BItem &it : compress ? e->items_c : e->items_d) p.bytes += item_bytes(it, S);
+                for (const BItem &it : compress ? e->items_c : e->items_d) p.bytes += bytes_of(it);
                 p.blocks = compress ? e->q_total_c : e->q_total_d;
             }
             out.push_back(p);
@@ -1590,7 +1601,7 @@ BatchEngine *batch_autotune(BatchEngine *e, cudaStream_t s, TuneReport *report)
         if (batch_status(x, s) != GTSC_OK) fail(GTSC_ERR_FORMAT, "autotune: a candidate step failed");
     };
     // 1. the schedule of each step (no rebuild)
-    BatchTuning best = e->tune;
+    BatchTuning best = batch_tuning(e);
     best.persistent_c = best.persistent_d = false;
     e->tune.persistent_c = e->tune.persistent_d = false;
     measure(e, rep.ms_default);
@@ -1621,22 +1632,22 @@ BatchEngine *batch_autotune(BatchEngine *e, cudaStream_t s, TuneReport *report)
         }
     set_minmax_params(e, best.minmax_tile, best.minmax_vpt, s);
     e->tune.persistent_c = keep_c;
-    // 3. the histogram tile (it sizes the top-k pass's tiles: a rebuild per candidate)
+    // 3. the histogram tile (it sizes scratch: a rebuild per candidate), on the compress step: its launches
+    // run beside other columns', so their times one after another say little
     const bool has_hist = std::any_of(e->items_c.begin(), e->items_c.end(), [](const BItem &it) { return it.op == B_HIST; });
     if (has_hist) {
-        e->tune.persistent_c = false;
-        float best_h = time_passes(e, {B_HIST, B_TOPK, B_HIST_FULL, B_TOPK_FULL}, s, 3);
-        e->tune.persistent_c = keep_c;
-        for (uint32_t tile : {8192u, 16384u, 32768u}) {
-            if (tile == best.hist_tile) continue;
+        batch_compress(e, s);
+        float best_h = time_step(e, true, nullptr, 0, outs, s, 5);
+        for (uint32_t tile : {4096u, 8192u, 16384u, 32768u}) {
+            if (tile == e->hist_tile) continue;
             BatchTuning cand = best;
             cand.hist_tile = tile;
-            cand.persistent_c = false;
+            cand.persistent_d = false;
             BatchEngine *x = batch_create(e->src_cols, e->src_trees, s, cand);
             float t = 1e30f;
             try {
                 batch_compress(x, s);
-                t = time_passes(x, {B_HIST, B_TOPK, B_HIST_FULL, B_TOPK_FULL}, s, 3);
+                t = time_step(x, true, nullptr, 0, outs, s, 5);
             } catch (...) {
                 batch_destroy(x);
                 throw;
@@ -1651,7 +1662,7 @@ BatchEngine *batch_autotune(BatchEngine *e, cudaStream_t s, TuneReport *report)
     }
     // the tuned batch
     BatchEngine *out = e;
-    if (best.hist_tile != e->tune.hist_tile) {
+    if (best.hist_tile != e->hist_tile) {
         out = batch_create(e->src_cols, e->src_trees, s, best);
         batch_destroy(e);
     }

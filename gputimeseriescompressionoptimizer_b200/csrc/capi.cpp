@@ -232,6 +232,7 @@ struct gtsc_batch {
 
 static BatchTuning to_tuning(const gtsc_batch_tuning &t)
 {
+    if (!t.hist_tile) fail(GTSC_ERR_ARG, "batch: the histogram tile must be a multiple of 256");
     BatchTuning b;
     b.minmax_tile = t.minmax_tile;
     b.minmax_vpt = t.minmax_values_per_thread;

@@ -208,8 +208,9 @@ int32_t gtsc_batch_schedule(gtsc_batch *b);
 /*
  * Launch parameters of a batch, and the autotuner that chooses them (no counterpart in the
  * reference, whose launch configuration is fixed, core/execution_policy.hpp:14-49).  Tiles are
- * values per block tile.  Defaults: min/max tile 8192 with 16 values per thread, histogram tile
- * 32768, level schedule for both steps.
+ * values per block tile.  Defaults: min/max tile 8192 with 16 values per thread, a histogram tile
+ * of 4096 to 32768 by the columns, level schedule for both steps.  gtsc_batch_get_tuning gives the
+ * parameters in use.
  */
 typedef struct {
     uint32_t minmax_tile;               /* 1024 .. 16384, a multiple of 256 x the values per thread */
@@ -231,7 +232,7 @@ gtsc_status gtsc_batch_get_tuning(gtsc_batch *b, gtsc_batch_tuning *tuning);
 /*
  * Times candidate parameters on the batch's own columns and trees with CUDA events: the schedule of
  * each step; then the min/max tile (1K .. 16K) x values per thread (1 .. 16) on the min/max
- * launches; then the histogram tile (8K .. 32K) on the histogram and top-k launches (a rebuild
+ * launches; then the histogram tile (4K .. 32K) on the compress step (a rebuild
  * each); a candidate is kept when it is at least 2 % faster.  The batch keeps the best parameters
  * (its device buffers, the framed output included, may move: call gtsc_batch_output again).
  * Synchronises; a few seconds for hundreds of columns.  *report may be NULL.
