@@ -871,12 +871,16 @@ __device__ __forceinline__ void block_top4(Cand (&l)[4], Cand (&r)[4])
     }
 }
 
-// The item's blocks that have work -- one per 2048 table slots taken and NaN keys listed -- each take a
+// The item's blocks that have work -- one per 512 table slots taken and NaN keys listed -- each take a
 // slice of the used-slot list (and of the NaN lists), reduce it to a top-4, clear their slots for the
 // next step and write the top-4 to the partial list; the last one to finish (threadfence + counter)
-// merges the partials, writes the result and resets the header.
+// merges the partials, writes the result and resets the header.  A table of which a fifth is taken (one
+// larger than L2: a 32nd) is walked in order instead: 12 bytes a slot each way in whole lines, where the
+// list takes four scattered accesses a value.  2^26 different int32 (a quarter taken): 23.3 -> 0.7 ms.
 template <int ES>
 __device__ __forceinline__ void put_top(const BItem &it, StreamDesc *S, const Cand (&r)[4]);
+
+constexpr uint64_t kWalkCap = 1 << 22;  // slots (12 bytes each) of a table that L2 holds
 
 // block `tile` of `blocks`
 template <int ES>
@@ -887,7 +891,7 @@ __device__ __forceinline__ void topk_blocks(const BItem &it, uint32_t tile, uint
     const HTab t = htab(it);
     const Order o = (Order)it.order;
     const uint64_t used = *(volatile unsigned int *)&t.hdr->used, n = view_len(it, S), nan_n = 4 * ((n + it.p[3] - 1) / it.p[3]);
-    const uint64_t want = (used + nan_n + 2047) / 2048;
+    const uint64_t want = (used + nan_n + 511) / 512;
     if (blocks > it.tiles) blocks = it.tiles;  // the partial list holds one entry a histogram tile
     const uint32_t T = want > blocks ? blocks : want ? (uint32_t)want : 1u;
     if (tile >= T) return;
@@ -895,6 +899,29 @@ __device__ __forceinline__ void topk_blocks(const BItem &it, uint32_t tile, uint
     const uint64_t lo = (uint64_t)tile * slice, hi = lo + slice < used ? lo + slice : used;
     const uint64_t nlo = (uint64_t)tile * nslice, nhi = nlo + nslice < nan_n ? nlo + nslice : nan_n;
     Cand l[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}}, r[4];
+    if (used * (t.cap > kWalkCap ? 32 : 5) > t.cap) {
+        const uint64_t pairs = t.cap / 2, step = (uint64_t)T * kBThreads;
+        ulonglong2 *keys = (ulonglong2 *)t.keys;
+        uint2 *counts = (uint2 *)t.counts;
+        for (uint64_t i = (uint64_t)tile * kBThreads + threadIdx.x; i < pairs; i += 2 * step) {
+            ulonglong2 k[2];
+            uint2 c[2];
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const bool in = i + q * step < pairs;
+                k[q] = in ? keys[i + q * step] : make_ulonglong2(EMPTY, EMPTY);
+                c[q] = in ? counts[i + q * step] : make_uint2(0, 0);
+            }
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                if (k[q].x == EMPTY && k[q].y == EMPTY) continue;
+                keys[i + q * step] = make_ulonglong2(EMPTY, EMPTY);
+                counts[i + q * step] = make_uint2(0, 0);
+                if (k[q].x != EMPTY) cpush(l, Cand{order_key(k[q].x, ES, o), c[q].x});
+                if (k[q].y != EMPTY) cpush(l, Cand{order_key(k[q].y, ES, o), c[q].y});
+            }
+        }
+    } else
     for (uint64_t i = lo + threadIdx.x; i < hi; i += 4 * kBThreads) {
         unsigned int h[4], c[4];
         unsigned long long k[4];
@@ -951,7 +978,7 @@ __device__ __forceinline__ void topk_blocks(const BItem &it, uint32_t tile, uint
 // ------------------------------------------------------------------------------- candidates
 constexpr uint32_t kSampleSmem = 3072 * 12 + 4 * 512 + 4 * 64 + 16;
 // The most frequent values of a node, in most columns without a full histogram: a sample names up to
-// 128 candidates; one pass counts each candidate exactly and every other value in one of 4096 hash
+// 400 candidates; one pass counts each candidate exactly and every other value in one of 4096 hash
 // buckets; a bucket's count bounds the count of each value in it, so when the least of the k best
 // candidates occurs more often than the largest bucket, those k are the most frequent ones, ties
 // included.  (A NaN never equals another: each occurs once, and the four smallest are candidates too.)
@@ -986,16 +1013,21 @@ __device__ __forceinline__ uint32_t cand_hash(word_t<ES> v)
 }
 static_assert(kCandBuckets == 1u << 9 && kBCandCoarse == 1u << 12, "cand_hash's bits");
 
-// One block an item: 2048 values spread over the column into a table in shared memory, the most
-// frequent of them (at least twice, unless all distinct ones fit) into the candidate table, the most
-// frequent first, as a bucket holds two.
+// One block an item: 2048 values spread over the column into a table in shared memory, all of them if there
+// are at most 400 different ones, else the most frequent, up to 128, into the candidate table, the most
+// frequent first, as a bucket holds two.  With 128 in any case, columns of 256 equally frequent values never
+// proved anything (2^22 doubles of 256 values and 1 % others, dictionary: 258 us, now 110; before there were
+// candidates 204); with 400 in any case Zipf ids took longer.  Where the sample shows that the counting will
+// prove nothing it flags the item, and the full histogram starts without it (2^24 int16 of 1000 values:
+// 261 -> 217 us, before there were candidates 245).
 template <int ES>
 __device__ __forceinline__ void p_hist_sample(const BItem &it, StreamDesc *S, unsigned char *smem)
 {
     using K = word_t<ES>;
     using T = HistTable<ES>;
-    constexpr uint32_t SAMPLE = 2048, SLOTS = 3072, MOST = 128, HEAVY = 8;
+    constexpr uint32_t SAMPLE = 2048, SLOTS = 3072, ALL = 400, MOST = 128, HEAVY = 8;
     static_assert(SAMPLE == 1u << 11 && SLOTS * 12 + 4 * kCandBuckets + 4 * 64 + 16 <= kSampleSmem, "the sample's shared memory");
+    const CandArea area(it);
     K *keys = (K *)smem;
     uint32_t *counts = (uint32_t *)(smem + SLOTS * 8), *fill = counts + SLOTS, *of_count = fill + kCandBuckets,
              *least = of_count + 64;
@@ -1040,20 +1072,50 @@ __device__ __forceinline__ void p_hist_sample(const BItem &it, StreamDesc *S, un
     for (uint32_t i = threadIdx.x; i < SLOTS; i += kBThreads)
         if (counts[i]) atomicAdd(of_count + (counts[i] < 63 ? counts[i] : 63), 1u);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t sum = 0, c = 64;
-        while (c > 1 && sum + of_count[c - 1] <= MOST) sum += of_count[--c];
-        *least = c;  // the smallest count taken
+    if (threadIdx.x < 32) {
+        const uint32_t lane = threadIdx.x, k = (uint32_t)it.mode;
+        uint32_t lo = of_count[lane], hi = of_count[32 + lane];  // -> values that occur lane, 32 + lane times or more
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t x = __shfl_down_sync(0xffffffffu, lo, d), y = __shfl_down_sync(0xffffffffu, hi, d);
+            if (lane + d < 32) {
+                lo += x;
+                hi += y;
+            }
+        }
+        lo += __shfl_sync(0xffffffffu, hi, 0);
+        // the largest count that more than `most` values reach, 0 if none does
+        auto reached = [&](uint32_t most) -> uint32_t {
+            const uint32_t h = __ballot_sync(0xffffffffu, hi > most), l = __ballot_sync(0xffffffffu, lane && lo > most);
+            return h ? 63 - __clz(h) : l ? 31 - __clz(l) : 0;
+        };
+        const uint32_t distinct = __shfl_sync(0xffffffffu, lo, 1), two = __shfl_sync(0xffffffffu, lo, 2),
+                       three = __shfl_sync(0xffffffffu, lo, 3);
+        const uint32_t taken = distinct <= ALL ? 1 : reached(MOST) + 1, kth = reached(k - 1);
+        if (lane == 0) {
+            least[0] = taken;                    // the smallest count taken
+            least[1] = distinct > MOST ? 3 : 2;  // passes (few values leave no bucket short)
+            // The counting pass is for nothing when the k-th best is no better than chance among values of one
+            // frequency: of such, m1 of which occur once and m2 twice, about m1 l^(c-1) / c! occur c times,
+            // l = 2 m2 / m1 (over 400 of them: l below 6).  A k-th best of two is chance only if many others
+            // occur twice.
+            if (taken > 1 && kth < 63) {
+                const float m1 = (float)(distinct - two), l = m1 > 0 ? fminf(2 * (float)(two - three) / m1, 6.f) : 0.f;
+                const float enough = (float)k * (kth == 2 ? 4.f : 0.25f);
+                float chance = m1;
+                for (uint32_t j = 2; j <= kth && (chance >= enough || (float)j <= l); j++) chance *= __fdividef(l, (float)j);
+                if (chance >= enough) *area.flag = 1;
+            }
+        }
     }
     __syncthreads();
-    const uint32_t t = *least;
-    const CandArea area(it);
+    const uint32_t t = least[0], passes = t > 1 ? 2 : least[1];
     K *image = (K *)area.keys;
 #pragma unroll 1
-    for (int pass = 0; pass < 2; pass++) {
+    for (uint32_t pass = 0; pass < passes; pass++) {
         for (uint32_t i = threadIdx.x; i < SLOTS; i += kBThreads) {
             const uint32_t c = counts[i];
-            if (c < t || c == 0 || (c >= HEAVY) != (pass == 0)) continue;
+            if (c < t || c == 0 || pass != (c >= HEAVY ? 0 : c > 1 ? 1 : passes - 1)) continue;
             const uint32_t b = cand_hash<ES>(keys[i]) >> 23, w = atomicAdd(fill + b, 1u);
             if (w < 2) image[2 * b + w] = keys[i];
         }
@@ -1096,7 +1158,14 @@ __device__ __forceinline__ void cand_flush(const BItem &it, const unsigned char 
     if (threadIdx.x < 4 && nan[threadIdx.x]) cand_nan(area.nan, nan[threadIdx.x]);
 }
 
-// A tile of the counting pass (n * s read).
+// clears the code words of values [t0, end) (out1 after its 16 + 4*es header)
+__device__ __forceinline__ void clear_codes(const BItem &it, uint64_t t0, uint64_t end, StreamDesc *S)
+{
+    uint32_t *words = (uint32_t *)(S[it.out[1]].ptr + 16 + 4 * it.es);
+    for (uint64_t w = t0 / 16 + threadIdx.x; w < (end + 15) / 16; w += blockDim.x) words[w] = 0u;
+}
+
+// A tile of the counting pass (n * s read).  A dictionary's 2-bit code words are cleared by the way.
 template <int ES, bool FP>
 __device__ __forceinline__ void cand_tile_of(const BItem &it, uint32_t tile, StreamDesc *S, unsigned char *smem)
 {
@@ -1107,11 +1176,7 @@ __device__ __forceinline__ void cand_tile_of(const BItem &it, uint32_t tile, Str
     const uint64_t n = vc.n, HT = it.p[3], t0 = (uint64_t)tile * HT;
     if (t0 >= n) return;
     const uint64_t end = n < t0 + HT ? n : t0 + HT;
-    if (it.mode == 4) {
-        // dict: clear this tile's share of the 2-bit code words (out1 after its 16 + 4*es header)
-        uint32_t *words = (uint32_t *)(S[it.out[1]].ptr + 16 + 4 * ES);
-        for (uint64_t w = t0 / 16 + threadIdx.x; w < (end + 15) / 16; w += blockDim.x) words[w] = 0u;
-    }
+    if (it.mode == 4) clear_codes(it, t0, end, S);
     const uint32_t keys = (uint32_t)__cvta_generic_to_shared(smem), counts = keys + 8 * kBCandSlots;
     const uint32_t lane = threadIdx.x & 31;
     constexpr Order FO = ES == 8 ? ORD_F64 : ORD_F32;
@@ -1188,7 +1253,12 @@ __device__ __forceinline__ void cand_tile(const BItem &it, uint32_t tile, Stream
 template <int ES>
 __device__ __forceinline__ void p_hist_count(const BItem &it, uint32_t tile, StreamDesc *S, unsigned char *smem)
 {
-    if ((uint64_t)tile * it.p[3] >= view_len(it, S)) return;
+    const uint64_t n = view_len(it, S), t0 = (uint64_t)tile * it.p[3];
+    if (t0 >= n) return;
+    if (*CandArea(it).flag) {
+        if (it.mode == 4) clear_codes(it, t0, n < t0 + it.p[3] ? n : t0 + it.p[3], S);
+        return;
+    }
     cand_load<ES>(it, smem);
     __syncthreads();
     cand_tile<ES>(it, tile, S, smem);
@@ -1219,6 +1289,7 @@ __device__ __forceinline__ void p_cand_top(const BItem &it, StreamDesc *S)
     __shared__ uint32_t s_max;
     const CandArea area(it);
     const Order o = (Order)it.order;
+    const bool flagged = *area.flag != 0;  // already, by the sample
     if (threadIdx.x == 0) s_max = 0;
     __syncthreads();
     constexpr int PER = (int)(kBCandSlots / kBThreads), COARSE = (int)(kBCandCoarse / kBThreads / 4);
@@ -1233,6 +1304,7 @@ __device__ __forceinline__ void p_cand_top(const BItem &it, StreamDesc *S)
     }
 #pragma unroll
     for (int j = 0; j < COARSE; j++) g[j] = ldg((const uint4 *)area.coarse + threadIdx.x + j * kBThreads);
+    if (flagged) return;
     Cand l[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}}, r[4];
 #pragma unroll
     for (int j = 0; j < COARSE; j++) most = max(max(most, max(g[j].x, g[j].y)), max(g[j].z, g[j].w));
@@ -1269,31 +1341,36 @@ k_bcount(const BItem *items, const uint32_t *item_of, StreamDesc *S, uint32_t to
 {
     __shared__ __align__(16) unsigned char smem[kCandSmem];
     constexpr uint32_t NONE = 0xffffffffu;
+    __shared__ bool s_flagged;  // the item's sample says that the counts would prove nothing
     uint32_t t = blockIdx.x, cur = NONE;
     while (t < total_tiles) {
         const uint32_t k = item_of[t];
         if (k != cur) {
             __syncthreads();  // the counters are complete, nobody reads the previous descriptor any more
-            if (cur != NONE) cand_flush(shared_item_ref(), smem);
+            if (cur != NONE && !s_flagged) cand_flush(shared_item_ref(), smem);
             __syncthreads();
             shared_item(items, k);
+            const uint32_t flag = threadIdx.x == 0 ? *CandArea(shared_item_ref()).flag : 0;  // loads beside the others
             each_size(shared_item_ref().es, [&](auto es) { cand_load<decltype(es)::value>(shared_item_ref(), smem); });
+            if (threadIdx.x == 0) s_flagged = flag != 0;
             __syncthreads();
             cur = k;
         }
         const BItem &it = shared_item_ref();
         const uint32_t tile = t - (uint32_t)it.tile_base;
-        if ((uint64_t)tile * it.p[3] >= view_len(it, S)) {
+        const uint64_t n = view_len(it, S), t0 = (uint64_t)tile * it.p[3];
+        if (t0 >= n) {
             const uint64_t next = it.tile_base + it.tiles;  // the next item's first tile
             if (next >= total_tiles) break;
             t = (uint32_t)(next + (blockIdx.x + gridDim.x - next % gridDim.x) % gridDim.x);
             continue;
         }
-        each_size(it.es, [&](auto es) { cand_tile<decltype(es)::value>(shared_item_ref(), tile, S, smem); });
+        if (!s_flagged) each_size(it.es, [&](auto es) { cand_tile<decltype(es)::value>(shared_item_ref(), tile, S, smem); });
+        else if (it.mode == 4) clear_codes(it, t0, n < t0 + it.p[3] ? n : t0 + it.p[3], S);
         t += gridDim.x;
     }
     __syncthreads();
-    if (cur != NONE) cand_flush(shared_item_ref(), smem);
+    if (cur != NONE && !s_flagged) cand_flush(shared_item_ref(), smem);
 }
 
 // The items of a launch whose flag is set, in order, f(index) for each; the block's threads look at 256

@@ -62,3 +62,18 @@ def test_item_loops_of_other_widths(G, O, rng, dt):
     if dt != OR.CHAR:
         cases.append((walk, [OR.DELTA, OR.SCALE, OR.AFL, OR.NONE]))
     run_batch(G, O, [c for c, _ in cases], [dt] * len(cases), [G.tree_from_path(p, dt) for _, p in cases])
+
+
+@pytest.mark.parametrize("dt", [OR.CHAR, OR.SHORT, OR.INT, OR.TIME, OR.DOUBLE], ids=["char", "short", "int", "time", "double"])
+def test_few_values_of_one_frequency_need_no_full_histogram(G, O, rng, dt):
+    """some hundred equally frequent values, and 1 % others: the candidates tell the most frequent ones"""
+    npt = OR.NP_TYPES[dt]
+    cols, trees = [], []
+    for k, n in [(100, 20_011), (100, 400_003), (256, 400_003), (256, 1_000_001)]:
+        x = rng.integers(0, k, n)
+        if np.dtype(npt).itemsize >= 4:
+            x[rng.integers(0, n, n // 100)] = rng.integers(0, 1 << 31, n // 100)
+        cols.append((x % (100 if dt == OR.CHAR else 1 << 31)).astype(npt))
+        trees.append(G.tree_from_path(PATHS[0], dt))
+    b, _, _ = run_batch(G, O, cols, [dt] * len(cols), trees)
+    assert sum(by for name, _, by, _ in b.profile(True) if name == "hist_full") == 0
