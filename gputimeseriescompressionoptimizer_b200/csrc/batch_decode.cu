@@ -281,7 +281,8 @@ __device__ void p_delta_sum(const BItem &it, uint32_t tile, uint32_t step, uint3
     }
 }
 
-// The second pass: a warp adds up the sums before its unit and scans the unit in rows of 512 bytes, 16
+// The second pass: a warp adds up the sums before its unit (the groups', as the split does: 2^26 -> 2^30
+// int32, 0.156 -> 2.69 ms) and scans the unit in rows of 512 bytes, 16
 // bytes a lane.  CHECK as unit_vec; `end`: elements of the unit to write, `cnt` of them with a difference.
 template <int ES, bool CHECK>
 __device__ __forceinline__ void delta_unit(const UnitSrc<ES> &u, word_t<ES> acc, uint8_t *out, uint32_t cnt, uint32_t end)

@@ -37,23 +37,6 @@ __device__ __forceinline__ void load_run(const uint8_t *p, uint64_t base, uint64
     }
 }
 
-// element i of a shared-memory array of ES-byte elements
-template <int ES>
-__device__ __forceinline__ uint64_t ld_elem_sm(const uint8_t *sm, uint64_t i)
-{
-    if (ES == 1) return sm[i];
-    if (ES == 2) return ((const uint16_t *)sm)[i];
-    if (ES == 4) return ((const uint32_t *)sm)[i];
-    return ((const unsigned long long *)sm)[i];
-}
-
-// element i of a stream that may not be element aligned (streams inside a blob)
-template <int ES>
-__device__ __forceinline__ uint64_t ld_elem_any(const uint8_t *p, uint64_t i, bool aligned)
-{
-    return aligned ? ld_elem<ES>(p, i) : ld_unaligned<ES>(p + i * ES);
-}
-
 // Stores elements [base, min(base + VPT, n)) to an element-aligned stream (16-byte stores when the
 // whole run is in range and the stream is 16-byte aligned).
 template <int ES, int VPT>
@@ -82,10 +65,7 @@ __device__ __forceinline__ void store_run(uint8_t *p, uint64_t base, uint64_t n,
 // shared-memory wavefront of 16-byte accesses) fall in eight distinct 16-byte bank groups, while a
 // striped access still covers whole rows.  The warp's lanes all take part; no block barrier is
 // involved.  `xs` is the block's exchange area (16-byte aligned, kXchgBlockBytes), one tile per
-// warp.  Used where it measured faster: the RLE expansion's output and the split's and RLE heads'
-// source runs.  Not in the delta decode: there it sped up the many-column step but slowed one long
-// column's decode by a quarter (its stores leave the block later, and one column's tiles form a
-// single look-back chain).
+// warp.  Used where it measured faster: the RLE expansion's output and the RLE heads' source runs.
 constexpr int kXchgWarpBytes = 32 * (int)kBVPT * 8;
 constexpr int kXchgBlockBytes = kBThreads / 32 * kXchgWarpBytes;
 
@@ -629,21 +609,6 @@ __device__ __forceinline__ uint64_t dview_elem(const DViewCtx &v, uint64_t i)
         }
     }
     return wrap_es(x + v.c0 + v.c1, ES);
-}
-
-// elements [base, base + VPT) of the view (0 past its end)
-template <int ES, int VPT>
-__device__ __forceinline__ void load_dview(const DViewCtx &v, uint64_t base, uint64_t (&out)[VPT])
-{
-    if (v.b == 0 && v.aligned) {
-        load_run<ES, VPT>(v.p, base, v.n, out);
-        const uint64_t c = v.c0 + v.c1;
-#pragma unroll
-        for (int j = 0; j < VPT; j++) out[j] = wrap_es(out[j] + c, ES);
-        return;
-    }
-#pragma unroll
-    for (int j = 0; j < VPT; j++) out[j] = base + j < v.n ? dview_elem<ES>(v, base + j) : 0;
 }
 
 // copies items[k] into the block's shared descriptor (every thread of the block calls it; the

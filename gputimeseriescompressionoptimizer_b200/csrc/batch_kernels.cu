@@ -1,7 +1,7 @@
 // batch_kernels.cu -- the compress passes of the batched engine.
 //
-// Each pass is one templated stage kernel launched with one block per (item, tile); the block finds
-// its item by binary search over the items' first tiles.  Passes that rank elements across tiles
+// Each pass is one templated stage kernel over the (item, tile) pairs of a launch; a table gives the
+// item of every tile.  Passes that rank elements across tiles
 // (RLE heads, GFC offsets) claim tiles from a counter and chain them with the decoupled
 // look-back of scan.cuh, per item.  Every pass reads its input length from the stream table and
 // writes its outputs' lengths there; tile 0 (or the tile that ends the input) writes metadata.
@@ -441,6 +441,18 @@ __device__ void p_afl_pack(const BItem &it, uint32_t tile, uint32_t step, uint32
                 if (4 * w + k < out_bytes) out[4 * w + k] = (uint8_t)(word >> (8 * k));
         }
     }
+    }
+}
+
+// calls f with an element size as a constant (an integral_constant)
+template <class F>
+__device__ __forceinline__ void with_size(int es, F f)
+{
+    switch (es) {
+    case 1: f(std::integral_constant<int, 1>()); break;
+    case 2: f(std::integral_constant<int, 2>()); break;
+    case 4: f(std::integral_constant<int, 4>()); break;
+    default: f(std::integral_constant<int, 8>()); break;
     }
 }
 
@@ -1126,8 +1138,8 @@ __device__ __forceinline__ void p_hist_sample(const BItem &it, StreamDesc *S, un
         for (uint32_t w = fill[b]; w < 2; w++) image[2 * b + w] = b == special ? T::MARK2 : T::MARK;
 }
 
-// shared memory of the counting pass: keys, counts, coarse counts, a word a lane for the additions of
-// NaNs (unused), the smallest NaNs
+// shared memory of the counting pass: keys, counts, coarse counts, a word a lane that takes the
+// additions of NaNs (nobody reads it), the smallest NaNs
 constexpr uint32_t kCandNan = 8 * kBCandSlots + 4 * (kBCandSlots + kBCandCoarse) + 4 * 32, kCandSmem = kCandNan + 32;
 
 // keeps the four largest of the nk given to it: what a place gives up moves on to the next
@@ -1323,17 +1335,6 @@ __device__ __forceinline__ void p_cand_top(const BItem &it, StreamDesc *S)
 }
 
 #ifndef GTSC_PERSISTENT_TU
-template <class F>
-__device__ __forceinline__ void each_size(int es, F f)
-{
-    switch (es) {
-    case 1: f(std::integral_constant<int, 1>()); break;
-    case 2: f(std::integral_constant<int, 2>()); break;
-    case 4: f(std::integral_constant<int, 4>()); break;
-    default: f(std::integral_constant<int, 8>()); break;
-    }
-}
-
 // The counting pass's stage launch: as many blocks as are resident, striding over the tiles; a block
 // keeps its counters while its tiles are of one item.
 __global__ void __launch_bounds__(kBThreads, 4)
@@ -1351,7 +1352,7 @@ k_bcount(const BItem *items, const uint32_t *item_of, StreamDesc *S, uint32_t to
             __syncthreads();
             shared_item(items, k);
             const uint32_t flag = threadIdx.x == 0 ? *CandArea(shared_item_ref()).flag : 0;  // loads beside the others
-            each_size(shared_item_ref().es, [&](auto es) { cand_load<decltype(es)::value>(shared_item_ref(), smem); });
+            with_size(shared_item_ref().es, [&](auto es) { cand_load<decltype(es)::value>(shared_item_ref(), smem); });
             if (threadIdx.x == 0) s_flagged = flag != 0;
             __syncthreads();
             cur = k;
@@ -1365,7 +1366,7 @@ k_bcount(const BItem *items, const uint32_t *item_of, StreamDesc *S, uint32_t to
             t = (uint32_t)(next + (blockIdx.x + gridDim.x - next % gridDim.x) % gridDim.x);
             continue;
         }
-        if (!s_flagged) each_size(it.es, [&](auto es) { cand_tile<decltype(es)::value>(shared_item_ref(), tile, S, smem); });
+        if (!s_flagged) with_size(it.es, [&](auto es) { cand_tile<decltype(es)::value>(shared_item_ref(), tile, S, smem); });
         else if (it.mode == 4) clear_codes(it, t0, n < t0 + it.p[3] ? n : t0 + it.p[3], S);
         t += gridDim.x;
     }
@@ -1401,7 +1402,7 @@ k_bhist(const BItem *items, int n_items, StreamDesc *S, uint32_t *status)
     flagged_items(items, n_items, [&](int k) {
         __syncthreads();
         const BItem &it = shared_item(items, k);
-        each_size(it.es, [&](auto es) {
+        with_size(it.es, [&](auto es) {
             constexpr int E = decltype(es)::value;
             const uint64_t n = view_len(it, S), tiles = (n + it.p[3] - 1) / it.p[3];
             bool dirty = false;  // the table holds counts, up to tile `last`
@@ -1434,7 +1435,7 @@ __global__ void __launch_bounds__(kBThreads, 4) k_btopk(const BItem *items, int 
     flagged_items(items, n_items, [&](int k) {
         __syncthreads();
         const BItem &it = shared_item(items, k);
-        each_size(it.es, [&](auto es) { topk_blocks<decltype(es)::value>(it, blockIdx.x, gridDim.x, S); });
+        with_size(it.es, [&](auto es) { topk_blocks<decltype(es)::value>(it, blockIdx.x, gridDim.x, S); });
     });
 }
 #endif
@@ -1444,18 +1445,6 @@ __global__ void __launch_bounds__(kBThreads, 4) k_btopk(const BItem *items, int 
 constexpr int kSplitOutside = 100;
 // code bytes of a warp in a dictionary's split: a unit's, from any place in a code word
 constexpr uint32_t kSplitCodes = kBSplitUnit + 16;
-
-// calls f with an element size as a constant (an integral_constant)
-template <class F>
-__device__ __forceinline__ void with_size(int es, F f)
-{
-    switch (es) {
-    case 1: f(std::integral_constant<int, 1>()); break;
-    case 2: f(std::integral_constant<int, 2>()); break;
-    case 4: f(std::integral_constant<int, 4>()); break;
-    default: f(std::integral_constant<int, 8>()); break;
-    }
-}
 
 // a split's element as a signed value, for the min / max of its classes
 template <int ES>
@@ -1703,7 +1692,9 @@ __device__ __forceinline__ void split_rows(const ViewCtx &vc, const uint8_t *src
 
 // The second pass: every unit's values to the match and the other stream (n * s read again -- from L2
 // for all but the largest columns -- and written).  The matches before a unit are the sums of the groups
-// before its tile's, of the tiles before it in the group and of the units before it in the tile; a
+// before its tile's, of the tiles before it in the group and of the units before it in the tile (a number
+// for every 2^19 values before it: a term in the square of the length, which does not show yet from 2^26
+// to 2^30 int32, both passes 0.169 -> 2.56 ms, where the look-back took 0.38 -> 5.92); a
 // value's rank in its unit comes from the stencil words.  Rows are stored straight to the two runs;
 // only a dictionary's 2-bit codes pass through shared memory, to be packed 16 a word.
 // 2^26 int32, both passes: patch 0.430 -> 0.182 ms, Zipf(1.1) dictionary 0.506 -> 0.233 ms (0.206 and
@@ -2354,8 +2345,7 @@ constexpr bool stage_persistent(int op)
 // resident blocks per SM the compiler keeps registers for (measured per pass on the mixed workload)
 constexpr int stage_min_blocks(int op)
 {
-    // the histogram at 4 (64 registers, no spills) measured 6 % faster than at 5 (48 registers, spilling)
-    return op == B_AFL_PACK || op == B_GFC_COMPRESS || op == B_TOPK || op == B_HIST ? 4 : 5;
+    return op == B_AFL_PACK || op == B_GFC_COMPRESS || op == B_TOPK ? 4 : 5;
 }
 
 template <int OP>
