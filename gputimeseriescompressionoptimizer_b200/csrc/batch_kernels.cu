@@ -1041,8 +1041,7 @@ __device__ __forceinline__ void p_hist_sample(const BItem &it, StreamDesc *S, un
     static_assert(SAMPLE == 1u << 11 && SLOTS * 12 + 4 * kCandBuckets + 4 * 64 + 16 <= kSampleSmem, "the sample's shared memory");
     const CandArea area(it);
     K *keys = (K *)smem;
-    uint32_t *counts = (uint32_t *)(smem + SLOTS * 8), *fill = counts + SLOTS, *of_count = fill + kCandBuckets,
-             *least = of_count + 64;
+    uint32_t *counts = (uint32_t *)(smem + SLOTS * 8), *fill = counts + SLOTS, *of_count = fill + kCandBuckets;
     const StreamDesc in = S[it.in[0]];
     const ViewCtx vc = view_ctx<ES>(it, in);
     const uint64_t n = vc.n;
@@ -1084,44 +1083,26 @@ __device__ __forceinline__ void p_hist_sample(const BItem &it, StreamDesc *S, un
     for (uint32_t i = threadIdx.x; i < SLOTS; i += kBThreads)
         if (counts[i]) atomicAdd(of_count + (counts[i] < 63 ? counts[i] : 63), 1u);
     __syncthreads();
-    if (threadIdx.x < 32) {
-        const uint32_t lane = threadIdx.x, k = (uint32_t)it.mode;
-        uint32_t lo = of_count[lane], hi = of_count[32 + lane];  // -> values that occur lane, 32 + lane times or more
+    // every warp by itself: how many values occur lane, 32 + lane times or more
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t lo = of_count[lane], hi = of_count[32 + lane];
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t x = __shfl_down_sync(0xffffffffu, lo, d), y = __shfl_down_sync(0xffffffffu, hi, d);
-            if (lane + d < 32) {
-                lo += x;
-                hi += y;
-            }
-        }
-        lo += __shfl_sync(0xffffffffu, hi, 0);
-        // the largest count that more than `most` values reach, 0 if none does
-        auto reached = [&](uint32_t most) -> uint32_t {
-            const uint32_t h = __ballot_sync(0xffffffffu, hi > most), l = __ballot_sync(0xffffffffu, lane && lo > most);
-            return h ? 63 - __clz(h) : l ? 31 - __clz(l) : 0;
-        };
-        const uint32_t distinct = __shfl_sync(0xffffffffu, lo, 1), two = __shfl_sync(0xffffffffu, lo, 2),
-                       three = __shfl_sync(0xffffffffu, lo, 3);
-        const uint32_t taken = distinct <= ALL ? 1 : reached(MOST) + 1, kth = reached(k - 1);
-        if (lane == 0) {
-            least[0] = taken;                    // the smallest count taken
-            least[1] = distinct > MOST ? 3 : 2;  // passes (few values leave no bucket short)
-            // The counting pass is for nothing when the k-th best is no better than chance among values of one
-            // frequency: of such, m1 of which occur once and m2 twice, about m1 l^(c-1) / c! occur c times,
-            // l = 2 m2 / m1 (over 400 of them: l below 6).  A k-th best of two is chance only if many others
-            // occur twice.
-            if (taken > 1 && kth < 63) {
-                const float m1 = (float)(distinct - two), l = m1 > 0 ? fminf(2 * (float)(two - three) / m1, 6.f) : 0.f;
-                const float enough = (float)k * (kth == 2 ? 4.f : 0.25f);
-                float chance = m1;
-                for (uint32_t j = 2; j <= kth && (chance >= enough || (float)j <= l); j++) chance *= __fdividef(l, (float)j);
-                if (chance >= enough) *area.flag = 1;
-            }
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t x = __shfl_down_sync(0xffffffffu, lo, d), y = __shfl_down_sync(0xffffffffu, hi, d);
+        if (lane + d < 32) {
+            lo += x;
+            hi += y;
         }
     }
-    __syncthreads();
-    const uint32_t t = least[0], passes = t > 1 ? 2 : least[1];
+    lo += __shfl_sync(0xffffffffu, hi, 0);
+    // the largest count that more than `most` values reach, 0 if none does
+    auto reached = [&](uint32_t most) -> uint32_t {
+        const uint32_t h = __ballot_sync(0xffffffffu, hi > most), l = __ballot_sync(0xffffffffu, lane && lo > most);
+        return h ? 63 - __clz(h) : l ? 31 - __clz(l) : 0;
+    };
+    const uint32_t distinct = __shfl_sync(0xffffffffu, lo, 1);
+    const uint32_t t = distinct <= ALL ? 1 : reached(MOST) + 1;                 // the smallest count taken
+    const uint32_t passes = distinct <= ALL && distinct > MOST ? 3 : 2;         // (few values leave no bucket short)
     K *image = (K *)area.keys;
 #pragma unroll 1
     for (uint32_t pass = 0; pass < passes; pass++) {
@@ -1132,6 +1113,18 @@ __device__ __forceinline__ void p_hist_sample(const BItem &it, StreamDesc *S, un
             if (w < 2) image[2 * b + w] = keys[i];
         }
         __syncthreads();
+    }
+    // The counting pass is for nothing when the k-th best is no better than chance among values of one
+    // frequency: of such, m1 of which occur once and m2 twice, about m1 l^(c-1) / c! occur c times,
+    // l = 2 m2 / m1 (over 400 of them: l below 6).  A k-th best of two is chance only if many others
+    // occur twice.
+    const uint32_t kth = reached((uint32_t)it.mode - 1), two = __shfl_sync(0xffffffffu, lo, 2), three = __shfl_sync(0xffffffffu, lo, 3);
+    if (threadIdx.x == kBThreads - 1 && t > 1 && kth < 63) {
+        const float m1 = (float)(distinct - two), l = m1 > 0 ? fminf(2 * (float)(two - three) / m1, 6.f) : 0.f;
+        const float enough = (float)it.mode * (kth == 2 ? 4.f : 0.25f);
+        float chance = m1;
+        for (uint32_t j = 2; j <= kth && (chance >= enough || (float)j <= l); j++) chance *= __fdividef(l, (float)j);
+        if (chance >= enough) *area.flag = 1;
     }
     const uint32_t special = cand_hash<ES>(T::MARK) >> 23;
     for (uint32_t b = threadIdx.x; b < kCandBuckets; b += kBThreads)
