@@ -409,7 +409,7 @@ PASS_NAMES = dict(enumerate(
      "f2i_stats", "f2i_enc", "f2i_raw", "gfc_compress", "gfc_scan", "gfc_compact", "none_copy", "afl_unpack",
      "delta_dec", "scale_add", "merge", "rle_scan", "rle_expand", "f2i_dec", "gfc_sizes", "gfc_dec", "vmeta",
      "merge_count", "split_count", "hist_sample", "hist_full", "topk_full",
-     "delta_sum"]))
+     "delta_sum", "split_short", "delta_short"]))
 PASS_NAMES.update({-1: "set_streams", -2: "zero", -3: "frame_sizes", -4: "frame_layout", -5: "frame_copy",
                    -6: "parse_frames", -7: "persistent"})
 

@@ -143,6 +143,15 @@ bool dyn_pass(int op)
 // blocks of the passes of a delta decode of n elements
 uint64_t delta_tiles(uint64_t n) { return std::max<uint64_t>(1, cdiv(n, kBDeltaTile)); }
 
+// Whether nodes of one kind take their two passes in one launch (kBShortTiles): where all of them are short,
+// as beside long columns a launch less is not seen and clusters wait for their blocks (256 mixed columns,
+// decompress: 2918 -> 2940 us), and all their clusters are resident at four blocks an SM, as the grids of two
+// passes leave out tiles that a column does not have.
+bool short_in_one(uint64_t nodes, uint64_t short_ones)
+{
+    return short_ones == nodes && nodes * kBShortTiles <= 4 * (uint64_t)sm_count();
+}
+
 // blocks of the counting pass of a merge over n elements
 uint64_t merge_count_tiles(uint64_t n) { return std::max<uint64_t>(1, cdiv(n, kBCountTile)); }
 
@@ -437,6 +446,16 @@ void BatchEngine::plan_passes()
         return it;
     };
 
+    uint64_t splits = 0, short_splits = 0, deltas = 0, short_deltas = 0;
+    for (auto &nd : nodes) {
+        const bool split = nd.enc == GTSC_PATCH || nd.enc == GTSC_PATCH_OUTSIDE || nd.enc == GTSC_DICT || nd.enc == GTSC_CONST;
+        splits += split;
+        deltas += nd.enc == GTSC_DELTA;
+        short_splits += split && nd.split_tiles <= kBShortTiles;
+        short_deltas += nd.enc == GTSC_DELTA && delta_tiles(nd.in_cap / nd.es) <= kBShortTiles;
+    }
+    const bool one_split = short_in_one(splits, short_splits), one_delta = short_in_one(deltas, short_deltas);
+
     // ---------------- compress passes (parents before children)
     for (size_t id = 0; id < nodes.size(); id++) {
         HNode &nd = nodes[id];
@@ -455,6 +474,12 @@ void BatchEngine::plan_passes()
             for (int kid : nd.kids) {
                 const int slot = folded_minmax(kid);
                 if (slot) cnt.p[1 + slot] = (uint64_t)kid + 1;
+            }
+            if (one_split) {
+                cnt.op = B_SPLIT_SHORT;
+                cnt.tiles = 1;  // one cluster
+                add(cnt);
+                return;
             }
             add(cnt);
             add(sp);
@@ -662,6 +687,13 @@ void BatchEngine::plan_passes()
         case GTSC_DELTA: {
             BItem it = ditem(B_DELTA_SUM, delta_tiles(n));
             it.p[0] = nd.dlb_off;
+            it.p[1] = it.tiles;
+            if (one_delta) {
+                it.op = B_DELTA_SHORT;
+                it.tiles = 1;  // one cluster
+                ps.push_back(it);
+                break;
+            }
             ps.push_back(it);
             it.op = B_DELTA_DEC;
             ps.push_back(it);
@@ -784,10 +816,10 @@ void BatchEngine::layout(cudaStream_t s)
             while (j < ps.size() && ps[j].level == ps[i].level && ps[j].op == ps[i].op) {
                 BItem it = ps[j].item;
                 it.scratch = A + nodes[ps[j].node].scratch;
-                if (ps[j].op == B_SPLIT_COUNT)  // the children whose min / max the split accumulates
+                if (ps[j].op == B_SPLIT_COUNT || ps[j].op == B_SPLIT_SHORT)  // the children whose min / max the split accumulates
                     for (int q = 2; q < 4; q++)
                         it.p[q] = it.p[q] ? (uint64_t)(uintptr_t)(A + nodes[it.p[q] - 1].scratch) : 0;
-                if (ps[j].op < B_NONE_COPY || ps[j].op == B_VMETA || (ps[j].op >= B_SPLIT_COUNT && ps[j].op <= B_TOPK_FULL))  // compress: the view's scale nodes
+                if (ps[j].op < B_NONE_COPY || ps[j].op == B_VMETA || ps[j].op == B_SPLIT_SHORT || (ps[j].op >= B_SPLIT_COUNT && ps[j].op <= B_TOPK_FULL))  // compress: the view's scale nodes
                     for (int v = 0; v < kMaxViewOps; v++) {
                         const int sn = nodes[ps[j].node].vnode[v];
                         it.vscr[v] = sn >= 0 ? A + nodes[sn].scratch : nullptr;
@@ -1435,7 +1467,7 @@ static uint64_t item_bytes(const BItem &it, const std::vector<StreamDesc> &S)
     case B_TOPK: case B_HIST_SAMPLE: case B_TOPK_FULL: case B_F2I_RAW: case B_GFC_SCAN: return 0;
     case B_DELTA_ENC: case B_SCALE_SUB: case B_AFL_PACK: case B_F2I_ENC: return in + L(it.out[0]) + L(it.out[1]);
     case B_SPLIT_COUNT: return in + L(it.out[0]);
-    case B_SPLIT: return in + L(it.out[0]) + L(it.out[1]) + L(it.out[2]);
+    case B_SPLIT: case B_SPLIT_SHORT: return in + L(it.out[0]) + L(it.out[1]) + L(it.out[2]);
     case B_RLE_HEADS: return in + L(it.out[0]) + L(it.out[2]) + L(it.out[1]);  // values, run starts
     case B_RLE_LENGTHS: return 2 * L(it.out[1]);
     case B_GFC_COMPRESS: return in + L(it.out[1]) + L(it.out[2]);
@@ -1443,7 +1475,7 @@ static uint64_t item_bytes(const BItem &it, const std::vector<StreamDesc> &S)
     case B_NONE_COPY: return 2 * in;
     case B_AFL_UNPACK: return L(it.in[1]) + L(it.out[0]);
     case B_DELTA_SUM: return D(1);
-    case B_DELTA_DEC: case B_SCALE_ADD: case B_F2I_DEC: return D(1) + L(it.out[0]);
+    case B_DELTA_DEC: case B_DELTA_SHORT: case B_SCALE_ADD: case B_F2I_DEC: return D(1) + L(it.out[0]);
     case B_MERGE: return in + (it.mode == SPLIT_DICT ? L(it.in[1]) : D(1)) + D(2) + L(it.out[0]);
     case B_RLE_SCAN: return D(1);
     case B_MERGE_COUNT: return L(it.in[0]);

@@ -48,6 +48,8 @@ enum BOp : int {
     B_HIST_FULL,       // compress: dict / const: the full histogram, where the bounds prove nothing
     B_TOPK_FULL,       // compress: its most frequent values
     B_DELTA_SUM,       // decode: sums of the differences of every unit
+    B_SPLIT_SHORT,     // compress: both split passes of a short column
+    B_DELTA_SHORT,     // decode: both delta passes of a short column
     B_NUM_OPS
 };
 
@@ -256,6 +258,12 @@ constexpr uint32_t kBSplitGroup = 64;                // tiles whose matches are 
 
 constexpr uint32_t kBPackUnit = 512;    // AFL packing: values of a warp's unit (whole 16-byte pieces at any width)
 constexpr uint32_t kBDeltaUnit = 1024, kBDeltaTile = 8 * kBDeltaUnit, kBDeltaGroup = 64;  // delta decode, alike
+
+// Split and delta decode of columns of up to 8 tiles (64 Ki values), where a batch has few and no longer ones
+// (short_in_one): both passes in one launch, a cluster of 8 blocks a column with its barrier between them.
+// A launch of its own for the first pass cost a column of 1000 to 60000 values 2-4 us.
+constexpr uint32_t kBShortTiles = 8;
+static_assert(kBShortTiles <= kBSplitGroup && kBShortTiles <= kBDeltaGroup, "one group of tiles");
 
 // scratch of a delta decode: sums (u64) of the groups, the tiles and the units
 __host__ __device__ inline uint64_t bdelta_groups(uint64_t tiles) { return (tiles + kBDeltaGroup - 1) / kBDeltaGroup; }

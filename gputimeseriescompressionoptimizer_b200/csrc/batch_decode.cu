@@ -215,8 +215,8 @@ struct DeltaSums {
     __device__ __forceinline__ DeltaSums(const BItem &it)
     {
         groups = (unsigned long long *)(it.scratch + it.p[0]);
-        tiles = groups + bdelta_groups(it.tiles);
-        units = tiles + it.tiles;
+        tiles = groups + bdelta_groups(it.p[1]);  // p[1]: the column's tiles
+        units = tiles + it.p[1];
     }
 };
 
@@ -343,7 +343,7 @@ __device__ __forceinline__ void delta_unit(const UnitSrc<ES> &u, word_t<ES> acc,
 // int32 in 5 bits, both passes: 0.400 -> 0.178 ms (0.115 of it here); the 256 mixed columns' delta decodes
 // 0.84 -> 0.72 ms.  Tried: four tiles a block behind one setup (long columns 3 % faster, short ones twice
 // as slow); blocks of short columns summing what lies before them instead of a pass (no faster).
-template <int ES>
+template <int ES, bool OWN = false>
 __device__ void p_delta_dec(const BItem &it, uint32_t tile, StreamDesc *S, uint32_t *status)
 {
     using V = word_t<ES>;
@@ -364,9 +364,9 @@ __device__ void p_delta_dec(const BItem &it, uint32_t tile, StreamDesc *S, uint3
     const DeltaSums ds(it);
     const uint32_t g = tile / kBDeltaGroup;
     unsigned long long part = 0;
-    for (uint32_t k = lane; k < g; k += 32) part += ldg(ds.groups + k);
-    for (uint32_t k = g * kBDeltaGroup + lane; k < tile; k += 32) part += ldg(ds.tiles + k);
-    if (lane < warp) part += ldg(ds.units + (uint64_t)tile * WARPS + lane);
+    for (uint32_t k = lane; k < g; k += 32) part += ld_sum<OWN>(ds.groups + k);
+    for (uint32_t k = g * kBDeltaGroup + lane; k < tile; k += 32) part += ld_sum<OWN>(ds.tiles + k);
+    if (lane < warp) part += ld_sum<OWN>(ds.units + (uint64_t)tile * WARPS + lane);
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(0xffffffffu, part, d);
     const V acc = (V)(ld_unaligned<ES>(meta.ptr) + part);
@@ -1160,6 +1160,34 @@ __device__ __forceinline__ void run_dec(const BItem &it, uint32_t tile, uint32_t
 #undef GTSC_ES_SWITCH
 }
 
+// tiles of a short column's differences (more = 0) or values (1)
+__device__ __forceinline__ uint32_t short_delta_tiles(const BItem &it, const StreamDesc *S, uint32_t more)
+{
+    const uint64_t t = (dview_len(it, S, 1, it.es) + more + kBDeltaTile - 1) / kBDeltaTile;
+    return (uint32_t)(t < it.p[1] ? t : it.p[1]);
+}
+
+#ifndef GTSC_PERSISTENT_TU
+// Both passes over short columns, a cluster a column and a block a tile.  One column, differences of 5000 /
+// 20001 int64 stored plainly, whole decompress step: 27.1 / 27.9 -> 22.9 / 26.7 us.
+__global__ void __cluster_dims__(kBShortTiles, 1, 1) __launch_bounds__(kBThreads, 4)
+k_bdelta_short(const BItem *items, StreamDesc *S, uint32_t *status)
+{
+    if (*(volatile uint32_t *)(status + 1)) return;  // the frames did not parse: no block has work
+    const BItem &it = shared_item(items, blockIdx.x / kBShortTiles);
+    const uint32_t tile = blockIdx.x % kBShortTiles;
+    if (tile < short_delta_tiles(it, S, 0)) run_dec<B_DELTA_SUM>(it, tile, 1, tile + 1, S, status, nullptr);
+    cluster_sync();
+    if (tile >= short_delta_tiles(it, S, 1)) return;
+    switch (it.es) {
+    case 1: p_delta_dec<1, true>(it, tile, S, status); break;
+    case 2: p_delta_dec<2, true>(it, tile, S, status); break;
+    case 4: p_delta_dec<4, true>(it, tile, S, status); break;
+    default: p_delta_dec<8, true>(it, tile, S, status); break;
+    }
+}
+#endif
+
 #ifdef GTSC_PERSISTENT_TU
 // ------------------------------------------------------------------------------- persistent step
 constexpr size_t kPersistSmemD = std::max<size_t>({kGfcRing * (kBThreads / 32), kXchgBlockBytes});
@@ -1190,8 +1218,15 @@ __global__ void __launch_bounds__(kBThreads, 4) k_bpersist_d(PersistArgs a)
 #define GTSC_RUN(OPC) case OPC: run_dec<OPC>(it, tile, 1, tile + 1, a.S, a.status, smem); break;
                 GTSC_RUN(B_NONE_COPY)
                 GTSC_RUN(B_AFL_UNPACK)
-                GTSC_RUN(B_DELTA_SUM)
-                GTSC_RUN(B_DELTA_DEC)
+            case B_DELTA_SUM: case B_DELTA_DEC: case B_DELTA_SHORT: {  // short: the column's tiles by this block
+                const bool one = op == B_DELTA_SHORT;
+                const uint32_t end = one ? short_delta_tiles(it, a.S, 1) : tile + 1;
+                if (op != B_DELTA_DEC) run_dec<B_DELTA_SUM>(it, tile, 1, one ? short_delta_tiles(it, a.S, 0) : end, a.S, a.status, smem);
+                if (one) __syncthreads();
+                if (op != B_DELTA_SUM)
+                    for (uint32_t t = tile; t < end; t++) run_dec<B_DELTA_DEC>(it, t, 1, t + 1, a.S, a.status, smem);
+                break;
+            }
                 GTSC_RUN(B_SCALE_ADD)
                 GTSC_RUN(B_MERGE)
                 GTSC_RUN(B_MERGE_COUNT)
@@ -1406,6 +1441,9 @@ void launch_batch_decode_stage(int op, const BItem *d_items, const uint32_t *d_i
         GTSC_STAGE(B_AFL_UNPACK)
         GTSC_STAGE(B_DELTA_SUM)
         GTSC_STAGE(B_DELTA_DEC)
+    case B_DELTA_SHORT:
+        k_bdelta_short<<<(unsigned)n_items * kBShortTiles, kBThreads, 0, s>>>(d_items, d_streams, d_status);
+        break;
         GTSC_STAGE(B_SCALE_ADD)
         GTSC_STAGE(B_MERGE)
         GTSC_STAGE(B_MERGE_COUNT)

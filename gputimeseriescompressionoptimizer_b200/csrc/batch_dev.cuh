@@ -611,6 +611,19 @@ __device__ __forceinline__ uint64_t dview_elem(const DViewCtx &v, uint64_t i)
     return wrap_es(x + v.c0 + v.c1, ES);
 }
 
+// a sum that the pass before left: by another launch, or (OWN) by this one
+template <bool OWN, class T>
+__device__ __forceinline__ T ld_sum(const T *p)
+{
+    return OWN ? *p : ldg(p);
+}
+
+// every thread of the cluster; what its blocks wrote before is seen by all of them after it
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // copies items[k] into the block's shared descriptor (every thread of the block calls it; the
 // caller makes sure no thread still reads the previous one); fields are then read from shared
 // memory instead of every thread loading the whole descriptor into registers

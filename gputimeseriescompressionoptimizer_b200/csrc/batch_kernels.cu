@@ -1694,7 +1694,7 @@ __device__ __forceinline__ void split_rows(const ViewCtx &vc, const uint8_t *src
 // 0.247 with the setup done for every tile).  One pass with
 // the rows held in registers behind a look-back took 0.26 and 0.29 ms (its warps wait at the barrier of
 // the look-back); the same with two tiles in flight a block 0.27 and 0.33 ms (too few warps).
-template <int ES, int MODE>
+template <int ES, int MODE, bool OWN>
 __device__ __forceinline__ void split_move(const BItem &it, uint32_t tile, uint32_t step, uint32_t end, StreamDesc *S,
                                            unsigned char *sm)
 {
@@ -1715,20 +1715,20 @@ __device__ __forceinline__ void split_move(const BItem &it, uint32_t tile, uint3
     const uint64_t w0 = (uint64_t)tile * kBSplitTile + warp * kBSplitUnit;  // the warp's first value
     if (w0 >= n) break;
     const uint32_t cnt = (uint32_t)(n - w0 < kBSplitUnit ? n - w0 : kBSplitUnit);
-    uint32_t word = 32 * lane < cnt ? ldg((const uint32_t *)(meta + (CONST ? ES + 1 : 1)) + w0 / 32 + lane) : 0u;
+    uint32_t word = 32 * lane < cnt ? ld_sum<OWN>((const uint32_t *)(meta + (CONST ? ES + 1 : 1)) + w0 / 32 + lane) : 0u;
     if (cnt < 32 * lane + 32 && cnt > 32 * lane) word &= (1u << (cnt - 32 * lane)) - 1;
     // the matches before the unit
     const unsigned long long *groups = (const unsigned long long *)(it.scratch + it.p[0]);
     const uint4 *counts = (const uint4 *)((const uint8_t *)groups + bsplit_group_bytes(it.tiles));
     unsigned long long part = 0;
     const uint32_t g = tile / kBSplitGroup;
-    for (uint32_t k = lane; k < g; k += 32) part += ldg(groups + k);
+    for (uint32_t k = lane; k < g; k += 32) part += ld_sum<OWN>(groups + k);
     auto halves = [](uint32_t w) { return (w & 0xffffu) + (w >> 16); };
     for (uint32_t k = g * kBSplitGroup + lane; k < tile; k += 32) {
-        const uint4 q = ldg(counts + k);
+        const uint4 q = ld_sum<OWN>(counts + k);
         part += halves(q.x) + halves(q.y) + halves(q.z) + halves(q.w);
     }
-    if (lane < warp) part += ldg((const uint16_t *)(counts + tile) + lane);
+    if (lane < warp) part += ld_sum<OWN>((const uint16_t *)(counts + tile) + lane);
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(0xffffffffu, part, d);
     const uint64_t yes0 = part, no0 = w0 - yes0;
@@ -1790,14 +1790,37 @@ __device__ __forceinline__ void split_move(const BItem &it, uint32_t tile, uint3
     }
 }
 
-template <int ES>
+template <int ES, bool OWN = false>
 __device__ __forceinline__ void p_split(const BItem &it, uint32_t tile, uint32_t step, uint32_t end, StreamDesc *S,
                                         unsigned char *sm)
 {
-    if (it.mode == SPLIT_DICT) split_move<ES, SPLIT_DICT>(it, tile, step, end, S, sm);
-    else if (it.mode == SPLIT_NOT_CONST) split_move<ES, SPLIT_NOT_CONST>(it, tile, step, end, S, sm);
-    else split_move<ES, SPLIT_LOWER>(it, tile, step, end, S, sm);
+    if (it.mode == SPLIT_DICT) split_move<ES, SPLIT_DICT, OWN>(it, tile, step, end, S, sm);
+    else if (it.mode == SPLIT_NOT_CONST) split_move<ES, SPLIT_NOT_CONST, OWN>(it, tile, step, end, S, sm);
+    else split_move<ES, SPLIT_LOWER, OWN>(it, tile, step, end, S, sm);
 }
+
+// tiles of a short column's split
+__device__ __forceinline__ uint32_t short_split_tiles(const BItem &it, const StreamDesc *S)
+{
+    const uint64_t t = (view_len(it, S) + kBSplitTile - 1) / kBSplitTile;
+    return t < 1 ? 1u : t < kBShortTiles ? (uint32_t)t : kBShortTiles;
+}
+
+#ifndef GTSC_PERSISTENT_TU
+// Both passes over short columns, a cluster a column and a block a tile.  One column, patch of 5000 / 20001
+// int32, whole compress step: 31 / 33 -> 29 / 31 us.
+__global__ void __cluster_dims__(kBShortTiles, 1, 1) __launch_bounds__(kBThreads, 4)
+k_bsplit_short(const BItem *items, StreamDesc *S)
+{
+    __shared__ __align__(16) unsigned char smem[kSplitCodes * (kBThreads / 32)];
+    const BItem &it = shared_item(items, blockIdx.x / kBShortTiles);
+    const uint32_t tile = blockIdx.x % kBShortTiles;
+    const bool mine = tile < short_split_tiles(it, S);
+    if (mine) p_split_count(it, tile, 1, tile + 1, S);
+    cluster_sync();
+    if (mine) with_size(it.es, [&](auto es) { p_split<decltype(es)::value, true>(it, tile, 1, tile + 1, S, smem); });
+}
+#endif
 
 // ------------------------------------------------------------------------------- RLE
 template <int ES>
@@ -2470,8 +2493,13 @@ __global__ void __launch_bounds__(kBThreads, 4) k_bpersist_c(PersistArgs a)
             GTSC_RUN(B_TOPK)
             GTSC_RUN(B_HIST_FULL)
             GTSC_RUN(B_TOPK_FULL)
-            GTSC_RUN(B_SPLIT_COUNT)
-            GTSC_RUN(B_SPLIT)
+        case B_SPLIT_COUNT: case B_SPLIT: case B_SPLIT_SHORT: {  // short: the column's tiles by this block
+            const uint32_t end = op == B_SPLIT_SHORT ? short_split_tiles(it, a.S) : tile + 1;
+            if (op != B_SPLIT) run_stage<B_SPLIT_COUNT>(it, tile, 1, end, a.S, a.status, smem);
+            if (op == B_SPLIT_SHORT) __syncthreads();
+            if (op != B_SPLIT_COUNT) run_stage<B_SPLIT>(it, tile, 1, end, a.S, a.status, smem);
+            break;
+        }
             GTSC_RUN(B_RLE_HEADS)
             GTSC_RUN(B_RLE_LENGTHS)
             GTSC_RUN(B_F2I_STATS)
@@ -2563,6 +2591,9 @@ void launch_batch_stage(int op, const BItem *d_items, const uint32_t *d_item_of,
         GTSC_STAGE(B_TOPK)
         GTSC_STAGE(B_SPLIT_COUNT)
         GTSC_STAGE(B_SPLIT)
+    case B_SPLIT_SHORT:
+        k_bsplit_short<<<(unsigned)n_items * kBShortTiles, kBThreads, 0, s>>>(d_items, d_streams);
+        break;
         GTSC_STAGE(B_RLE_HEADS)
         GTSC_STAGE(B_RLE_LENGTHS)
         GTSC_STAGE(B_F2I_STATS)
