@@ -155,6 +155,10 @@ bool short_in_one(uint64_t nodes, uint64_t short_ones)
 // blocks of the counting pass of a merge over n elements
 uint64_t merge_count_tiles(uint64_t n) { return std::max<uint64_t>(1, cdiv(n, kBCountTile)); }
 
+// the prefixes of a merge's units (8 bytes each; two more than the column's, as its output may be larger by
+// less than 256 bytes)
+uint64_t merge_prefix_bytes(uint64_t n) { return align_up(8 * cdiv(n, kBMergeUnit) + 16, 256); }
+
 constexpr uint32_t kMinMaxTileMin = 1024;  // the smallest min/max tile (tiles are reserved for it)
 
 uint64_t gfc_warps_for(bool dbl, uint64_t n)
@@ -398,7 +402,7 @@ void BatchEngine::plan_passes()
         case GTSC_PATCH: case GTSC_PATCH_OUTSIDE: case GTSC_DICT: case GTSC_CONST:
             nd.dlb_off = nd.c_bytes;
             nd.dpre_off = nd.dlb_off + align_up(lookback_bytes(merge_count_tiles(n)), 256);
-            d = nd.dpre_off + align_up(8 * cdiv(n, kBMergeUnit) + 16, 256) - nd.c_bytes;
+            d = nd.dpre_off + merge_prefix_bytes(n) - nd.c_bytes;
             break;
         case GTSC_RLE:
             nd.dlb_off = nd.c_bytes;
@@ -710,6 +714,7 @@ void BatchEngine::plan_passes()
             BItem cnt = it;
             cnt.op = B_MERGE_COUNT;
             cnt.tiles = (uint32_t)merge_count_tiles(n);
+            cnt.p[2] = merge_prefix_bytes(n) / 8 * kBMergeUnit;
             pass_d.push_back(Pass{-1, B_MERGE_COUNT, id, cnt});
             ps.push_back(it);
             break;

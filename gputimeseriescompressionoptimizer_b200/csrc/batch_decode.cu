@@ -451,9 +451,10 @@ __device__ void p_merge_count(const BItem &it, uint32_t tile, StreamDesc *S)
     static_assert(kBMergeUnit == 32 * 32 && UNITS % (WARPS * 4) == 0, "a warp row of stencil words is one unit");
     uint64_t n;
     const uint8_t *bits = merge_stencil<ES>(it, S[it.in[0]], n) + 1;
-    // the frame of a longer column than this one: its units would pass the prefixes, of which there are as
-    // many as the output holds units.  Nothing is counted then, and the merge reports it.
-    if (n * ES > S[it.out[0]].cap) n = 0;
+    // the frame of a longer column than this one: its units would pass the prefixes, which hold those of p[2]
+    // values, the output's and some more.  Nothing is counted then, and the merge reports it.  (A number of
+    // the item: the output's own, from the stream table, cost a short column half a microsecond.)
+    if (n > it.p[2]) n = 0;
     // a tile past the output has no successor waiting on its look-back descriptor
     if (tile > 0 && (uint64_t)tile * kBCountTile >= n) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
